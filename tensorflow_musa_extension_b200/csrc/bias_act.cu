@@ -3,8 +3,8 @@
 // y = act(x + bias[channel]) with act in {identity, relu, swish, sigmoid};
 // `swish` is the three-op chain Mul(x, Sigmoid(BiasAdd(x, b))).  The tensor is
 // viewed as [outer, channels, inner]; channels-last inputs (inner == 1) take a
-// 128-bit path where the bias pack comes from L1, everything else a pack path
-// with one bias value per pack or an element-wise path.
+// 128-bit path with a thread's bias values in registers, everything else a pack
+// path with one bias value per pack or an element-wise path.
 //
 // Semantics follow the un-fused ops the chain replaces: BiasAdd
 // (musa_ext/kernels/nn/musa_biasadd_op.cc:23-61), Relu
@@ -12,7 +12,6 @@
 // (musa_ext/kernels/nn/musa_sigmoid_op.cc:18-35).
 #include "common.cuh"
 #include "trace.h"
-#include "tuning.h"
 #include "../../include/musa_plugin_kernels.h"
 
 namespace musa_b200 {
@@ -124,97 +123,115 @@ __device__ __forceinline__ Pack<T, kEpt> ActivatePack(const Pack<T, kEpt>& px,
   return out;
 }
 
-// Channels-last pack kernel.  Pack p of the flat tensor covers channels
-// [(p % cv) * kEpt, +kEpt); the column is tracked incrementally, no division
-// in the loop.
-template <typename T, int kEpt, int kUnroll, int kAct, bool kHasBias>
+// Activation without a bias: the tensor is one flat run of packs.
+template <typename T, int kEpt, int kAct>
 __global__ void __launch_bounds__(256)
-    BiasActLastKernel(const T* __restrict__ x, const T* __restrict__ bias,
-                      T* __restrict__ y, int64_t n_packs, int cv) {
+    ActivateFlatKernel(const T* __restrict__ x, T* __restrict__ y, int64_t n_packs) {
   using P = Pack<T, kEpt>;
-  constexpr bool kFast = sizeof(T) == 2;
+  constexpr int kUnroll = 4;
   const P* xp = reinterpret_cast<const P*>(x);
-  const P* bp = reinterpret_cast<const P*>(bias);
   P* yp = reinterpret_cast<P*>(y);
-  const int64_t tile = static_cast<int64_t>(blockDim.x) * kUnroll;
-  const int64_t n_tiles = (n_packs + tile - 1) / tile;
-  const int step = static_cast<int>(blockDim.x % cv);
-
-  // When the block width is a multiple of the row width in packs, a thread
-  // meets the same bias pack in every pack it handles: fetch it once.
-  const bool fixed_col = kHasBias && step == 0;
-  P fixed_bias;
-  if (fixed_col) fixed_bias = LoadKeep(bp + (threadIdx.x % cv));
-
-  for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-    const int64_t base = t * tile + threadIdx.x;
-    int col = fixed_col ? 0 : static_cast<int>(base % cv);
-    P px[kUnroll];
-    P pb[kUnroll];
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * (256 * kUnroll) + threadIdx.x;
+  P px[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-      if (i < n_packs) {
-        px[u] = LoadStream(xp + i);
-        if constexpr (kHasBias) {
-          if (fixed_col) {
-            pb[u] = fixed_bias;
-          } else {
-            pb[u] = LoadKeep(bp + col);
-          }
-        }
-      }
-      if (!fixed_col) {
-        col += step;
-        if (col >= cv) col -= cv;
-      }
-    }
+  for (int u = 0; u < kUnroll; ++u) {
+    if (base + u * 256 < n_packs) px[u] = LoadStream(xp + base + u * 256);
+  }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-      if (i < n_packs) {
-        StoreStream(yp + i, ActivatePack<T, kEpt, kAct, kHasBias>(px[u], pb[u]));
-      }
+  for (int u = 0; u < kUnroll; ++u) {
+    if (base + u * 256 < n_packs) {
+      StoreStream(yp + base + u * 256, ActivatePack<T, kEpt, kAct, false>(px[u], px[u]));
     }
   }
 }
 
-// Channels-last with a row of packs that divides the CTA width (channel counts
-// of 8 .. 2048 in fp16 / bf16 that are powers of two, and the like): with a grid
-// stride that is a multiple of the CTA width a thread meets the same bias pack
-// in every pack it handles.  It is fetched once, and the loop is nothing but
-// four loads, the math and four stores around two pointer bumps - the index
-// bookkeeping of the general kernel costs as many issue slots as a sigmoid.
-template <typename T, int kEpt, int kAct>
+// Channels-last rows of any length, the tensor read as one flat run of 128-bit
+// packs.  The channels that pack i covers repeat with a period of
+// C / gcd(C, kEpt) packs, so the run is cut into lines of a whole number of
+// periods and a CTA takes the same `width` columns of kLines neighbouring
+// lines: a thread meets the same kEpt channels in every pack it handles, their
+// bias values stay in registers, and what is left is kLines loads, the math and
+// kLines stores (the per-pack index bookkeeping of a general loop costs as many
+// issue slots as a sigmoid).
+//
+// Bound by HBM.  One tile of lines per CTA, not a persistent grid: the lines
+// of a tile lie in one DRAM neighbourhood, and a grid-wide stride instead (one
+// wave of CTAs, every pack of a thread 4.8 MB from the next) measured 95.9
+// against 79.9 us at fp32 [65536, 1024].  Swish, us per launch, against the
+// element form (rows that are not whole packs) or a pack form that looked its
+// bias pack up for every pack (rows of whole packs) before: fp32 [4096, 1001]
+// 17.2 -> 7.6, [65536, 1001] 212 -> 85 (81 at the copy rate); fp16
+// [4096, 1001] 14.5 -> 6.6; fp32 [16384, 1536] 56.8 -> 32.6, fp16 22.6 -> 17.5.
+template <typename T, int kEpt, int kAct, bool kWholeRows, int kLines>
 __global__ void __launch_bounds__(256)
-    BiasActFixedKernel(const T* __restrict__ x, const T* __restrict__ bias,
-                       T* __restrict__ y, int64_t n_packs, int cv) {
+    BiasActLinesKernel(const T* __restrict__ x, const T* __restrict__ bias,
+                       T* __restrict__ y, int64_t n, unsigned channels, unsigned line,
+                       unsigned width, unsigned segments) {
   using P = Pack<T, kEpt>;
-  const P pb = LoadKeep(reinterpret_cast<const P*>(bias) + (threadIdx.x % cv));
-  // A tile is 4 * 256 consecutive packs (16 KB): the four loads of a warp stay
-  // inside one DRAM neighbourhood.
-  const int64_t n_tiles = (n_packs + 1023) / 1024;
-  for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-    const int64_t base = t * 1024 + threadIdx.x;
-    const P* xp = reinterpret_cast<const P*>(x) + base;
-    P* yp = reinterpret_cast<P*>(y) + base;
-    if (base + 768 < n_packs) {
-      const P a0 = LoadStream(xp);
-      const P a1 = LoadStream(xp + 256);
-      const P a2 = LoadStream(xp + 512);
-      const P a3 = LoadStream(xp + 768);
-      StoreStream(yp, ActivatePack<T, kEpt, kAct, true>(a0, pb));
-      StoreStream(yp + 256, ActivatePack<T, kEpt, kAct, true>(a1, pb));
-      StoreStream(yp + 512, ActivatePack<T, kEpt, kAct, true>(a2, pb));
-      StoreStream(yp + 768, ActivatePack<T, kEpt, kAct, true>(a3, pb));
-    } else {
+  // The sigmoid chains of 16-bit rows that are not whole packs round once, as
+  // the element form does.
+  constexpr bool kPairs = kWholeRows || kAct == MUSA_ACT_IDENTITY || kAct == MUSA_ACT_RELU;
+  const int64_t n_packs = n / kEpt;
+  unsigned tile = blockIdx.x, col = threadIdx.x;
+  if (segments > 1) {
+    tile = blockIdx.x / segments;
+    col += (blockIdx.x - tile * segments) * width;
+  }
+  // Elements past the last whole pack.
+  if (!kWholeRows && blockIdx.x == gridDim.x - 1 && threadIdx.x < kEpt) {
+    const int64_t t = n_packs * kEpt + threadIdx.x;
+    if (t < n) {
+      y[t] = FromF32<T>(
+          Activate<kAct, sizeof(T) == 2>(ToF32(x[t]), ToF32(bias[t % channels])));
+    }
+  }
+  if (threadIdx.x >= width || col >= line) return;
+  const int64_t first = static_cast<int64_t>(tile) * (kLines * static_cast<int64_t>(line)) + col;
+  const P* xp = reinterpret_cast<const P*>(x) + first;
+  P* yp = reinterpret_cast<P*>(y) + first;
+  const int64_t step = line;
+  const bool whole = first + (kLines - 1) * step < n_packs;
+  P a[kLines];
+  if (whole) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (base + u * 256 < n_packs) {
-          StoreStream(yp + u * 256,
-                      ActivatePack<T, kEpt, kAct, true>(LoadStream(xp + u * 256), pb));
-        }
+    for (int u = 0; u < kLines; ++u) a[u] = LoadStream(xp + u * step);
+  } else {
+#pragma unroll
+    for (int u = 0; u < kLines; ++u) {
+      if (first + u * step < n_packs) a[u] = LoadStream(xp + u * step);
+    }
+  }
+  P pb;
+  if constexpr (kWholeRows) {
+    pb = LoadKeep(reinterpret_cast<const P*>(bias) + col % (channels / kEpt));
+  } else {
+    unsigned c = col * kEpt % channels;
+#pragma unroll
+    for (int e = 0; e < kEpt; ++e) {
+      pb.v[e] = bias[c];
+      c = c + 1 == channels ? 0 : c + 1;
+    }
+  }
+  const auto Apply = [&](const P& v) {
+    if constexpr (kPairs) {
+      return ActivatePack<T, kEpt, kAct, true>(v, pb);
+    } else {
+      P out;
+#pragma unroll
+      for (int e = 0; e < kEpt; ++e) {
+        out.v[e] = FromF32<T>(
+            Activate<kAct, sizeof(T) == 2>(ToF32(v.v[e]), ToF32(pb.v[e])));
       }
+      return out;
+    }
+  };
+  if (whole) {
+#pragma unroll
+    for (int u = 0; u < kLines; ++u) StoreStream(yp + u * step, Apply(a[u]));
+  } else {
+#pragma unroll
+    for (int u = 0; u < kLines; ++u) {
+      if (first + u * step < n_packs) StoreStream(yp + u * step, Apply(a[u]));
     }
   }
 }
@@ -337,6 +354,47 @@ int GridFor(int64_t work_items, int per_sm_cap) {
   return static_cast<int>(blocks);
 }
 
+// Lines of BiasActLinesKernel: as many whole channel periods as fit 256 packs,
+// or one period, cut into segments of equal width (at most 256 packs) where it
+// is longer.
+struct LinePlan {
+  unsigned line, width, segments;
+};
+LinePlan PlanLines(int64_t channels, int vec) {
+  int64_t period = channels;
+  for (int v = vec; v > 1 && period % 2 == 0; v >>= 1) period /= 2;
+  LinePlan p;
+  p.line = static_cast<unsigned>(period < 256 ? 256 / period * period : period);
+  p.segments = (p.line + 255) / 256;
+  p.width = (p.line + p.segments - 1) / p.segments;
+  return p;
+}
+
+template <typename T, int kAct, bool kWholeRows>
+int LaunchLines(const T* x, const T* bias, T* y, int64_t n, int64_t channels,
+                cudaStream_t stream) {
+  constexpr int kVec = VecWidth<T>::value;
+  const LinePlan p = PlanLines(channels, kVec);
+  const unsigned threads = (p.width + 31) / 32 * 32;
+  const int64_t lines = CeilDiv(n / kVec, p.line);
+  // Four lines a CTA where that still gives every SM four CTAs; below, one line
+  // a CTA, so that small tensors reach all SMs (fp32 [512, 256]: 2.8 us against
+  // 3.5 with four lines; with the line drawn at eight CTAs an SM, fp32
+  // [4096, 1024] takes 8.1 us with one line against 7.6 with four).
+  const auto Grid = [&](int per_cta) {
+    return GridFor(CeilDiv(lines, per_cta) * p.segments, 0);
+  };
+  if (Grid(4) >= 4 * SmCount()) {
+    BiasActLinesKernel<T, kVec, kAct, kWholeRows, 4><<<Grid(4), threads, 0, stream>>>(
+        x, bias, y, n, static_cast<unsigned>(channels), p.line, p.width, p.segments);
+  } else {
+    BiasActLinesKernel<T, kVec, kAct, kWholeRows, 1><<<Grid(1), threads, 0, stream>>>(
+        x, bias, y, n, static_cast<unsigned>(channels), p.line, p.width, p.segments);
+  }
+  CountKernelLaunch();
+  return static_cast<int>(cudaGetLastError());
+}
+
 template <typename T, int kAct, bool kHasBias>
 int LaunchTyped(const T* x, const T* bias, T* y, int64_t outer,
                 int64_t channels, int64_t inner, cudaStream_t stream) {
@@ -346,10 +404,8 @@ int LaunchTyped(const T* x, const T* bias, T* y, int64_t outer,
   if (!kHasBias && aligned && n >= kVec) {
     // Activation alone: the tensor is one flat run of packs plus a tail.
     const int64_t n_packs = n / kVec;
-    const int grid =
-        GridFor(CeilDiv(n_packs, 256 * 4), GetTuning(kTuneBiasActCtasPerSm));
-    BiasActLastKernel<T, kVec, 4, kAct, false>
-        <<<grid, 256, 0, stream>>>(x, bias, y, n_packs, 1);
+    ActivateFlatKernel<T, kVec, kAct>
+        <<<GridFor(CeilDiv(n_packs, 256 * 4), 0), 256, 0, stream>>>(x, y, n_packs);
     CountKernelLaunch();
     const int64_t done = n_packs * kVec;
     if (done < n) {
@@ -359,38 +415,15 @@ int LaunchTyped(const T* x, const T* bias, T* y, int64_t outer,
     }
     return static_cast<int>(cudaGetLastError());
   }
-  if (inner == 1 && channels % kVec == 0 && aligned &&
-      (!kHasBias || Aligned16(bias)) && channels / kVec <= 0x7fffffff) {
-    const int64_t n_packs = n / kVec;
-    const int cv = static_cast<int>(channels / kVec);
-    const int per_sm = GetTuning(kTuneBiasActCtasPerSm);
-    const int unroll = GetTuning(kTuneBiasActUnroll);
-    if constexpr (kHasBias) {
-      if (256 % cv == 0 && unroll != 2 && unroll != 8) {
-        const int grid = GridFor(CeilDiv(n_packs, 1024), per_sm);
-        BiasActFixedKernel<T, kVec, kAct>
-            <<<grid, 256, 0, stream>>>(x, bias, y, n_packs, cv);
-        CountKernelLaunch();
-        return static_cast<int>(cudaGetLastError());
+  if constexpr (kHasBias) {
+    if (inner == 1 && aligned && n >= kVec && channels < (1 << 28)) {
+      if (channels % kVec == 0 && Aligned16(bias)) {
+        return LaunchLines<T, kAct, true>(x, bias, y, n, channels, stream);
       }
+      return LaunchLines<T, kAct, false>(x, bias, y, n, channels, stream);
     }
-    if (unroll == 2) {
-      const int grid = GridFor(CeilDiv(n_packs, 256 * 2), per_sm);
-      BiasActLastKernel<T, kVec, 2, kAct, kHasBias>
-          <<<grid, 256, 0, stream>>>(x, bias, y, n_packs, cv);
-      CountKernelLaunch();
-    } else if (unroll == 8) {
-      const int grid = GridFor(CeilDiv(n_packs, 256 * 8), per_sm);
-      BiasActLastKernel<T, kVec, 8, kAct, kHasBias>
-          <<<grid, 256, 0, stream>>>(x, bias, y, n_packs, cv);
-      CountKernelLaunch();
-    } else {
-      const int grid = GridFor(CeilDiv(n_packs, 256 * 4), per_sm);
-      BiasActLastKernel<T, kVec, 4, kAct, kHasBias>
-          <<<grid, 256, 0, stream>>>(x, bias, y, n_packs, cv);
-      CountKernelLaunch();
-    }
-  } else if (inner % kVec == 0 && aligned) {
+  }
+  if (inner % kVec == 0 && aligned) {
     // Planes of whole packs: one bias value per pack.
     const int64_t n_packs = n / kVec;
     const int grid = GridFor(CeilDiv(n_packs, 256), 16);

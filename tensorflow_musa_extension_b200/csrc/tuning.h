@@ -8,8 +8,7 @@ namespace musa_b200 {
 enum TuningKey {
   kTuneAdamCtasPerSm = 0,   // 0: one tile per CTA; k: persistent, k CTAs per SM
   kTuneAdamUnroll = 1,      // packs in flight per thread and stream: 1, 2, 4
-  kTuneBiasActCtasPerSm = 2,
-  kTuneBiasActUnroll = 3,
+                            // 2, 3: not in use
   kTuneBnCtasPerSm = 4,     // CTAs per SM of the BatchNorm statistics grids; 0: what fits
   kTuneBnClusterFold = 5,   // CTAs per cluster of the stats kernel that fold their partial rows on chip
                             // (the element-wise kernel adds the rest: no finalize kernel); 0, 1: off

@@ -178,3 +178,22 @@ def test_sigmoid_quads_with_far_negative_members(kernel_lib, dtype):
     b = np.zeros(8, dt)
     sw = to_numpy(raw_ops.MusaBiasAddSwish(to_torch(x), to_torch(b)))
     assert_close(sw, np_ref.bias_add_swish(x, b), RTOL["lowp"], tiny * 1000, "swish")
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("rows,c", [(1, 9), (3, 257), (700, 130), (5, 1023), (9, 1025), (600, 1001),
+                                    (601, 1026), (40, 4104), (130, 2051), (2500, 86), (1200, 384)])
+def test_lines_of_any_row_length(kernel_lib, dtype, rows, c):
+    """Row lengths around the line and segment edges (one pack more and less
+    than 256 packs, several segments, a ragged last one), tails of less than a
+    pack, one and four lines per CTA; relu is exact, swish within the rounding
+    of its type."""
+    rng = np.random.default_rng(rows * c)
+    dt = np_dtype(dtype)
+    x = rng.standard_normal((rows, c)).astype(dt)
+    b = rng.normal(0, 0.1, c).astype(dt)
+    assert_close(to_numpy(raw_ops.MusaBiasAddRelu(to_torch(x), to_torch(b))),
+                 np_ref.bias_add_relu(x, b), 0)
+    rt, at = _tol(dtype)
+    assert_close(to_numpy(raw_ops.MusaBiasAddSwish(to_torch(x), to_torch(b))),
+                 np_ref.bias_add_swish(x, b), rt, at)
