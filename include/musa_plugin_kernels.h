@@ -98,6 +98,20 @@ void LaunchApplyAdamMixed_BFloat16(float* var, float* m, float* v,
                                    float beta2, float epsilon, int64_t n,
                                    bool use_nesterov, cudaStream_t stream);
 
+/* The same-type or mixed update of `count` variables that share their
+ * hyper-parameters, from HOST tables: var[i], m[i], v[i] are device pointers to
+ * sizes[i] values of `state_dtype`, grad[i] to sizes[i] values of `grad_dtype`
+ * (MUSA_DT_*; either equal, or fp16 / bf16 gradients beside fp32 state).  One
+ * launch for up to 128 variables; results are those of one launcher call per
+ * variable in list order (variables that share memory are updated one by one).
+ * No counterpart symbol in the reference, which launches per variable. */
+int LaunchApplyAdamGroupHostTable(int state_dtype, int grad_dtype, void* const* var,
+                                  void* const* m, void* const* v,
+                                  const void* const* grad, const int64_t* sizes,
+                                  int count, float lr_t, float beta1, float beta2,
+                                  float epsilon, bool use_nesterov,
+                                  cudaStream_t stream);
+
 /* ResourceApplyAdam / ApplyAdam for double tensors, one streaming pass
  * (56 B/element).  No launcher of this name exists in the reference: it serves
  * T = double with a chain of thirteen element-wise library calls

@@ -41,6 +41,8 @@ PROTOTYPES = {
     "LaunchApplyAdamMixed_Float": (None, _ADAM_SAME),
     "LaunchApplyAdamMixed_Half": (None, _ADAM_SAME),
     "LaunchApplyAdamMixed_BFloat16": (None, _ADAM_SAME),
+    "LaunchApplyAdamGroupHostTable":
+        (c_int, [c_int, c_int] + [c_vp] * 5 + [c_int] + [c_f32] * 4 + [c_bool, c_vp]),
     "LaunchApplyAdam_F64": (None, [c_vp, c_vp, c_vp, c_vp, c_f64, c_f64, c_f64, c_f64,
                                    c_i64, ctypes.c_bool, c_vp]),
     "LaunchBiasAct_F32": (c_int, _BIAS_ACT),

@@ -6,7 +6,9 @@
 // (musa_ext/kernels/training/musa_apply_sparse_adam_kernel.mu:140-157,
 //  musa_ext/kernels/training/musa_applyadam_bf16_kernel.mu:82-112,
 //  musa_ext/kernels/training/musa_applyadam_mixed_kernel.mu:55-86).
+#include <algorithm>
 #include <new>
+#include <vector>
 
 #include "common.cuh"
 #include "trace.h"
@@ -183,6 +185,196 @@ void LaunchAdam(StateT* var, StateT* m, StateT* v, const GradT* grad,
     LaunchWithNesterov<StateT, GradT, 1, 4>(var, m, v, grad, p, n, nesterov,
                                             stream);
   }
+}
+
+// ---- One step of many variables in one launch.  An optimizer step over a
+// model meets a few large and many small variables (biases, normalisation
+// parameters) with the same hyper-parameters: launched one by one, a variable
+// of a few hundred elements costs what one of 100,000 costs (about 2.5 us on the
+// device, more on the host), and every large one ends in a wave that is partly
+// empty.  Here the descriptors travel in the kernel's parameters and a CTA finds
+// its variable by bisection over the first tiles; a tile is what a CTA of
+// AdamKernel takes.  The 16 variables of an encoder block of width 768 (7.1 M
+// parameters, bf16 gradients): 63.7 us in 16 launches, 30.8 in one
+// (28.6 at the copy rate).
+constexpr int kAdamGroupMax = 128;
+struct AdamGroup {
+  void* var[kAdamGroupMax];
+  void* m[kAdamGroupMax];
+  void* v[kAdamGroupMax];
+  const void* grad[kAdamGroupMax];
+  int64_t n[kAdamGroupMax];
+  unsigned tile_begin[kAdamGroupMax + 1];   // first tile of each variable in the grid
+  int count;
+};
+
+template <typename StateT, typename GradT, bool kNesterov>
+__global__ void __launch_bounds__(256)
+    AdamGroupKernel(const __grid_constant__ AdamGroup g, AdamParams p) {
+  constexpr int kEpt = VecWidth<StateT>::value;
+  constexpr int kUnroll = 2;
+  constexpr int kTile = 256 * kUnroll * kEpt;
+  using SPack = Pack<StateT, kEpt>;
+  using GPack = Pack<GradT, kEpt>;
+  int k = 0, hi = g.count;
+  while (k + 1 < hi) {
+    const int mid = (k + hi) / 2;
+    if (g.tile_begin[mid] <= blockIdx.x) {
+      k = mid;
+    } else {
+      hi = mid;
+    }
+  }
+  const int64_t n = g.n[k];
+  const int64_t begin = static_cast<int64_t>(blockIdx.x - g.tile_begin[k]) * kTile;
+  StateT* var = static_cast<StateT*>(g.var[k]) + begin;
+  StateT* m = static_cast<StateT*>(g.m[k]) + begin;
+  StateT* v = static_cast<StateT*>(g.v[k]) + begin;
+  const GradT* grad = static_cast<const GradT*>(g.grad[k]) + begin;
+  const int left = n - begin < kTile ? static_cast<int>(n - begin) : kTile;
+  // A tile starts a multiple of the pack width into the variable, so it is
+  // aligned where the variable is.
+  const bool vec = ((reinterpret_cast<uintptr_t>(var) | reinterpret_cast<uintptr_t>(m) |
+                     reinterpret_cast<uintptr_t>(v)) & 15u) == 0 &&
+                   reinterpret_cast<uintptr_t>(grad) % (sizeof(GradT) * kEpt) == 0;
+  const auto Element = [&](int i) {
+    float fvar = ToF32(var[i]), fm = ToF32(m[i]), fv = ToF32(v[i]);
+    AdamStep<kNesterov>(fvar, fm, fv, ToF32(grad[i]), p);
+    var[i] = FromF32<StateT>(fvar);
+    m[i] = FromF32<StateT>(fm);
+    v[i] = FromF32<StateT>(fv);
+  };
+  if (!vec) {
+    for (int i = threadIdx.x; i < left; i += 256) Element(i);
+    return;
+  }
+  const int packs = left / kEpt;
+  SPack pv[kUnroll], pm[kUnroll], pvv[kUnroll];
+  GPack pg[kUnroll];
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const int i = threadIdx.x + u * 256;
+    if (i < packs) {
+      pg[u] = LoadStream(reinterpret_cast<const GPack*>(grad) + i);
+      pm[u] = LoadStream(reinterpret_cast<const SPack*>(m) + i);
+      pvv[u] = LoadStream(reinterpret_cast<const SPack*>(v) + i);
+      pv[u] = LoadStream(reinterpret_cast<const SPack*>(var) + i);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const int i = threadIdx.x + u * 256;
+    if (i < packs) {
+#pragma unroll
+      for (int e = 0; e < kEpt; ++e) {
+        float fvar = ToF32(pv[u].v[e]), fm = ToF32(pm[u].v[e]), fv = ToF32(pvv[u].v[e]);
+        AdamStep<kNesterov>(fvar, fm, fv, ToF32(pg[u].v[e]), p);
+        pv[u].v[e] = FromF32<StateT>(fvar);
+        pm[u].v[e] = FromF32<StateT>(fm);
+        pvv[u].v[e] = FromF32<StateT>(fv);
+      }
+      StoreStream(reinterpret_cast<SPack*>(m) + i, pm[u]);
+      StoreStream(reinterpret_cast<SPack*>(v) + i, pvv[u]);
+      StoreStream(reinterpret_cast<SPack*>(var) + i, pv[u]);
+    }
+  }
+  const int tail = packs * kEpt + threadIdx.x;
+  if (threadIdx.x < kEpt && tail < left) Element(tail);
+}
+
+// Whether two variables of the list share memory that one of them writes: the
+// updates then have to run one after the other.
+bool AdamGroupOverlaps(void* const* var, void* const* m, void* const* v,
+                       const void* const* grad, const int64_t* sizes, int count,
+                       size_t state_bytes, size_t grad_bytes) {
+  struct Span {
+    uintptr_t begin, end;
+    bool write;
+  };
+  std::vector<Span> spans;
+  spans.reserve(4 * static_cast<size_t>(count));
+  for (int i = 0; i < count; ++i) {
+    if (sizes[i] <= 0) continue;
+    const size_t sb = state_bytes * static_cast<size_t>(sizes[i]);
+    for (const void* q : {static_cast<const void*>(var[i]), static_cast<const void*>(m[i]),
+                          static_cast<const void*>(v[i])}) {
+      spans.push_back({reinterpret_cast<uintptr_t>(q), reinterpret_cast<uintptr_t>(q) + sb, true});
+    }
+    const auto g = reinterpret_cast<uintptr_t>(grad[i]);
+    spans.push_back({g, g + grad_bytes * static_cast<size_t>(sizes[i]), false});
+  }
+  std::sort(spans.begin(), spans.end(),
+            [](const Span& a, const Span& b) { return a.begin < b.begin; });
+  uintptr_t end_any = 0, end_write = 0;   // of the spans that begin earlier
+  for (const Span& s : spans) {
+    if (s.begin < (s.write ? end_any : end_write)) return true;
+    end_any = std::max(end_any, s.end);
+    if (s.write) end_write = std::max(end_write, s.end);
+  }
+  return false;
+}
+
+template <typename StateT, typename GradT>
+int LaunchAdamGroup(void* const* var, void* const* m, void* const* v,
+                    const void* const* grad, const int64_t* sizes, int count, float lr_t,
+                    float beta1, float beta2, float epsilon, bool nesterov,
+                    cudaStream_t stream) {
+  int64_t total = 0;
+  for (int i = 0; i < count; ++i) {
+    if (sizes[i] < 0) return MUSA_KERNELS_EINVAL;
+    if (sizes[i] > 0 && (!var[i] || !m[i] || !v[i] || !grad[i])) return MUSA_KERNELS_EINVAL;
+    total += sizes[i];
+  }
+  MUSA_TRACE("LaunchApplyAdamGroup", (6 * sizeof(StateT) + sizeof(GradT)) * total);
+  if (AdamGroupOverlaps(var, m, v, grad, sizes, count, sizeof(StateT), sizeof(GradT))) {
+    for (int i = 0; i < count; ++i) {
+      LaunchAdam<StateT, GradT>(static_cast<StateT*>(var[i]), static_cast<StateT*>(m[i]),
+                                static_cast<StateT*>(v[i]), static_cast<const GradT*>(grad[i]),
+                                lr_t, beta1, beta2, epsilon, sizes[i], nesterov, stream);
+    }
+    return static_cast<int>(cudaGetLastError());
+  }
+  AdamParams p;
+  p.lr_t = lr_t;
+  p.beta1 = beta1;
+  p.one_minus_b1 = 1.0f - beta1;
+  p.beta2 = beta2;
+  p.one_minus_b2 = 1.0f - beta2;
+  p.epsilon = epsilon;
+  constexpr int64_t kTile = 256 * 2 * VecWidth<StateT>::value;
+  int next = 0;
+  while (next < count) {
+    AdamGroup g;
+    g.count = 0;
+    int64_t tiles = 0;
+    for (; next < count && g.count < kAdamGroupMax; ++next) {
+      const int64_t n = sizes[next];
+      if (n == 0) continue;
+      const int64_t t = CeilDiv(n, kTile);
+      if (tiles + t > 0x7fffffffLL) {
+        if (g.count == 0) return MUSA_KERNELS_ETOOLARGE;
+        break;   // this variable opens the next launch
+      }
+      g.var[g.count] = var[next];
+      g.m[g.count] = m[next];
+      g.v[g.count] = v[next];
+      g.grad[g.count] = grad[next];
+      g.n[g.count] = n;
+      g.tile_begin[g.count] = static_cast<unsigned>(tiles);
+      tiles += t;
+      ++g.count;
+    }
+    if (g.count == 0) break;
+    g.tile_begin[g.count] = static_cast<unsigned>(tiles);
+    const dim3 grid(static_cast<unsigned>(tiles));
+    if (nesterov) {
+      AdamGroupKernel<StateT, GradT, true><<<grid, 256, 0, stream>>>(g, p);
+    } else {
+      AdamGroupKernel<StateT, GradT, false><<<grid, 256, 0, stream>>>(g, p);
+    }
+    CountKernelLaunch();
+  }
+  return static_cast<int>(cudaGetLastError());
 }
 
 // ---- Range-sharded Adam whose update IS the all-gather: a replica updates
@@ -412,6 +604,29 @@ void LaunchApplyAdamSameType_Half(void* var, void* m, void* v, const void* grad,
                              static_cast<__half*>(v),
                              static_cast<const __half*>(grad), lr_t, beta1,
                              beta2, epsilon, n, use_nesterov, stream);
+}
+
+int LaunchApplyAdamGroupHostTable(int state_dtype, int grad_dtype, void* const* var,
+                                  void* const* m, void* const* v, const void* const* grad,
+                                  const int64_t* sizes, int count, float lr_t, float beta1,
+                                  float beta2, float epsilon, bool use_nesterov,
+                                  cudaStream_t stream) {
+  if (count < 0) return MUSA_KERNELS_EINVAL;
+  if (count == 0) return MUSA_KERNELS_OK;
+  if (!var || !m || !v || !grad || !sizes) return MUSA_KERNELS_EINVAL;
+#define MUSA_ADAM_GROUP(S, G)                                                              \
+  return LaunchAdamGroup<S, G>(var, m, v, grad, sizes, count, lr_t, beta1, beta2, epsilon, \
+                               use_nesterov, stream)
+  if (state_dtype == MUSA_DT_F32) {
+    if (grad_dtype == MUSA_DT_F32) MUSA_ADAM_GROUP(float, float);
+    if (grad_dtype == MUSA_DT_F16) MUSA_ADAM_GROUP(float, __half);
+    if (grad_dtype == MUSA_DT_BF16) MUSA_ADAM_GROUP(float, __nv_bfloat16);
+  } else if (state_dtype == grad_dtype) {
+    if (state_dtype == MUSA_DT_F16) MUSA_ADAM_GROUP(__half, __half);
+    if (state_dtype == MUSA_DT_BF16) MUSA_ADAM_GROUP(__nv_bfloat16, __nv_bfloat16);
+  }
+#undef MUSA_ADAM_GROUP
+  return MUSA_KERNELS_EUNSUPPORTED;
 }
 
 int LaunchAdamShardBroadcastFloat(float* const* var_replicas, int world, int rank,

@@ -12,6 +12,8 @@ the same hyper-parameters, slot names ("m", "v") and dispatch:
   amsgrad=True                                 -> rejected (the reference falls
                                                   back to stock Keras there)
 """
+import ctypes
+
 import torch
 
 from . import raw_ops
@@ -31,7 +33,8 @@ def apply_adam_mixed(var, m, v, beta1_power, beta2_power, lr, beta1, beta2,
 
 
 class MusaAdam:
-    """Adam over device tensors, one fused kernel per variable and step."""
+    """Adam over device tensors: one fused launch for neighbouring variables of
+    one state and gradient type."""
 
     _LOWP_GRAD_DTYPES = (torch.float32, torch.bfloat16, torch.float16)
 
@@ -58,27 +61,76 @@ class MusaAdam:
             self._slots[key] = {"m": torch.zeros_like(t), "v": torch.zeros_like(t)}
         return self._slots[key][slot_name]
 
+    def _groupable(self, t, m, v, grad):
+        """Whether the update can share a launch with its neighbours: device
+        tensors in the form that the op hands to its kernel as they are.
+        Everything else (host gradients, wrong shapes or types) goes through
+        the op, which converts or refuses."""
+        return (isinstance(grad, torch.Tensor) and isinstance(t, torch.Tensor)
+                and t.is_cuda and grad.is_cuda and grad.device == t.device
+                and (t.dtype == torch.float32 and grad.dtype in self._LOWP_GRAD_DTYPES
+                     or t.dtype == grad.dtype and t.dtype in self._LOWP_GRAD_DTYPES)
+                and m.dtype == t.dtype and v.dtype == t.dtype
+                and t.shape == grad.shape and t.shape == m.shape and t.shape == v.shape
+                and t.is_contiguous() and grad.is_contiguous()
+                and m.is_contiguous() and v.is_contiguous())
+
+    def _apply_group(self, group, b1p, b2p):
+        """One launch for consecutive variables of one device, state type and
+        gradient type; the scalars are read as the ops read them."""
+        t, grad = group[0][0], group[0][3]
+        sc = [raw_ops._scalar_in(x, t.dtype) for x in (
+            self.learning_rate, b1p, b2p, self.beta_1, self.beta_2, self.epsilon)]
+        n = len(group)
+        tables = [(ctypes.c_void_p * n)(*[q[k].data_ptr() for q in group]) for k in range(4)]
+        sizes = (ctypes.c_int64 * n)(*[q[0].numel() for q in group])
+        with torch.cuda.device(t.device):
+            rc = raw_ops._lib().LaunchApplyAdamGroupHostTable(
+                raw_ops._DT_CODE[t.dtype], raw_ops._DT_CODE[grad.dtype], *tables, sizes, n,
+                raw_ops._adam_alpha(*sc[:3]), sc[3], sc[4], sc[5], self.use_nesterov,
+                raw_ops._stream())
+        raw_ops._check(rc, "MusaAdam")
+
     def apply_gradients(self, grads_and_vars):
-        """One step over (grad, var) pairs; returns the new iteration count."""
+        """One step over (grad, var) pairs; returns the new iteration count.
+        Neighbouring variables of one kind are updated by one launch."""
         step = self.iterations + 1
         b1p = self.beta_1 ** step
         b2p = self.beta_2 ** step
-        for grad, var in grads_and_vars:
-            if grad is None:
-                continue
-            t = var.tensor() if isinstance(var, raw_ops.Variable) else var
-            m = self.get_slot(var, "m")
-            v = self.get_slot(var, "v")
-            if t.dtype == torch.float32:
-                if grad.dtype not in self._LOWP_GRAD_DTYPES:
-                    raise InvalidArgumentError(
-                        "MusaAdam: unsupported grad dtype %s" % (grad.dtype,))
-                raw_ops.MusaResourceApplyAdamMixed(
-                    t, m, v, b1p, b2p, self.learning_rate, self.beta_1, self.beta_2,
-                    self.epsilon, grad, use_nesterov=self.use_nesterov)
-            else:
-                raw_ops.ResourceApplyAdam(
-                    t, m, v, b1p, b2p, self.learning_rate, self.beta_1, self.beta_2,
-                    self.epsilon, grad, use_nesterov=self.use_nesterov)
+        group, kind = [], None
+
+        def flush():
+            nonlocal group
+            pending, group = group, []
+            if pending:
+                self._apply_group(pending, b1p, b2p)
+
+        try:
+            for grad, var in grads_and_vars:
+                if grad is None:
+                    continue
+                t = var.tensor() if isinstance(var, raw_ops.Variable) else var
+                m = self.get_slot(var, "m")
+                v = self.get_slot(var, "v")
+                if self._groupable(t, m, v, grad):
+                    if kind != (t.device, t.dtype, grad.dtype):
+                        flush()
+                        kind = (t.device, t.dtype, grad.dtype)
+                    group.append((t, m, v, grad))
+                    continue
+                flush()
+                if t.dtype == torch.float32:
+                    if grad.dtype not in self._LOWP_GRAD_DTYPES:
+                        raise InvalidArgumentError(
+                            "MusaAdam: unsupported grad dtype %s" % (grad.dtype,))
+                    raw_ops.MusaResourceApplyAdamMixed(
+                        t, m, v, b1p, b2p, self.learning_rate, self.beta_1, self.beta_2,
+                        self.epsilon, grad, use_nesterov=self.use_nesterov)
+                else:
+                    raw_ops.ResourceApplyAdam(
+                        t, m, v, b1p, b2p, self.learning_rate, self.beta_1, self.beta_2,
+                        self.epsilon, grad, use_nesterov=self.use_nesterov)
+        finally:
+            flush()   # an error leaves the variables before it updated
         self.iterations = step
         return step

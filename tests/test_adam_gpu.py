@@ -454,3 +454,55 @@ def test_multicast_transport_refuses_what_it_cannot_run(kernel_lib):
              st) == 0
     torch.cuda.synchronize()
     assert not t.any()
+
+
+@pytest.mark.parametrize("state,grad_dtype", [("float32", "float32"), ("float32", "bfloat16"),
+                                              ("float32", "float16"), ("bfloat16", "bfloat16"),
+                                              ("float16", "float16")])
+@pytest.mark.parametrize("nesterov", [False, True])
+def test_musa_adam_group_equals_one_op_per_variable(kernel_lib, state, grad_dtype, nesterov):
+    """Many variables in one launch: the bits of one op call per variable, for
+    sizes around a tile (2048 fp32, 4096 16-bit values), a variable that is not
+    16-byte aligned, an empty one, more variables than one launch holds, and
+    variables that share memory (updated one after the other)."""
+    from tensorflow_musa_extension_b200.optimizers import MusaAdam
+    sizes = [1, 3, 2047, 2048, 2049, 4095, 4096, 4097, 0, 70001] + [17] * 130
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    dt, gdt = getattr(torch, state), getattr(torch, grad_dtype)
+
+    def normal(n, std, d):
+        return (torch.randn(n, device="cuda", generator=gen) * std).to(d)
+
+    pool = normal(5000, 0.05, dt)
+    pools = (pool, pool.clone())            # one for each way of updating
+
+    def variables(k):
+        views = [pools[k][1:1001], pools[k][500:2000], pools[k][500:2000]]   # unaligned, overlapping
+        return [x.clone() for x in base] + views
+
+    base = [normal(n, 0.05, dt) for n in sizes]
+    grads = [normal(n, 1e-3, gdt) for n in sizes] + [normal(n, 1e-3, gdt)
+                                                      for n in (1000, 1500, 1500)]
+    one, many = variables(0), variables(1)
+    opt = MusaAdam(use_nesterov=nesterov)
+    ms = [torch.zeros_like(t) for t in one]
+    vs = [torch.zeros_like(t) for t in one]
+    op = raw_ops.MusaResourceApplyAdamMixed if state == "float32" else raw_ops.ResourceApplyAdam
+    for step in (1, 2):
+        opt.apply_gradients(list(zip(grads, many)))
+        for t, m, v, g in zip(one, ms, vs, grads):
+            op(t, m, v, 0.9 ** step, 0.999 ** step, 1e-3, 0.9, 0.999, 1e-7, g,
+               use_nesterov=nesterov)
+    for t, m, v, u in zip(one, ms, vs, many):
+        assert torch.equal(t, u)
+        assert torch.equal(m, opt.get_slot(u, "m")) and torch.equal(v, opt.get_slot(u, "v"))
+
+
+def test_musa_adam_error_keeps_earlier_updates(kernel_lib):
+    from tensorflow_musa_extension_b200.optimizers import MusaAdam
+    a, b = torch.ones(10, device="cuda"), torch.ones(10, device="cuda")
+    opt = MusaAdam()
+    with pytest.raises(errors.InvalidArgumentError, match="same shape"):
+        opt.apply_gradients([(torch.ones(10, device="cuda"), a), (torch.ones(9, device="cuda"), b)])
+    assert not torch.equal(a, torch.ones_like(a)) and torch.equal(b, torch.ones_like(b))
+    assert opt.iterations == 0
