@@ -632,6 +632,28 @@ int LaunchBnFinalizeFromSums(const float* sums, double total_count,
                              float* saved_mean, float* saved_var,
                              int64_t channels, float exp_avg_factor,
                              cudaStream_t stream);
+/* FusedBatchNormV3 / FusedBatchNormGradV3 with every output written by the op's
+ * own kernels, for any dtype code.  As LaunchBnFwdTrain_*, LaunchBnFwdInfer_*
+ * and LaunchBnGrad_*, and beside them: `reserve_3` (one float, may be NULL) and
+ * `reserve_4`, `reserve_5` ([channels], may be NULL) receive zeros; the
+ * inference form copies est_mean / est_var to the four statistics outputs.
+ * Empty inputs return without a launch and write nothing. */
+int LaunchBnFwdTrainOp(int dtype, const void* x, const float* scale, const float* offset,
+                       const float* est_mean, const float* est_var, void* y, float* batch_mean,
+                       float* batch_var, float* saved_mean, float* saved_var, float* reserve_3,
+                       int64_t outer, int64_t channels, int64_t inner, float epsilon,
+                       float exp_avg_factor, void* workspace, size_t workspace_bytes,
+                       cudaStream_t stream);
+int LaunchBnFwdInferOp(int dtype, const void* x, const float* scale, const float* offset,
+                       const float* est_mean, const float* est_var, void* y, float* batch_mean,
+                       float* batch_var, float* saved_mean, float* saved_var, float* reserve_3,
+                       int64_t outer, int64_t channels, int64_t inner, float epsilon,
+                       cudaStream_t stream);
+int LaunchBnGradOp(int dtype, const void* dy, const void* x, const float* scale,
+                   const float* mean, const float* variance, void* dx, float* dscale,
+                   float* doffset, float* reserve_4, float* reserve_5, int64_t outer,
+                   int64_t channels, int64_t inner, float epsilon, bool is_training,
+                   void* workspace, size_t workspace_bytes, cudaStream_t stream);
 /* y = (x - mean) * rsqrt(var + eps) * scale + offset (same as inference). */
 int LaunchBnApply(int dtype, const void* x, const float* scale,
                   const float* offset, const float* mean, const float* variance,

@@ -109,6 +109,13 @@ PROTOTYPES = {
     "LaunchBnGrad_F32": (c_int, _BN_GRAD),
     "LaunchBnGrad_F16": (c_int, _BN_GRAD),
     "LaunchBnGrad_BF16": (c_int, _BN_GRAD),
+    "LaunchBnFwdTrainOp":
+        (c_int, [c_int] + [c_vp] * 11 + [c_i64, c_i64, c_i64, c_f32, c_f32, c_vp, c_size, c_vp]),
+    "LaunchBnFwdInferOp":
+        (c_int, [c_int] + [c_vp] * 11 + [c_i64, c_i64, c_i64, c_f32, c_vp]),
+    "LaunchBnGradOp":
+        (c_int, [c_int] + [c_vp] * 10
+         + [c_i64, c_i64, c_i64, c_f32, c_bool, c_vp, c_size, c_vp]),
     "BnNoAllocMaxChannels": (c_size, []),
     "LaunchBnFwdTrainNoAlloc":
         (c_int, [c_int] + [c_vp] * 10 + [c_i64, c_i64, c_i64, c_f32, c_f32, c_vp]),

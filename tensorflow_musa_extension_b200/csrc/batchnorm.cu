@@ -284,6 +284,12 @@ struct FinalizeArgs {
   // and everything it writes is the result over all replicas.
   const ExchangeDev* xchg;
   unsigned* xchg_epoch;   // the exchange's epoch counter (advanced by the statistics kernel)
+  // Outputs of the op that hold zeros, written beside the statistics instead of
+  // by fill launches (2 us each on the device, about 5 us on the host): one
+  // float (forward: reserve_space_3) and up to two [C] vectors (gradient:
+  // reserve_space_4 / _5).  NULL: none.
+  float* zero_scalar;
+  float* zero_vec[2];
 };
 
 __device__ __forceinline__ float LoadAsF32(const void* base, int dtype,
@@ -293,8 +299,25 @@ __device__ __forceinline__ float LoadAsF32(const void* base, int dtype,
   return __bfloat162float(static_cast<const __nv_bfloat16*>(base)[i]);
 }
 
+__device__ __forceinline__ void WriteZeros(const FinalizeArgs& a, int64_t c) {
+  if (a.zero_scalar != nullptr && c == 0) *a.zero_scalar = 0.0f;
+  if (a.zero_vec[0] != nullptr) a.zero_vec[0][c] = 0.0f;
+  if (a.zero_vec[1] != nullptr) a.zero_vec[1][c] = 0.0f;
+}
+
+// Inference: the op passes the given statistics through as its outputs.
+__device__ __forceinline__ void WriteGivenStats(const FinalizeArgs& a, int64_t c, float mean,
+                                                float var) {
+  a.batch_mean[c] = mean;
+  a.batch_var[c] = var;
+  a.saved_mean[c] = mean;
+  a.saved_var[c] = var;
+  WriteZeros(a, c);
+}
+
 __device__ __forceinline__ void WriteFwdStats(const FinalizeArgs& a, int64_t c,
                                               double mean, double var) {
+  WriteZeros(a, c);
   if (var < 0.0) var = 0.0;
   // bessel = R / (R - 1), or 1 when there is one value per channel; taken on
   // the host (an fp64 divide per thread is not free on the device).
@@ -456,17 +479,15 @@ __global__ void __launch_bounds__(kThreads)
   };
 
   if (active) {
+    // The shift is requested here and first used (a wait of one memory round
+    // trip) after the prologue's copies are on their way.
+    P first;
+    float mean_c[kVec];
     if constexpr (kMode == kFwd) {
-      const P first = LoadKeep(reinterpret_cast<const P*>(x) + col);
-      WidenPack<kVec>(first, nshift);
-#pragma unroll
-      for (int q = 0; q < kPairs; ++q) nshift[q] = Neg2(nshift[q]);
+      first = LoadKeep(reinterpret_cast<const P*>(x) + col);
     } else {
 #pragma unroll
-      for (int q = 0; q < kPairs; ++q) {
-        nshift[q] = make_float2(-mean[col * kVec + 2 * q],
-                                -mean[col * kVec + 2 * q + 1]);
-      }
+      for (int e = 0; e < kVec; ++e) mean_c[e] = __ldg(mean + col * kVec + e);
     }
     // This thread's rows: r0 + ty + j * TY, j = 0 .. n_j - 1 (32-bit counters:
     // a CTA never owns 2^31 rows), in n_full whole stages of kU rows and a
@@ -564,6 +585,16 @@ __global__ void __launch_bounds__(kThreads)
         ++s_issue;
       }
       CpAsyncCommit();
+    }
+    if constexpr (kMode == kFwd) {
+      WidenPack<kVec>(first, nshift);
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) nshift[q] = Neg2(nshift[q]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        nshift[q] = make_float2(-mean_c[2 * q], -mean_c[2 * q + 1]);
+      }
     }
     unsigned fill = (kStages - 1) * kStageBytes;   // ring offset of the next stage to fill
     unsigned drain = 0;                            // ring offset of the next stage to read
@@ -1064,6 +1095,7 @@ __global__ void __launch_bounds__(8 * kLanes) BnFinalizeKernel(FinalizeArgs a) {
           a.sums[c] = s1_f;
           a.sums[a.channels + c] = s2_f;
         }
+        WriteZeros(a, c);
         if (a.doffset) a.doffset[c] = s1_f;
         if (a.dscale) {
           const float inv = 1.0f / sqrtf(a.variance[c] + a.epsilon);
@@ -1184,14 +1216,21 @@ struct ApplyArgs {
   const float* fold_rows;
   int fold_n;
   bool fold_use;
+  // Inference forward: the first row of CTAs copies mean / variance to the four
+  // statistics outputs of stat_out (and writes its zeros).
+  bool pass_stats;
 };
 
+// CTAs per SM that the registers are held to: the fp32 gradient fits three
+// (80 registers), the 16-bit forms with their eight channels a thread two, the
+// element form the four that its launch assumes.
 template <typename T, int kVec, int kUnroll, int kMode>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kVec == 1 ? 4 : sizeof(T) == 4 && kUnroll == 4 ? 3 : 2)
     BnApplyLastKernel(const T* __restrict__ x, const T* __restrict__ dy,
                       T* __restrict__ out, ApplyArgs a, int64_t rows,
                       int64_t cv, int64_t channels, int64_t rows_per_cta,
-                      bool reverse, bool last_use, bool early_loads, bool interleave) {
+                      bool reverse, bool last_use, bool early_loads, bool early_inputs,
+                      bool interleave) {
   using P = Pack<T, kVec>;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int TX = blockDim.x, TY = blockDim.y;
@@ -1270,22 +1309,42 @@ __global__ void __launch_bounds__(kThreads)
   // first.
   const bool active = col < cv;
   if (early_loads && active) load_batch(ty, 0);
-  // The shift of the shifted sums (first row of x: an input of the op, like
-  // the early rows).
-  P first_row;
-  if (kMode == kFwd && a.fold_rows != nullptr && active) first_row = LoadKeep(xp);
+  // Prologue: the coefficients of the CTA's nch channels, ONE channel per
+  // thread, meet in shared memory; every thread then picks up those of its pack.
+  // (Each thread used to form all kVec channels of its pack: with the loads
+  // spread over the branches that was a chain of kVec memory round trips and
+  // kVec square roots and divisions on every thread.  Inference on 0.4 MB 7.5 ->
+  // 5.4 us, fp16 [200704,256] forward 33.4 -> 30.6, gradient 48.4 -> 46.0.)  `early_inputs`: the whole op is one launcher
+  // call, so its per-channel inputs are as final as x and are requested before
+  // the wait too.
+  extern __shared__ __align__(16) float apply_smem[];   // coefficients [4][nch], fold rows
+  __shared__ double s_tot[2][kThreads];   // fold: TX * kVec <= kThreads (the launcher sees to it)
+  const int tid = ty * TX + tx;
+  const int nch = TX * kVec;
+  const int64_t c0 = static_cast<int64_t>(blockIdx.x) * nch;
+  const int seg = channels - c0 < nch ? static_cast<int>(channels - c0) : nch;
+  float* const fold_smem = apply_smem + 4 * nch;   // [fold_n][2][nch]
+  const bool fold = a.fold_rows != nullptr;
+  const bool own_stats = kMode == kFwd && (fold || a.stat_sums != nullptr);
+  float scale_c = 0.0f, offset_c = 0.0f, mean_c = 0.0f, var_c = 0.0f, shift_c = 0.0f;
+  auto load_inputs = [&](int64_t c) {
+    scale_c = a.scale[c];
+    if constexpr (kMode == kFwd) {
+      offset_c = a.offset[c];
+      // The shift of the shifted sums: the first row of x.
+      if (fold) shift_c = ToF32(x[c]);
+    } else {
+      mean_c = a.mean[c];
+      var_c = a.variance[c];
+    }
+  };
+  if (early_inputs && tid < seg) load_inputs(c0 + tid);
   GridDepWait();
   GridDepLaunch();
   // Second level of the reduction when no finalize kernel ran (fold_rows):
   // the CTA fetches the partial rows of its own channels into shared memory
-  // with one round of 16-byte copies and adds them in fp64, in row order.
-  extern __shared__ __align__(16) float fold_smem[];   // [fold_n][2][TX * kVec]
-  __shared__ double s_tot[2][kThreads];     // TX * kVec <= kThreads (the launcher sees to it)
-  if (a.fold_rows != nullptr) {
-    const int tid = ty * TX + tx;
-    const int nch = TX * kVec;
-    const int64_t c0 = static_cast<int64_t>(blockIdx.x) * nch;
-    const int seg = channels - c0 < nch ? static_cast<int>(channels - c0) : nch;
+  // with one round of 16-byte copies and adds them in fp64, in a fixed order.
+  if (fold) {
     if constexpr (kVec >= 4) {
       const int per_seg = seg / 4;                       // 16-byte copies per row segment
       const int copies = a.fold_n * 2 * per_seg;
@@ -1302,92 +1361,103 @@ __global__ void __launch_bounds__(kThreads)
       const int which = o / nch, ch = o - which * nch;
       double acc = 0.0;
       if (ch < seg) {
-        for (int r = 0; r < a.fold_n; ++r) {
-          acc += static_cast<double>(fold_smem[(r * 2 + which) * nch + ch]);
+        // Four chains of adds (rows r, r + 4, ...), joined in order.
+        double part[4] = {0.0, 0.0, 0.0, 0.0};
+        const float* at = fold_smem + which * nch + ch;
+        int r = 0;
+        for (; r + 4 <= a.fold_n; r += 4) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) part[q] += static_cast<double>(at[(r + q) * 2 * nch]);
         }
+        for (; r < a.fold_n; ++r) part[0] += static_cast<double>(at[r * 2 * nch]);
+        acc = (part[0] + part[1]) + (part[2] + part[3]);
       }
       s_tot[which][ch] = acc;
     }
     __syncthreads();
   }
-  if (!active) return;
 
   // 16-bit outputs round to 8 or 11 bits, so the per-channel affine forms are
   // folded to two (forward) or three (gradient) coefficients and one or two
   // FMAs per element; fp32 keeps the centred form (x - mean) to the end.
   constexpr bool kFold = sizeof(T) == 2;
-  const bool writer = blockIdx.y == 0 && ty == 0;
-  float mean[kVec], ca[kVec], cb[kVec], cc[kVec];
-#pragma unroll
-  for (int e = 0; e < kVec; ++e) {
-    const int64_t c = col * kVec + e;
-    float var_c;
-    if (kMode == kFwd && a.fold_rows != nullptr) {
-      // Shifted sums (the statistics kernel subtracted the first row).
-      const double K = static_cast<double>(ToF32(first_row.v[e]));
-      const double md = s_tot[0][tx * kVec + e] * a.stat_out.inv_count;
-      const double m = K + md;
-      double v = s_tot[1][tx * kVec + e] * a.stat_out.inv_count - md * md;
-      if (v < 0.0) v = 0.0;
-      mean[e] = static_cast<float>(m);
-      var_c = static_cast<float>(v);
-      if (writer) WriteFwdStats(a.stat_out, c, m, v);
-    } else if (kMode == kFwd && a.stat_sums != nullptr) {
-      double m, v;
-      if (a.stat_moments) {
-        m = static_cast<double>(a.stat_sums[c]);
-        v = static_cast<double>(a.stat_sums[channels + c]) * a.stat_out.inv_count;
+  const bool writer = blockIdx.y == 0;
+  for (int ch = tid; ch < seg; ch += kThreads) {
+    const int64_t c = c0 + ch;
+    if (!early_inputs || ch != tid) load_inputs(c);
+    if constexpr (kMode == kFwd) {
+      if (own_stats) {
+        double m, v;
+        if (fold) {
+          // Shifted sums (the statistics kernel subtracted the first row).
+          const double md = s_tot[0][ch] * a.stat_out.inv_count;
+          m = static_cast<double>(shift_c) + md;
+          v = s_tot[1][ch] * a.stat_out.inv_count - md * md;
+        } else if (a.stat_moments) {
+          m = static_cast<double>(a.stat_sums[c]);
+          v = static_cast<double>(a.stat_sums[channels + c]) * a.stat_out.inv_count;
+        } else {
+          m = static_cast<double>(a.stat_sums[c]) * a.stat_out.inv_count;
+          v = static_cast<double>(a.stat_sums[channels + c]) * a.stat_out.inv_count - m * m;
+        }
+        if (v < 0.0) v = 0.0;
+        mean_c = static_cast<float>(m);
+        var_c = static_cast<float>(v);
+        if (writer) WriteFwdStats(a.stat_out, c, m, v);
       } else {
-        m = static_cast<double>(a.stat_sums[c]) * a.stat_out.inv_count;
-        v = static_cast<double>(a.stat_sums[channels + c]) * a.stat_out.inv_count - m * m;
+        mean_c = a.mean[c];
+        var_c = a.variance[c];
+        if (writer && a.pass_stats) WriteGivenStats(a.stat_out, c, mean_c, var_c);
       }
-      if (v < 0.0) v = 0.0;
-      mean[e] = static_cast<float>(m);
-      var_c = static_cast<float>(v);
-      if (writer) WriteFwdStats(a.stat_out, c, m, v);
-    } else {
-      mean[e] = a.mean[c];
-      var_c = a.variance[c];
     }
     const float inv = 1.0f / sqrtf(var_c + a.epsilon);
-    ca[e] = a.scale[c] * inv;
-    if constexpr (kMode == kFwd) {
-      cb[e] = a.offset[c];
-      cc[e] = 0.0f;
-    } else {
-      if (a.fold_rows != nullptr) {
-        const float t1 = static_cast<float>(s_tot[0][tx * kVec + e]);
-        const float t2 = static_cast<float>(s_tot[1][tx * kVec + e]);
-        cb[e] = a.fold_use ? t1 * a.inv_count : 0.0f;
-        cc[e] = a.fold_use ? t2 * inv * inv * a.inv_count : 0.0f;
-        if (writer && a.dscale != nullptr) {
-          a.doffset[c] = t1;
-          a.dscale[c] = t2 * inv;
-        }
-      } else if (a.sums != nullptr) {
-        cb[e] = a.sums[c] * a.inv_count;
-        cc[e] = a.sums[channels + c] * inv * inv * a.inv_count;
-      } else {
-        cb[e] = 0.0f;
-        cc[e] = 0.0f;
+    const float ca1 = scale_c * inv;
+    float cb1 = offset_c, cc1 = 0.0f;
+    if constexpr (kMode == kGrad) {
+      const bool given_sums = !fold && a.sums != nullptr;
+      float t1 = 0.0f, t2 = 0.0f;
+      if (fold) {
+        t1 = static_cast<float>(s_tot[0][ch]);
+        t2 = static_cast<float>(s_tot[1][ch]);
+      } else if (given_sums) {
+        t1 = a.sums[c];
+        t2 = a.sums[channels + c];
       }
-      if (writer && a.dscale != nullptr && a.sums != nullptr) {
-        a.doffset[c] = a.sums[c];
-        a.dscale[c] = a.sums[channels + c] * inv;
+      const bool use = fold ? a.fold_use : given_sums;
+      cb1 = use ? t1 * a.inv_count : 0.0f;
+      cc1 = use ? t2 * inv * inv * a.inv_count : 0.0f;
+      if (writer && a.dscale != nullptr && (fold || given_sums)) {
+        a.doffset[c] = t1;
+        a.dscale[c] = t2 * inv;
+        WriteZeros(a.stat_out, c);
       }
     }
     if constexpr (kFold) {
       if constexpr (kMode == kFwd) {
         // y = x * ca + (offset - mean * ca)
-        cb[e] = fmaf(-mean[e], ca[e], cb[e]);
+        cb1 = fmaf(-mean_c, ca1, cb1);
       } else {
         // dx = dy * ca + x * (-ca * cc) + ca * (cc * mean - cb)
-        const float fb = -ca[e] * cc[e];
-        const float fc = ca[e] * fmaf(cc[e], mean[e], -cb[e]);
-        cb[e] = fb;
-        cc[e] = fc;
+        const float fb = -ca1 * cc1;
+        const float fc = ca1 * fmaf(cc1, mean_c, -cb1);
+        cb1 = fb;
+        cc1 = fc;
       }
     }
+    apply_smem[ch] = ca1;
+    apply_smem[nch + ch] = cb1;
+    if constexpr (kMode == kGrad) apply_smem[2 * nch + ch] = cc1;
+    if constexpr (!kFold) apply_smem[3 * nch + ch] = mean_c;
+  }
+  __syncthreads();
+  if (!active) return;
+  float ca[kVec], cb[kVec], cc[kVec], mean[kVec];
+#pragma unroll
+  for (int e = 0; e < kVec; ++e) {
+    ca[e] = apply_smem[tx * kVec + e];
+    cb[e] = apply_smem[nch + tx * kVec + e];
+    cc[e] = kMode == kGrad ? apply_smem[2 * nch + tx * kVec + e] : 0.0f;
+    mean[e] = kFold ? 0.0f : apply_smem[3 * nch + tx * kVec + e];
   }
 
   P* op = reinterpret_cast<P*>(out) + col;
@@ -1474,8 +1544,11 @@ __global__ void __launch_bounds__(kThreads)
   const int64_t n0 = static_cast<int64_t>(blockIdx.y) * outer_per_cta;
   int64_t n1 = n0 + outer_per_cta;
   if (n1 > outer) n1 = outer;
-  const float inv = 1.0f / sqrtf(a.variance[c] + a.epsilon);
-  const float mean = a.mean[c];
+  const float mean = a.mean[c], var = a.variance[c];
+  const float inv = 1.0f / sqrtf(var + a.epsilon);
+  if (kMode == kFwd && a.pass_stats && blockIdx.y == 0 && lane == 0) {
+    WriteGivenStats(a.stat_out, c, mean, var);
+  }
   const float ca = a.scale[c] * inv;
   float cb, cc = 0.0f;
   if constexpr (kMode == kFwd) {
@@ -1561,7 +1634,11 @@ __global__ void __launch_bounds__(kThreads)
   if (n1 > outer) n1 = outer;
   if (threadIdx.x < kG) {
     const int64_t c = c0 + threadIdx.x;
-    const float inv = 1.0f / sqrtf(a.variance[c] + a.epsilon);
+    const float mean = a.mean[c], var = a.variance[c];
+    const float inv = 1.0f / sqrtf(var + a.epsilon);
+    if (kMode == kFwd && a.pass_stats && blockIdx.y == 0) {
+      WriteGivenStats(a.stat_out, c, mean, var);
+    }
     float cb, cc = 0.0f;
     if constexpr (kMode == kFwd) {
       cb = a.offset[c];
@@ -1569,7 +1646,7 @@ __global__ void __launch_bounds__(kThreads)
       cb = a.sums ? a.sums[c] * a.inv_count : 0.0f;
       cc = a.sums ? a.sums[channels + c] * inv * inv * a.inv_count : 0.0f;
     }
-    coef[threadIdx.x] = make_float4(a.mean[c], a.scale[c] * inv, cb, cc);
+    coef[threadIdx.x] = make_float4(mean, a.scale[c] * inv, cb, cc);
   }
   if (threadIdx.x == 0) coef[kG] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   __syncthreads();
@@ -1955,6 +2032,8 @@ inline int ApplyMaxTx() {
 // rows itself, or -1 when its column blocks are wider than a CTA has threads
 // (the prologue gives every channel of the block one thread).
 constexpr int64_t kApplyFoldSmemMax = 64 * 1024;
+// ... and of the coefficients of `nch` channels, which every launch has.
+inline size_t ApplyCoefBytes(int nch) { return static_cast<size_t>(nch) * 4 * sizeof(float); }
 template <typename T>
 inline int64_t ApplyFoldBytes(int64_t cv, int fold_n) {
   constexpr int kVec = VecWidth<T>::value;
@@ -1966,12 +2045,14 @@ inline int64_t ApplyFoldBytes(int64_t cv, int fold_n) {
 template <typename T, int kVec, int kU, int kMode>
 void LaunchApplyLast(const T* x, const T* dy, T* out, const ApplyArgs& a, const Geom& g,
                      int64_t cv, bool reverse, bool last_use, bool early_loads,
-                     cudaStream_t stream) {
+                     bool early_inputs, cudaStream_t stream) {
   auto kernel = BnApplyLastKernel<T, kVec, kU, kMode>;
   static std::atomic<int> resident_by_device[kMaxDevices];
   int resident = PerDevice(resident_by_device, [&] {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kApplyFoldSmemMax)) != cudaSuccess) {
+                             static_cast<int>(kApplyFoldSmemMax +
+                                              ApplyCoefBytes(kThreads * kVec))) !=
+        cudaSuccess) {
       cudaGetLastError();
     }
     int n = 0;
@@ -1981,9 +2062,9 @@ void LaunchApplyLast(const T* x, const T* dy, T* out, const ApplyArgs& a, const 
     }
     return n > 0 ? n : 1;
   });
-  size_t smem = 0;
+  size_t smem = ApplyCoefBytes(PlanTx(cv, ApplyMaxTx()) * kVec);
   if (a.fold_rows != nullptr) {
-    smem = static_cast<size_t>(ApplyFoldBytes<T>(cv, a.fold_n));
+    smem += static_cast<size_t>(ApplyFoldBytes<T>(cv, a.fold_n));
     // Shared memory of an SM over a CTA's dynamic + static + reserved bytes.
     const int by_smem = static_cast<int>(233472 / (smem + 4096 + 1024));
     if (by_smem < resident) resident = by_smem > 0 ? by_smem : 1;
@@ -1991,14 +2072,18 @@ void LaunchApplyLast(const T* x, const T* dy, T* out, const ApplyArgs& a, const 
   const Plan p = PlanLast(g.outer, g.channels, cv, kU, false, resident, ApplyMaxTx());
   LaunchChained(GetTuning(kTuneBnPdl) != 0, kernel, dim3(p.gx, p.gy), dim3(p.tx, p.ty), smem,
                 stream, x, dy, out, a, g.outer, cv, g.channels, p.rows_per_cta, reverse,
-                last_use, early_loads, GetTuning(kTuneBnInterleave) != 0);
+                last_use, early_loads, early_inputs, GetTuning(kTuneBnInterleave) != 0);
 }
 
-// `early_loads`: the caller launched the statistics kernel of the same op on
-// `stream` just before (see BnApplyLastKernel).
+// How much the element-wise kernel may read before its wait for the kernel it
+// depends on: nothing (a launch of its own), x / dy (the caller's statistics
+// pass on `stream` read them), or every input of the op (the statistics kernel
+// was launched by the same launcher call).
+enum EarlyReads { kReadAfterWait = 0, kReadRowsEarly = 1, kReadInputsEarly = 2 };
+
 template <typename T, int kMode>
 void LaunchApply(const T* x, const T* dy, T* out, const ApplyArgs& a,
-                 const Geom& g, cudaStream_t stream, bool early_loads = false) {
+                 const Geom& g, cudaStream_t stream, EarlyReads early_reads = kReadAfterWait) {
   constexpr int kVec = VecWidth<T>::value;
   constexpr int kUnroll = 4;
   const bool reverse = GetTuning(kTuneBnApplyReverse) != 0;
@@ -2020,22 +2105,24 @@ void LaunchApply(const T* x, const T* dy, T* out, const ApplyArgs& a,
       const int64_t cv = g.channels / kVec;
       // The forward pass has one input stream: twice the rows in flight.
       const bool deep = kMode == kFwd && GetTuning(kTuneBnApplyDeep) != 0;
-      const bool early = early_loads && GetTuning(kTuneBnApplyEarlyLoads) != 0;
+      const bool tuned_early = GetTuning(kTuneBnApplyEarlyLoads) != 0;
+      const bool early = early_reads >= kReadRowsEarly && tuned_early;
+      const bool inputs = early_reads == kReadInputsEarly && tuned_early;
       if (deep) {
         constexpr int kDeep = kMode == kFwd ? 8 : kUnroll;
         LaunchApplyLast<T, kVec, kDeep, kMode>(x, dy, out, a, g, cv, reverse, last_use, early,
-                                               stream);
+                                               inputs, stream);
       } else {
         LaunchApplyLast<T, kVec, kUnroll, kMode>(x, dy, out, a, g, cv, reverse, last_use, early,
-                                                 stream);
+                                                 inputs, stream);
       }
     } else {
       const Plan p =
           PlanLast(g.outer, g.channels, g.channels, kUnroll, false, 4);
       BnApplyLastKernel<T, 1, kUnroll, kMode>
-          <<<dim3(p.gx, p.gy), dim3(p.tx, p.ty), 0, stream>>>(
+          <<<dim3(p.gx, p.gy), dim3(p.tx, p.ty), ApplyCoefBytes(p.tx), stream>>>(
               x, dy, out, a, g.outer, g.channels, g.channels, p.rows_per_cta,
-              reverse, false, false, false);
+              reverse, false, false, false, false);
       CountKernelLaunch();
     }
     return;
@@ -2102,7 +2189,7 @@ int FwdTrain(const void* x, const float* scale, const float* offset,
              float* batch_mean, float* batch_var, float* saved_mean,
              float* saved_var, int64_t outer, int64_t channels, int64_t inner,
              float epsilon, float exp_avg_factor, void* workspace,
-             size_t workspace_bytes, cudaStream_t stream) {
+             size_t workspace_bytes, cudaStream_t stream, float* zero_scalar = nullptr) {
   const Geom g{outer, channels, inner};
   if (int rc = CheckGeom(g)) return rc;
   MUSA_TRACE("LaunchBnFwdTrain", 2 * sizeof(T) * outer * channels * inner);
@@ -2133,6 +2220,7 @@ int FwdTrain(const void* x, const float* scale, const float* offset,
   f.saved_mean = saved_mean;
   f.saved_var = saved_var;
   f.exp_avg_factor = exp_avg_factor;
+  f.zero_scalar = zero_scalar;
   ApplyArgs a{};
   a.scale = scale;
   a.offset = offset;
@@ -2157,7 +2245,7 @@ int FwdTrain(const void* x, const float* scale, const float* offset,
     f.splits = splits;
     LaunchFinalize(kTailFwdStats, f, stream);
   }
-  LaunchApply<T, kFwd>(xt, nullptr, static_cast<T*>(y), a, g, stream, true);
+  LaunchApply<T, kFwd>(xt, nullptr, static_cast<T*>(y), a, g, stream, kReadInputsEarly);
   return LastError();
 }
 
@@ -2165,7 +2253,7 @@ template <typename T>
 int FwdInfer(const void* x, const float* scale, const float* offset,
              const float* est_mean, const float* est_var, void* y,
              int64_t outer, int64_t channels, int64_t inner, float epsilon,
-             cudaStream_t stream) {
+             cudaStream_t stream, const FinalizeArgs* pass_to = nullptr) {
   const Geom g{outer, channels, inner};
   if (int rc = CheckGeom(g)) return rc;
   MUSA_TRACE("LaunchBnApply", 2 * sizeof(T) * outer * channels * inner);
@@ -2179,6 +2267,10 @@ int FwdInfer(const void* x, const float* scale, const float* offset,
   a.mean = est_mean;
   a.variance = est_var;
   a.epsilon = epsilon;
+  if (pass_to != nullptr) {
+    a.pass_stats = true;
+    a.stat_out = *pass_to;
+  }
   LaunchApply<T, kFwd>(static_cast<const T*>(x), nullptr, static_cast<T*>(y), a,
                        g, stream);
   return LastError();
@@ -2189,7 +2281,7 @@ int Grad(const void* dy, const void* x, const float* scale, const float* mean,
          const float* variance, void* dx, float* dscale, float* doffset,
          int64_t outer, int64_t channels, int64_t inner, float epsilon,
          bool is_training, void* workspace, size_t workspace_bytes,
-         cudaStream_t stream) {
+         cudaStream_t stream, float* zeros_a = nullptr, float* zeros_b = nullptr) {
   const Geom g{outer, channels, inner};
   if (int rc = CheckGeom(g)) return rc;
   MUSA_TRACE("LaunchBnGrad", 3 * sizeof(T) * outer * channels * inner);
@@ -2214,6 +2306,8 @@ int Grad(const void* dy, const void* x, const float* scale, const float* mean,
   f.doffset = doffset;
   f.epsilon = epsilon;
   f.sums = sums;
+  f.zero_vec[0] = zeros_a;
+  f.zero_vec[1] = zeros_b;
   ApplyArgs a{};
   a.scale = scale;
   a.mean = mean;
@@ -2232,11 +2326,12 @@ int Grad(const void* dy, const void* x, const float* scale, const float* mean,
     a.fold_use = is_training;
     a.dscale = dscale;
     a.doffset = doffset;
+    a.stat_out = f;
   } else {
     f.splits = splits;
     LaunchFinalize(kTailGrad, f, stream);
   }
-  LaunchApply<T, kGrad>(xt, dyt, static_cast<T*>(dx), a, g, stream, true);
+  LaunchApply<T, kGrad>(xt, dyt, static_cast<T*>(dx), a, g, stream, kReadInputsEarly);
   return LastError();
 }
 
@@ -2325,7 +2420,7 @@ int GradApplyFromSums(const void* dy, const void* x, const float* scale,
   // dy and x were read by the preceding LaunchBnGradStatsSums* call on this
   // stream: final before it (see ApplyFromSums).
   LaunchApply<T, kGrad>(static_cast<const T*>(x), static_cast<const T*>(dy),
-                        static_cast<T*>(dx), a, g, stream, true);
+                        static_cast<T*>(dx), a, g, stream, kReadRowsEarly);
   return LastError();
 }
 
@@ -2583,7 +2678,7 @@ int ApplyFromSums(int dtype, const void* x, const float* scale, const float* off
   // stream took: it was final before that call, so the first rows may be
   // requested before the wait for the kernel that delivers the statistics.
   MUSA_BY_DTYPE(dtype, (LaunchApply<T, kFwd>(static_cast<const T*>(x), nullptr,
-                                             static_cast<T*>(y), a, g, stream, true),
+                                             static_cast<T*>(y), a, g, stream, kReadRowsEarly),
                         LastError()));
 }
 }  // namespace
@@ -2700,6 +2795,46 @@ int LaunchBnFinalizeFromSums(const float* sums, double total_count,
   return FinalizeFromSums(sums, false, total_count, est_mean, est_var, batch_mean,
                           batch_var, saved_mean, saved_var, channels, exp_avg_factor,
                           stream);
+}
+
+// The ops with every output written on the device by the op's own kernels
+// (the zeros and the passed-through statistics too).
+int LaunchBnFwdTrainOp(int dtype, const void* x, const float* scale, const float* offset,
+                       const float* est_mean, const float* est_var, void* y, float* batch_mean,
+                       float* batch_var, float* saved_mean, float* saved_var, float* reserve_3,
+                       int64_t outer, int64_t channels, int64_t inner, float epsilon,
+                       float exp_avg_factor, void* workspace, size_t workspace_bytes,
+                       cudaStream_t stream) {
+  MUSA_BY_DTYPE(dtype, FwdTrain<T>(x, scale, offset, est_mean, est_var, y, batch_mean, batch_var,
+                                   saved_mean, saved_var, outer, channels, inner, epsilon,
+                                   exp_avg_factor, workspace, workspace_bytes, stream,
+                                   reserve_3));
+}
+
+int LaunchBnFwdInferOp(int dtype, const void* x, const float* scale, const float* offset,
+                       const float* est_mean, const float* est_var, void* y, float* batch_mean,
+                       float* batch_var, float* saved_mean, float* saved_var, float* reserve_3,
+                       int64_t outer, int64_t channels, int64_t inner, float epsilon,
+                       cudaStream_t stream) {
+  if (!batch_mean || !batch_var || !saved_mean || !saved_var) return MUSA_KERNELS_EINVAL;
+  FinalizeArgs f{};
+  f.batch_mean = batch_mean;
+  f.batch_var = batch_var;
+  f.saved_mean = saved_mean;
+  f.saved_var = saved_var;
+  f.zero_scalar = reserve_3;
+  MUSA_BY_DTYPE(dtype, FwdInfer<T>(x, scale, offset, est_mean, est_var, y, outer, channels, inner,
+                                   epsilon, stream, &f));
+}
+
+int LaunchBnGradOp(int dtype, const void* dy, const void* x, const float* scale,
+                   const float* mean, const float* variance, void* dx, float* dscale,
+                   float* doffset, float* reserve_4, float* reserve_5, int64_t outer,
+                   int64_t channels, int64_t inner, float epsilon, bool is_training,
+                   void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  MUSA_BY_DTYPE(dtype, Grad<T>(dy, x, scale, mean, variance, dx, dscale, doffset, outer, channels,
+                               inner, epsilon, is_training, workspace, workspace_bytes, stream,
+                               reserve_4, reserve_5));
 }
 
 int LaunchBnApply(int dtype, const void* x, const float* scale,

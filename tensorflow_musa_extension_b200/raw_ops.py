@@ -228,32 +228,27 @@ def FusedBatchNormV3(x, scale, offset, mean, variance, epsilon=0.0001,
     with torch.cuda.device(dev):
         y = torch.empty_like(x)
         stats = [torch.empty(c, dtype=torch.float32, device=dev) for _ in range(4)]
-        reserve_3 = torch.zeros((), dtype=torch.float32, device=dev)
-        sfx = _SUFFIX[x.dtype]
+        reserve_3 = torch.empty((), dtype=torch.float32, device=dev)
+        outs = [_ptr(t) for t in (y, *stats, reserve_3)]
         if x.numel() == 0:
-            for s in stats:
+            for s in (*stats, reserve_3):
                 s.zero_()
         elif is_training:
             nbytes = _lib().BnWorkspaceBytes(outer, c, inner)
             ws = _workspace(nbytes, dev)
-            fn = getattr(_lib(), "LaunchBnFwdTrain_" + sfx)
-            rc = fn(_ptr(x), _ptr(scale), _ptr(offset),
-                    _ptr(mean) if have_est else None,
-                    _ptr(variance) if have_est else None, _ptr(y),
-                    _ptr(stats[0]), _ptr(stats[1]), _ptr(stats[2]), _ptr(stats[3]),
-                    outer, c, inner, float(epsilon), float(exponential_avg_factor),
-                    _ptr(ws), ws.numel(), _stream())
+            rc = _lib().LaunchBnFwdTrainOp(
+                _DT_CODE[x.dtype], _ptr(x), _ptr(scale), _ptr(offset),
+                _ptr(mean) if have_est else None,
+                _ptr(variance) if have_est else None, *outs, outer, c, inner,
+                float(epsilon), float(exponential_avg_factor), _ptr(ws), ws.numel(), _stream())
             _check(rc, "FusedBatchNormV3")
         else:
-            fn = getattr(_lib(), "LaunchBnFwdInfer_" + sfx)
-            rc = fn(_ptr(x), _ptr(scale), _ptr(offset), _ptr(mean), _ptr(variance),
-                    _ptr(y), outer, c, inner, float(epsilon), _stream())
+            # The op passes the given statistics through in inference mode: the
+            # kernel writes the copies.
+            rc = _lib().LaunchBnFwdInferOp(
+                _DT_CODE[x.dtype], _ptr(x), _ptr(scale), _ptr(offset), _ptr(mean),
+                _ptr(variance), *outs, outer, c, inner, float(epsilon), _stream())
             _check(rc, "FusedBatchNormV3")
-            # The op passes the given statistics through in inference mode.
-            stats[0].copy_(mean)
-            stats[1].copy_(variance)
-            stats[2].copy_(mean)
-            stats[3].copy_(variance)
     return FusedBatchNormV3Output(*hf.back_many((y, *stats, reserve_3)))
 
 
@@ -307,18 +302,18 @@ def FusedBatchNormGradV3(y_backprop, x, scale, reserve_space_1, reserve_space_2,
         dx = torch.empty_like(x)
         dscale = torch.empty(c, dtype=torch.float32, device=dev)
         doffset = torch.empty(c, dtype=torch.float32, device=dev)
-        r4 = torch.zeros(c, dtype=torch.float32, device=dev)
-        r5 = torch.zeros(c, dtype=torch.float32, device=dev)
+        r4 = torch.empty(c, dtype=torch.float32, device=dev)
+        r5 = torch.empty(c, dtype=torch.float32, device=dev)
         if x.numel() == 0:
-            dscale.zero_()
-            doffset.zero_()
+            for t in (dscale, doffset, r4, r5):
+                t.zero_()
         else:
             nbytes = _lib().BnWorkspaceBytes(outer, c, inner)
             ws = _workspace(nbytes, dev)
-            fn = getattr(_lib(), "LaunchBnGrad_" + _SUFFIX[x.dtype])
-            rc = fn(_ptr(dy), _ptr(x), _ptr(scale), _ptr(mean), _ptr(var), _ptr(dx),
-                    _ptr(dscale), _ptr(doffset), outer, c, inner, float(epsilon),
-                    bool(is_training), _ptr(ws), ws.numel(), _stream())
+            rc = _lib().LaunchBnGradOp(
+                _DT_CODE[x.dtype], _ptr(dy), _ptr(x), _ptr(scale), _ptr(mean), _ptr(var),
+                _ptr(dx), _ptr(dscale), _ptr(doffset), _ptr(r4), _ptr(r5), outer, c, inner,
+                float(epsilon), bool(is_training), _ptr(ws), ws.numel(), _stream())
             _check(rc, "FusedBatchNormGradV3")
     return FusedBatchNormGradV3Output(*hf.back_many((dx, dscale, doffset, r4, r5)))
 

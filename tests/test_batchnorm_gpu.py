@@ -603,3 +603,53 @@ def test_forward_in_place(kernel_lib, rows, c):
     assert torch.equal(tz, ty)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,shape,layout", [
+    ("bfloat16", (3, 5, 7, 64), "NHWC"),     # whole packs, one column block
+    ("float32", (2, 3, 3, 2056), "NHWC"),    # many column blocks, the last one partly filled
+    ("float16", (4, 3, 5, 37), "NHWC"),      # single elements
+    ("bfloat16", (3, 16, 7, 7), "NCHW"),     # channel groups
+    ("float16", (2, 12, 8, 8), "NCHW"),      # whole planes
+    ("float32", (1, 1, 3, 5), "NCHW"),       # one channel
+])
+def test_outputs_beside_the_statistics(kernel_lib, dtype, shape, layout):
+    """The zeros (reserve_space_3 .. 5) and the passed-through statistics of the
+    inference form come from the op's own kernels, in every geometry and from
+    buffers with arbitrary contents."""
+    c = shape[-1] if layout == "NHWC" else shape[1]
+    x, s_, o, dy = bn_inputs(41, shape, dtype, 0.5, 2.0)
+    gen = np.random.default_rng(c)
+    rm = to_torch(gen.standard_normal(c).astype(np.float32))
+    rv = to_torch((gen.random(c) + 0.5).astype(np.float32))
+    tx, tdy, ts, to_ = to_torch(x), to_torch(dy), to_torch(s_), to_torch(o)
+    outer, inner = (tx.numel() // c, 1) if layout == "NHWC" else (shape[0], shape[2] * shape[3])
+    code = raw_ops._DT_CODE[tx.dtype]
+    st = torch.cuda.current_stream().cuda_stream
+    need = kernel_lib.BnWorkspaceBytes(outer, c, inner)
+    ws = torch.full((max(need, 16),), 0x5A, dtype=torch.uint8, device="cuda")
+
+    def fresh(n):
+        return [torch.full((c,), float("nan"), device="cuda") for _ in range(n)]
+
+    def ptrs(ts_):
+        return [t.data_ptr() for t in ts_]
+
+    y, stats, r3 = torch.empty_like(tx), fresh(4), torch.full((), float("nan"), device="cuda")
+    assert kernel_lib.LaunchBnFwdInferOp(
+        code, *ptrs((tx, ts, to_, rm, rv, y, *stats, r3)), outer, c, inner, EPS, st) == 0
+    for got, want in zip(stats, (rm, rv, rm, rv)):
+        assert torch.equal(got, want)
+    assert float(r3) == 0.0
+    stats, r3 = fresh(4), torch.full((), float("nan"), device="cuda")
+    assert kernel_lib.LaunchBnFwdTrainOp(
+        code, *ptrs((tx, ts, to_)), None, None, *ptrs((y, *stats, r3)), outer, c, inner, EPS, 1.0,
+        ws.data_ptr(), ws.numel(), st) == 0
+    assert float(r3) == 0.0 and all(bool(torch.isfinite(t).all()) for t in stats)
+    for training in (True, False):
+        dx, outs = torch.empty_like(tx), fresh(4)
+        assert kernel_lib.LaunchBnGradOp(
+            code, *ptrs((tdy, tx, ts, stats[2], stats[3], dx, *outs)), outer, c, inner, EPS,
+            training, ws.data_ptr(), ws.numel(), st) == 0
+        assert all(bool(torch.isfinite(t).all()) for t in outs[:2])
+        assert not outs[2].any() and not outs[3].any()
