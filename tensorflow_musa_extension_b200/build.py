@@ -19,6 +19,8 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 BUILD_DIR = os.path.join(PKG_DIR, "build")
 LIB_NAME = "libmusa_plugin_kernels.so"
 LIB_PATH = os.path.join(PKG_DIR, LIB_NAME)
+NATIVE_SRC = os.path.join(CSRC, "python", "native_ops.cc")
+NATIVE_PATH = os.path.join(PKG_DIR, "_native_ops.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -38,6 +40,8 @@ def _nvcc():
 def sources():
     out = []
     for root, _, files in os.walk(CSRC):
+        if os.path.basename(root) == "python":   # the extension module: build_native()
+            continue
         for f in sorted(files):
             if f.endswith((".cu", ".cc")):
                 out.append(os.path.join(root, f))
@@ -86,7 +90,39 @@ def build(force=False, verbose=False):
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
+    build_native(force, verbose)
     return LIB_PATH
+
+
+def build_native(force=False, verbose=False):
+    """Compiles the extension module of the native host path (host code only)
+    against the installed torch."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    libs = os.path.join(root, "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+           "-I" + sysconfig.get_paths()["include"],
+           "-isystem", os.path.join(root, "include"),
+           "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-isystem", os.path.join(cuda, "include"), NATIVE_SRC, "-o", NATIVE_PATH,
+           "-L" + libs, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+           "-Wl,-rpath," + libs]
+    tag = os.path.join(BUILD_DIR, "native_ops.stamp")
+    with open(NATIVE_SRC, "rb") as fh:
+        want = hashlib.sha256(fh.read() + _headers_digest().encode() + " ".join(cmd).encode()
+                              + torch.__version__.encode()).hexdigest()
+    have = open(tag).read() if os.path.exists(tag) else ""
+    if force or have != want or not os.path.exists(NATIVE_PATH):
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        subprocess.run(cmd, check=True)
+        with open(tag, "w") as fh:
+            fh.write(want)
+    return NATIVE_PATH
 
 
 if __name__ == "__main__":

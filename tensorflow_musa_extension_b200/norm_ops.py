@@ -35,6 +35,9 @@ def MusaLayerNorm(x, gamma, beta, epsilon=0.00001, name=None):
     axis, y = (x - mean) * rsqrt(var + epsilon) * gamma + beta
     (musa_ext/kernels/fusion/musa_layernorm_op.cc:26-100, op definition
     :118-124)."""
+    out = _r._native().layer_norm(x, gamma, beta, epsilon)
+    if out is not None:
+        return _r._native_result(out, None, "MusaLayerNorm")
     _r._require_cuda()
     hf = _r._HostForm()
     xd, g, b = hf.to_device(x), hf.to_device(gamma), hf.to_device(beta)
@@ -61,6 +64,9 @@ def MusaLayerNormGrad(dy, x, gamma, beta, epsilon=0.00001, name=None):
     statistics are recomputed from x
     (musa_ext/kernels/fusion/musa_layernorm_grad_op.cc:23-141, op definition
     :143-158)."""
+    out = _r._native().layer_norm_grad(dy, x, gamma, beta, epsilon)
+    if out is not None:
+        return _r._native_result(out, MusaLayerNormGradOutput, "MusaLayerNormGrad")
     _r._require_cuda()
     hf = _r._HostForm()
     d, xd, g, b = (hf.to_device(t) for t in (dy, x, gamma, beta))
@@ -98,6 +104,9 @@ def MusaRmsNorm(x, gamma, epsilon=0.00001, name=None):
     """MusaRmsNorm for T in {float, bfloat16}: returns (y, normalized,
     inv_rms), inv_rms shaped like x with a last axis of 1
     (musa_ext/kernels/nn/musa_rmsnorm_op.cc:24-87, op definition :175-201)."""
+    out = _r._native().rms_norm(x, gamma, epsilon)
+    if out is not None:
+        return _r._native_result(out, MusaRmsNormOutput, "MusaRmsNorm")
     _r._require_cuda()
     hf = _r._HostForm()
     xd, g = hf.to_device(x), hf.to_device(gamma)
@@ -126,6 +135,9 @@ def MusaRmsNorm(x, gamma, epsilon=0.00001, name=None):
 def MusaRmsNormGradDx(x, inv_rms, gamma, dy, name=None):
     """MusaRmsNormGradDx: the gradient of MusaRmsNorm with respect to x
     (musa_ext/kernels/nn/musa_rmsnorm_op.cc:96-146, op definition :163-173)."""
+    out = _r._native().rms_norm_grad_dx(x, inv_rms, gamma, dy)
+    if out is not None:
+        return _r._native_result(out, None, "MusaRmsNormGradDx")
     _r._require_cuda()
     hf = _r._HostForm()
     xd, inv, g, d = (hf.to_device(t) for t in (x, inv_rms, gamma, dy))

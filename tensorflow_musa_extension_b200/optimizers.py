@@ -12,8 +12,6 @@ the same hyper-parameters, slot names ("m", "v") and dispatch:
   amsgrad=True                                 -> rejected (the reference falls
                                                   back to stock Keras there)
 """
-import ctypes
-
 import torch
 
 from . import raw_ops
@@ -55,40 +53,21 @@ class MusaAdam:
     def get_slot(self, var, slot_name):
         if slot_name not in ("m", "v"):
             raise InvalidArgumentError("unknown slot %r" % (slot_name,))
-        key = id(var)
-        if key not in self._slots:
+        slots = self._slots.get(id(var))
+        if slots is None:
             t = var.tensor() if isinstance(var, raw_ops.Variable) else var
-            self._slots[key] = {"m": torch.zeros_like(t), "v": torch.zeros_like(t)}
-        return self._slots[key][slot_name]
-
-    def _groupable(self, t, m, v, grad):
-        """Whether the update can share a launch with its neighbours: device
-        tensors in the form that the op hands to its kernel as they are.
-        Everything else (host gradients, wrong shapes or types) goes through
-        the op, which converts or refuses."""
-        return (isinstance(grad, torch.Tensor) and isinstance(t, torch.Tensor)
-                and t.is_cuda and grad.is_cuda and grad.device == t.device
-                and (t.dtype == torch.float32 and grad.dtype in self._LOWP_GRAD_DTYPES
-                     or t.dtype == grad.dtype and t.dtype in self._LOWP_GRAD_DTYPES)
-                and m.dtype == t.dtype and v.dtype == t.dtype
-                and t.shape == grad.shape and t.shape == m.shape and t.shape == v.shape
-                and t.is_contiguous() and grad.is_contiguous()
-                and m.is_contiguous() and v.is_contiguous())
+            slots = {"m": torch.zeros_like(t), "v": torch.zeros_like(t)}
+            self._slots[id(var)] = slots
+        return slots[slot_name]
 
     def _apply_group(self, group, b1p, b2p):
         """One launch for consecutive variables of one device, state type and
         gradient type; the scalars are read as the ops read them."""
-        t, grad = group[0][0], group[0][3]
+        t = group[0][0]
         sc = [raw_ops._scalar_in(x, t.dtype) for x in (
             self.learning_rate, b1p, b2p, self.beta_1, self.beta_2, self.epsilon)]
-        n = len(group)
-        tables = [(ctypes.c_void_p * n)(*[q[k].data_ptr() for q in group]) for k in range(4)]
-        sizes = (ctypes.c_int64 * n)(*[q[0].numel() for q in group])
-        with torch.cuda.device(t.device):
-            rc = raw_ops._lib().LaunchApplyAdamGroupHostTable(
-                raw_ops._DT_CODE[t.dtype], raw_ops._DT_CODE[grad.dtype], *tables, sizes, n,
-                raw_ops._adam_alpha(*sc[:3]), sc[3], sc[4], sc[5], self.use_nesterov,
-                raw_ops._stream())
+        rc = raw_ops._native().adam_group(group, raw_ops._adam_alpha(*sc[:3]), sc[3], sc[4],
+                                          sc[5], self.use_nesterov)
         raw_ops._check(rc, "MusaAdam")
 
     def apply_gradients(self, grads_and_vars):
@@ -112,10 +91,17 @@ class MusaAdam:
                 t = var.tensor() if isinstance(var, raw_ops.Variable) else var
                 m = self.get_slot(var, "m")
                 v = self.get_slot(var, "v")
-                if self._groupable(t, m, v, grad):
-                    if kind != (t.device, t.dtype, grad.dtype):
+                # Whether the update can share a launch with its neighbours:
+                # device tensors in the form that the op hands to its kernel
+                # as they are.  Everything else (host gradients, wrong shapes
+                # or types) goes through the op, which converts or refuses.
+                this = -1
+                if isinstance(grad, torch.Tensor) and grad.is_cuda:
+                    this = raw_ops._native().adam_kind(t, m, v, grad)
+                if this >= 0:
+                    if kind != this:
                         flush()
-                        kind = (t.device, t.dtype, grad.dtype)
+                        kind = this
                     group.append((t, m, v, grad))
                     continue
                 flush()

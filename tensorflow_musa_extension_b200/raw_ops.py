@@ -14,6 +14,7 @@ implementation behind these functions: without a device or without the kernel
 library they raise.
 """
 import collections
+import ctypes
 import threading
 
 import numpy as np
@@ -37,6 +38,7 @@ _SUFFIX = {torch.float32: "F32", torch.float16: "F16", torch.bfloat16: "BF16",
 _DT_CODE = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 
 _bound = None
+_bound_native = None
 _bind_lock = threading.Lock()
 
 
@@ -47,6 +49,21 @@ def _lib():
             if _bound is None:
                 _bound = _capi.bind(_loader.get_library())
     return _bound
+
+
+def _native():
+    """The native host path: one C++ function per op that checks, allocates and
+    launches.  It answers None for every call that is not contiguous device
+    tensors of the op's types (host buffers, conversions, errors); the op then
+    takes its general path below."""
+    global _bound_native
+    if _bound_native is None:
+        _require_cuda()
+        lib = _lib()
+        from . import _native_ops
+        _native_ops.bind(lib._handle)
+        _bound_native = _native_ops
+    return _bound_native
 
 
 def _require_cuda():
@@ -133,6 +150,14 @@ def _check(rc, what):
     raise InternalError("%s: CUDA error %d" % (what, rc))
 
 
+def _native_result(out, kind, what):
+    """Outputs of a native call as the op's named tuple (`kind` None: its one
+    output); an int is the launcher's error code."""
+    if type(out) is int:
+        _check(out, what)
+    return out[0] if kind is None else kind._make(out)
+
+
 _ws_cache = {}
 
 
@@ -204,6 +229,10 @@ def FusedBatchNormV3(x, scale, offset, mean, variance, epsilon=0.0001,
     """FusedBatchNormV3 on T in {float, half, bfloat16} with float statistics
     (registration: musa_ext/kernels/nn/musa_fused_batchnorm_op.cc:303-325;
     Compute: :42-182).  Returns the op's six outputs."""
+    out = _native().bn_forward(x, scale, offset, mean, variance, epsilon,
+                               exponential_avg_factor, data_format, is_training)
+    if out is not None:
+        return _native_result(out, FusedBatchNormV3Output, "FusedBatchNormV3")
     _require_cuda()
     hf = _HostForm()
     x = hf.to_device(x)
@@ -278,6 +307,10 @@ def FusedBatchNormGradV3(y_backprop, x, scale, reserve_space_1, reserve_space_2,
     is the mean, reserve_space_2 the population variance; reserve_space_3 is
     accepted and ignored.  Outputs 3 and 4 are zero-filled [C], as the
     reference emits them (:220-242)."""
+    out = _native().bn_gradient(y_backprop, x, scale, reserve_space_1, reserve_space_2,
+                                epsilon, data_format, is_training)
+    if out is not None:
+        return _native_result(out, FusedBatchNormGradV3Output, "FusedBatchNormGradV3")
     _require_cuda()
     hf = _HostForm()
     dy = hf.to_device(y_backprop)
@@ -395,6 +428,8 @@ def _np_dtype_of(t):
 def _scalar_in(value, torch_dtype):
     """A host scalar input read as the op's T and widened to double (the
     kernel reads `scalar<T>()`; musa_applyadam_op.cc:224-229)."""
+    if type(value) is float and torch_dtype is torch.float32:
+        return ctypes.c_float(value).value
     if isinstance(value, torch.Tensor):
         value = value.detach().cpu().to(torch.float64).item()
     arr = np.asarray(value)
@@ -585,6 +620,10 @@ _ACT_FLOAT = (torch.float32, torch.float16, torch.bfloat16)
 
 
 def _bias_act(opname, value, bias, data_format, act, dtypes):
+    if bias is not None:
+        out = _native().bias_act(value, bias, data_format, act)
+        if out is not None:
+            return _native_result(out, None, opname)
     _require_cuda()
     hf = _HostForm()
     x = hf.to_device(value)
@@ -754,6 +793,9 @@ def MusaBiasAddReluGrad(gradients, features, data_format="NHWC", name=None):
     ReluGrad->BiasAddGrad fusion pattern emits; the reference runs the two ops
     separately (musa_ext/kernels/nn/musa_relu_grad_op.cc,
     musa_ext/kernels/nn/musa_biasadd_grad_op.cc)."""
+    out = _native().bias_relu_grad(gradients, features, data_format)
+    if out is not None:
+        return _native_result(out, MusaBiasAddReluGradOutput, "MusaBiasAddReluGrad")
     _require_cuda()
     hf = _HostForm()
     g, f = _relu_grad_inputs("MusaBiasAddReluGrad", gradients, features, hf)
