@@ -1695,6 +1695,546 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// ------------------------------------------------- one kernel per op ----
+//
+// Layers that fit the shared memory of the SMs (up to about 25 MB of inputs)
+// need no second pass over memory and no kernel boundary: a CLUSTER of up to
+// 16 CTAs owns a block of `tx` channel packs and all rows, each CTA keeps its
+// row range of x (and dy) in shared memory, the CTAs' sums meet through
+// distributed shared memory at one hardware barrier, and every CTA normalises
+// its rows from where they are.  What bounds such a layer is latency: launch,
+// one memory round trip, one cluster barrier, one drain, against two or three
+// kernels and two trips.  The element-wise arithmetic, the shift of the sums
+// and the fp64 epilogue are those of the kernels above.  Device time of a call
+// (chain -> this form, inputs in L2): fp32 [1568,64] forward 5.8 -> 4.2 us,
+// gradient 6.1 -> 4.4; bf16 [1568,2048] 8.6 -> 6.0 and 9.5 -> 6.7; bf16
+// [6272,1024] forward 11.7 -> 7.9; channel-major bf16 [64,512,7,7] 10.8 -> 6.6
+// and 12.3 -> 7.0, [64,512,14,14] forward 18.4 -> 8.9, fp32 [8,64,14,14]
+// 8.3 -> 4.0.  The limit on the inputs is where the form stops fitting: 64 to
+// 128 CTAs hold 13 to 25 MB, and near that the two are level (fp32
+// [25088,128], 12.8 MB: 10.8 against 9.4-10.2).
+constexpr int kOnChipThreads = 512;
+constexpr int kOnChipWarps = kOnChipThreads / 32;
+constexpr int kOnChipMaxTx = 8;
+constexpr int kOnChipMaxCluster = 16;
+// 16-byte slots per thread (25 x 512 x 16 = 200 KB beside 11 KB of static
+// shared memory).
+constexpr int kOnChipSlots = 25;
+constexpr int64_t kOnChipMaxBytes = 16 << 20;   // inputs of the pass
+constexpr int kOnChipChunks = 4;   // asynchronous copies are waited for in this many steps
+
+// A cluster barrier in two halves: the second phase only keeps the CTA's
+// shared memory alive until its neighbours have read it.
+__device__ __forceinline__ void ClusterArrive() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void ClusterWait() {
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// The sums of one channel over the CTAs of the cluster, in rank order and fp64;
+// `p1`, `p2` are the channel's two entries in this CTA's shared memory.
+__device__ __forceinline__ void ClusterTotals(const float* p1, const float* p2, int world,
+                                              double& S1, double& S2) {
+  float v1[kOnChipMaxCluster], v2[kOnChipMaxCluster];
+#pragma unroll
+  for (int q = 0; q < kOnChipMaxCluster; ++q) {
+    v1[q] = q < world ? LoadClusterF32(p1, static_cast<unsigned>(q)) : 0.0f;
+    v2[q] = q < world ? LoadClusterF32(p2, static_cast<unsigned>(q)) : 0.0f;
+  }
+  S1 = 0.0;
+  S2 = 0.0;
+#pragma unroll
+  for (int q = 0; q < kOnChipMaxCluster; ++q) {
+    S1 += static_cast<double>(v1[q]);
+    S2 += static_cast<double>(v2[q]);
+  }
+}
+
+// Grid (column blocks, cluster CTAs), cluster (1, cluster CTAs), block
+// (tx, 512 / tx); rows_per_cta rows per CTA, `slots` = row slots per thread.
+template <typename T, int kMode>
+__global__ void __launch_bounds__(kOnChipThreads, 1)
+    BnOnChipKernel(const T* x, const T* dy, T* out, ApplyArgs a, int64_t rows, int64_t cv,
+                   int64_t channels, int64_t rows_per_cta, int slots) {
+  constexpr int kVec = VecWidth<T>::value;
+  constexpr int kPairs = kVec / 2;
+  constexpr bool kNarrow = sizeof(T) == 2;   // coefficients folded as in BnApplyLastKernel
+  using P = Pack<T, kVec>;
+  extern __shared__ uint4 onchip_tile[];     // [stream][slot][thread]
+  __shared__ float warp_sum[kOnChipWarps][2 * kOnChipMaxTx * kVec];
+  __shared__ float part[2 * kOnChipMaxTx * kVec];      // this CTA's sums, read by the cluster
+  __shared__ float coef[4][kOnChipMaxTx * kVec];
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int TX = blockDim.x, TY = blockDim.y;
+  const int tid = ty * TX + tx;
+  const int nch = TX * kVec;
+  const int64_t c0 = static_cast<int64_t>(blockIdx.x) * nch;
+  const int seg = channels - c0 < nch ? static_cast<int>(channels - c0) : nch;
+  const int64_t col = static_cast<int64_t>(blockIdx.x) * TX + tx;
+  const int64_t r0 = static_cast<int64_t>(blockIdx.y) * rows_per_cta;
+  const int64_t r1 = r0 + rows_per_cta < rows ? r0 + rows_per_cta : rows;
+  // This thread's rows: r0 + ty + j * TY, j = 0 .. n - 1 (n <= slots).
+  const int64_t left = r1 - r0 - ty;
+  const int n = col < cv && left > 0 ? static_cast<int>((left + TY - 1) / TY) : 0;
+  const int64_t first = (r0 + ty) * cv + col;
+  const int64_t step = static_cast<int64_t>(TY) * cv;
+  const P* xp = reinterpret_cast<const P*>(x) + first;
+  const P* dp = reinterpret_cast<const P*>(dy) + first;
+  uint4* const mine = onchip_tile + tid;
+  uint4* const mine_dy = mine + slots * kOnChipThreads;
+  const int per_chunk = (slots + kOnChipChunks - 1) / kOnChipChunks;
+  GridDepWait();
+  GridDepLaunch();
+  // Everything the CTA reads is requested at once.
+#pragma unroll
+  for (int q = 0; q < kOnChipChunks; ++q) {
+    const int j1 = (q + 1) * per_chunk < n ? (q + 1) * per_chunk : n;
+    for (int j = q * per_chunk; j < j1; ++j) {
+      CpAsync16(mine + j * kOnChipThreads, xp + j * step);
+      if constexpr (kMode == kGrad) CpAsync16(mine_dy + j * kOnChipThreads, dp + j * step);
+    }
+    CpAsyncCommit();
+  }
+  // Per-channel inputs (thread c of the CTA: channel c0 + c), and the shift of
+  // this thread's pack: the first row of x (forward), the mean (gradient).
+  float scale_c = 0.0f, offset_c = 0.0f, mean_c = 0.0f, var_c = 0.0f, shift_c = 0.0f;
+  if (tid < seg) {
+    scale_c = a.scale[c0 + tid];
+    if constexpr (kMode == kFwd) {
+      offset_c = a.offset[c0 + tid];
+      shift_c = ToF32(x[c0 + tid]);
+    } else {
+      mean_c = a.mean[c0 + tid];
+      var_c = a.variance[c0 + tid];
+    }
+  }
+  float2 nshift[kPairs], a1[kPairs], a2[kPairs];
+#pragma unroll
+  for (int q = 0; q < kPairs; ++q) {
+    nshift[q] = a1[q] = a2[q] = make_float2(0.0f, 0.0f);
+  }
+  if (col < cv) {
+    if constexpr (kMode == kFwd) {
+      const P row0 = *(reinterpret_cast<const P*>(x) + col);
+      WidenPack<kVec>(row0, nshift);
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) nshift[q] = Neg2(nshift[q]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        nshift[q] = make_float2(-a.mean[col * kVec + 2 * q], -a.mean[col * kVec + 2 * q + 1]);
+      }
+    }
+  }
+  const auto Accumulate = [&](int j) {
+    const uint4 rx = mine[j * kOnChipThreads];
+    float2 xv[kPairs], gv[kPairs];
+    WidenPack<kVec>(*reinterpret_cast<const P*>(&rx), xv);
+    if constexpr (kMode == kGrad) {
+      const uint4 rd = mine_dy[j * kOnChipThreads];
+      WidenPack<kVec>(*reinterpret_cast<const P*>(&rd), gv);
+    }
+#pragma unroll
+    for (int q = 0; q < kPairs; ++q) {
+      const float2 d = Add2(xv[q], nshift[q]);
+      if constexpr (kMode == kFwd) {
+        a1[q] = Add2(a1[q], d);
+        a2[q] = Fma2(d, d, a2[q]);
+      } else {
+        a1[q] = Add2(a1[q], gv[q]);
+        a2[q] = Fma2(gv[q], d, a2[q]);
+      }
+    }
+  };
+  // A thread reads back only the slots that it filled itself: its own wait for
+  // its copies is all the synchronisation.
+#pragma unroll
+  for (int q = 0; q < kOnChipChunks; ++q) {
+    if (q == 0) CpAsyncWait<kOnChipChunks - 1>();
+    if (q == 1) CpAsyncWait<kOnChipChunks - 2>();
+    if (q == 2) CpAsyncWait<kOnChipChunks - 3>();
+    if (q == 3) CpAsyncWait<0>();
+    const int j1 = (q + 1) * per_chunk < n ? (q + 1) * per_chunk : n;
+#pragma unroll 2
+    for (int j = q * per_chunk; j < j1; ++j) Accumulate(j);
+  }
+
+  // Row lanes of a warp (threads tx apart share a column), warps of the CTA,
+  // CTAs of the cluster: a fixed order of adds at each level.
+#pragma unroll
+  for (int q = 0; q < kPairs; ++q) {
+    for (int m = 16; m >= TX; m >>= 1) {
+      a1[q].x += __shfl_xor_sync(0xffffffffu, a1[q].x, m);
+      a1[q].y += __shfl_xor_sync(0xffffffffu, a1[q].y, m);
+      a2[q].x += __shfl_xor_sync(0xffffffffu, a2[q].x, m);
+      a2[q].y += __shfl_xor_sync(0xffffffffu, a2[q].y, m);
+    }
+  }
+  const int warp = tid >> 5, lane = tid & 31;
+  if (lane < TX) {
+#pragma unroll
+    for (int q = 0; q < kPairs; ++q) {
+      warp_sum[warp][lane * kVec + 2 * q] = a1[q].x;
+      warp_sum[warp][lane * kVec + 2 * q + 1] = a1[q].y;
+      warp_sum[warp][nch + lane * kVec + 2 * q] = a2[q].x;
+      warp_sum[warp][nch + lane * kVec + 2 * q + 1] = a2[q].y;
+    }
+  }
+  __syncthreads();
+  if (tid < 2 * nch) {
+    float acc = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kOnChipWarps; ++w) acc += warp_sum[w][tid];
+    part[tid] = acc;
+  }
+  ClusterArrive();
+  ClusterWait();
+  const int world = gridDim.y;
+  const bool writer = blockIdx.y == 0;
+  if (tid < seg) {
+    double S1, S2;
+    ClusterTotals(part + tid, part + nch + tid, world, S1, S2);
+    const int64_t c = c0 + tid;
+    float ca, cb, cc = 0.0f;
+    if constexpr (kMode == kFwd) {
+      const double md = S1 * a.stat_out.inv_count;
+      const double m = static_cast<double>(shift_c) + md;
+      double v = S2 * a.stat_out.inv_count - md * md;
+      if (v < 0.0) v = 0.0;
+      mean_c = static_cast<float>(m);
+      var_c = static_cast<float>(v);
+      if (writer) WriteFwdStats(a.stat_out, c, m, v);
+      ca = scale_c * (1.0f / sqrtf(var_c + a.epsilon));
+      cb = offset_c;
+      if constexpr (kNarrow) cb = fmaf(-mean_c, ca, cb);
+    } else {
+      const float inv = 1.0f / sqrtf(var_c + a.epsilon);
+      const float t1 = static_cast<float>(S1), t2 = static_cast<float>(S2);
+      ca = scale_c * inv;
+      cb = a.fold_use ? t1 * a.inv_count : 0.0f;
+      cc = a.fold_use ? t2 * inv * inv * a.inv_count : 0.0f;
+      if (writer) {
+        a.doffset[c] = t1;
+        a.dscale[c] = t2 * inv;
+        WriteZeros(a.stat_out, c);
+      }
+      if constexpr (kNarrow) {
+        const float fb = -ca * cc;
+        const float fc = ca * fmaf(cc, mean_c, -cb);
+        cb = fb;
+        cc = fc;
+      }
+    }
+    coef[0][tid] = ca;
+    coef[1][tid] = cb;
+    coef[2][tid] = cc;
+    coef[3][tid] = -mean_c;
+  }
+  ClusterArrive();   // this CTA has read its neighbours' sums
+  __syncthreads();
+  if (n > 0) {
+    float2 A[kPairs], B[kPairs], C[kPairs], M[kPairs];
+#pragma unroll
+    for (int q = 0; q < kPairs; ++q) {
+      const int e = tx * kVec + 2 * q;
+      A[q] = make_float2(coef[0][e], coef[0][e + 1]);
+      B[q] = make_float2(coef[1][e], coef[1][e + 1]);
+      C[q] = make_float2(coef[2][e], coef[2][e + 1]);
+      M[q] = make_float2(coef[3][e], coef[3][e + 1]);
+    }
+    P* op = reinterpret_cast<P*>(out) + first;
+#pragma unroll 2
+    for (int j = 0; j < n; ++j) {
+      const uint4 rx = mine[j * kOnChipThreads];
+      float2 xv[kPairs], gv[kPairs], rv[kPairs];
+      WidenPack<kVec>(*reinterpret_cast<const P*>(&rx), xv);
+      if constexpr (kMode == kGrad) {
+        const uint4 rd = mine_dy[j * kOnChipThreads];
+        WidenPack<kVec>(*reinterpret_cast<const P*>(&rd), gv);
+      }
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        if constexpr (kNarrow && kMode == kFwd) {
+          rv[q] = Fma2(xv[q], A[q], B[q]);
+        } else if constexpr (kNarrow) {
+          rv[q] = Fma2(gv[q], A[q], Fma2(xv[q], B[q], C[q]));
+        } else {
+          const float2 d = Add2(xv[q], M[q]);
+          if constexpr (kMode == kFwd) {
+            rv[q] = Fma2(d, A[q], B[q]);
+          } else {
+            rv[q] = Mul2(A[q], Fma2(Neg2(d), C[q], Add2(gv[q], Neg2(B[q]))));
+          }
+        }
+      }
+      P o;
+      NarrowPack<kVec>(rv, o);
+      StoreStream(op + j * step, o);
+    }
+  }
+  ClusterWait();   // nobody leaves while a neighbour still reads its sums
+}
+
+// The same for channel-major tensors ([outer, C, inner], inner > 1).  A cluster
+// owns `group` neighbouring channels, whose planes are one run of
+// group * inner / kVec whole packs per n; the outer axis is cut over its CTAs.
+// A group of several channels has runs of at most 512 packs: thread (lane_n, p)
+// keeps pack p of the run for n = n0 + lane_n, + lanes, ...: the pack covers
+// channel lo and, where the planes are not whole packs, maybe the start of
+// lo + 1, the same two for every n.  A single channel (planes of whole packs, of
+// any length) is walked as one flattened sequence of packs, 512 apart.
+constexpr int kOnChipMaxGroup = 16;
+
+template <typename T, int kMode>
+__global__ void __launch_bounds__(kOnChipThreads, 1)
+    BnOnChipPlanesKernel(const T* x, const T* dy, T* out, ApplyArgs a, int64_t outer,
+                         int64_t channels, int inner, int group, int64_t outer_per_cta,
+                         int slots) {
+  constexpr int kVec = VecWidth<T>::value;
+  constexpr int kPairs = kVec / 2;
+  using P = Pack<T, kVec>;
+  extern __shared__ uint4 onchip_tile[];   // [stream][slot][thread]
+  __shared__ float4 contrib[kOnChipThreads];   // (s1, s2) of lo, (s1, s2) of lo + 1
+  __shared__ float2 warp_sum[kOnChipWarps];
+  __shared__ float part[2 * kOnChipMaxGroup];
+  __shared__ float shift_s[kOnChipMaxGroup + 1];
+  __shared__ float4 coef[kOnChipMaxGroup + 1];   // -mean, ca, cb, cc
+  const int tid = threadIdx.x;
+  const bool flat = group == 1;
+  const int run = group * inner / kVec;
+  const int lanes = flat ? 1 : kOnChipThreads / run;   // (of the walk by n)
+  const int lane_n = tid / run, p = tid - lane_n * run;
+  const int64_t c0 = static_cast<int64_t>(blockIdx.x) * group;
+  const int64_t n0 = static_cast<int64_t>(blockIdx.y) * outer_per_cta;
+  const int64_t n1 = n0 + outer_per_cta < outer ? n0 + outer_per_cta : outer;
+  const int64_t plane_set = channels * inner;   // elements between consecutive n
+  int n = 0;                                    // this thread's packs
+  if (flat) {
+    const int64_t left = (n1 - n0) * run - tid;
+    if (left > 0) n = static_cast<int>((left + kOnChipThreads - 1) / kOnChipThreads);
+  } else if (lane_n < lanes) {
+    const int64_t left = n1 - n0 - lane_n;
+    if (left > 0) n = static_cast<int>((left + lanes - 1) / lanes);
+  }
+  // Where the next pack is: `inc` elements on, and across the end of a plane
+  // (flat walk only) `wrap` more.
+  const int64_t first = (n0 + lane_n) * plane_set + c0 * inner + static_cast<int64_t>(p) * kVec;
+  const int di = flat ? kOnChipThreads % run : 0;
+  const int64_t inc = flat ? kOnChipThreads / run * plane_set + di * kVec : lanes * plane_set;
+  const int64_t wrap = plane_set - static_cast<int64_t>(run) * kVec;
+  const auto Advance = [&](int64_t& at, int& pos) {
+    at += inc;
+    pos += di;
+    if (pos >= run) {
+      pos -= run;
+      at += wrap;
+    }
+  };
+  uint4* const mine = onchip_tile + tid;
+  uint4* const mine_dy = mine + slots * kOnChipThreads;
+  const int per_chunk = (slots + kOnChipChunks - 1) / kOnChipChunks;
+  GridDepWait();
+  GridDepLaunch();
+  {
+    int64_t at = first;
+    int pos = p;
+#pragma unroll
+    for (int q = 0; q < kOnChipChunks; ++q) {
+      const int j1 = (q + 1) * per_chunk < n ? (q + 1) * per_chunk : n;
+      for (int j = q * per_chunk; j < j1; ++j) {
+        CpAsync16(mine + j * kOnChipThreads, x + at);
+        if constexpr (kMode == kGrad) CpAsync16(mine_dy + j * kOnChipThreads, dy + at);
+        Advance(at, pos);
+      }
+      CpAsyncCommit();
+    }
+  }
+  float scale_c = 0.0f, offset_c = 0.0f, mean_c = 0.0f, var_c = 0.0f, shift_c = 0.0f;
+  if (tid < group) {
+    const int64_t c = c0 + tid;
+    scale_c = a.scale[c];
+    if constexpr (kMode == kFwd) {
+      offset_c = a.offset[c];
+      shift_c = ToF32(x[c * inner]);
+    } else {
+      mean_c = a.mean[c];
+      var_c = a.variance[c];
+      shift_c = mean_c;
+    }
+    shift_s[tid] = shift_c;
+  }
+  if (tid == group) shift_s[group] = 0.0f;
+  __syncthreads();
+  int lo = 0, before = kVec;
+  if (n > 0 && !flat) GroupSlot(p, inner, kVec, &lo, &before);
+  const bool whole = before >= kVec;
+  const float sh_lo = shift_s[lo], sh_hi = shift_s[lo + 1];
+  const float2 nshift = make_float2(-sh_lo, -sh_lo);
+  float2 a1 = make_float2(0.0f, 0.0f), a2 = make_float2(0.0f, 0.0f);
+  float s1h = 0.0f, s2h = 0.0f;
+  const auto Accumulate = [&](int j) {
+    const uint4 rx = mine[j * kOnChipThreads];
+    float2 xv[kPairs], gv[kPairs];
+    WidenPack<kVec>(*reinterpret_cast<const P*>(&rx), xv);
+    if constexpr (kMode == kGrad) {
+      const uint4 rd = mine_dy[j * kOnChipThreads];
+      WidenPack<kVec>(*reinterpret_cast<const P*>(&rd), gv);
+    }
+    if (whole) {
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        const float2 d = Add2(xv[q], nshift);
+        if constexpr (kMode == kFwd) {
+          a1 = Add2(a1, d);
+          a2 = Fma2(d, d, a2);
+        } else {
+          a1 = Add2(a1, gv[q]);
+          a2 = Fma2(gv[q], d, a2);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < kVec; ++e) {
+        const bool in_lo = e < before;
+        const float v = (e & 1) ? xv[e / 2].y : xv[e / 2].x;
+        const float d = v - (in_lo ? sh_lo : sh_hi);
+        float t1, t2;
+        if constexpr (kMode == kFwd) {
+          t1 = d;
+          t2 = d * d;
+        } else {
+          t1 = (e & 1) ? gv[e / 2].y : gv[e / 2].x;
+          t2 = t1 * d;
+        }
+        if (in_lo) {
+          a1.x += t1;
+          a2.x += t2;
+        } else {
+          s1h += t1;
+          s2h += t2;
+        }
+      }
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < kOnChipChunks; ++q) {
+    if (q == 0) CpAsyncWait<kOnChipChunks - 1>();
+    if (q == 1) CpAsyncWait<kOnChipChunks - 2>();
+    if (q == 2) CpAsyncWait<kOnChipChunks - 3>();
+    if (q == 3) CpAsyncWait<0>();
+    const int j1 = (q + 1) * per_chunk < n ? (q + 1) * per_chunk : n;
+    for (int j = q * per_chunk; j < j1; ++j) Accumulate(j);
+  }
+  contrib[tid] = make_float4(a1.x + a1.y, a2.x + a2.y, s1h, s2h);
+  __syncthreads();
+  // Channel k: 512 / group threads (a power of two, at least a warp) add the
+  // entries of its packs, then shuffles, then the channel's warps in order.
+  {
+    const int width = kOnChipThreads / group;
+    const int k = tid / width, w = tid - k * width;
+    const int p_first = k * inner / kVec;
+    const int packs = ((k + 1) * inner - 1) / kVec - p_first + 1;
+    float t1 = 0.0f, t2 = 0.0f;
+    if (flat) {
+      t1 = a1.x + a1.y;
+      t2 = a2.x + a2.y;
+    }
+    for (int i = w; !flat && i < packs * lanes; i += width) {
+      const int ln = i / packs;
+      const int pk = p_first + i - ln * packs;
+      const float4 v = contrib[ln * run + pk];
+      const bool is_lo = pk * kVec / inner == k;   // else the pack crosses into k from k - 1
+      t1 += is_lo ? v.x : v.z;
+      t2 += is_lo ? v.y : v.w;
+    }
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+      t1 += __shfl_xor_sync(0xffffffffu, t1, m);
+      t2 += __shfl_xor_sync(0xffffffffu, t2, m);
+    }
+    if ((tid & 31) == 0) warp_sum[tid >> 5] = make_float2(t1, t2);
+    __syncthreads();
+    if (tid < group) {
+      const int per = kOnChipWarps / group;
+      t1 = 0.0f;
+      t2 = 0.0f;
+      for (int q = 0; q < per; ++q) {
+        t1 += warp_sum[tid * per + q].x;
+        t2 += warp_sum[tid * per + q].y;
+      }
+      part[tid] = t1;
+      part[kOnChipMaxGroup + tid] = t2;
+    }
+  }
+  ClusterArrive();
+  ClusterWait();
+  if (tid < group) {
+    double S1, S2;
+    ClusterTotals(part + tid, part + kOnChipMaxGroup + tid, gridDim.y, S1, S2);
+    const int64_t c = c0 + tid;
+    const bool writer = blockIdx.y == 0;
+    float cb, cc = 0.0f;
+    if constexpr (kMode == kFwd) {
+      const double md = S1 * a.stat_out.inv_count;
+      const double m = static_cast<double>(shift_c) + md;
+      double v = S2 * a.stat_out.inv_count - md * md;
+      if (v < 0.0) v = 0.0;
+      mean_c = static_cast<float>(m);
+      var_c = static_cast<float>(v);
+      if (writer) WriteFwdStats(a.stat_out, c, m, v);
+      cb = offset_c;
+    }
+    const float inv = 1.0f / sqrtf(var_c + a.epsilon);
+    if constexpr (kMode == kGrad) {
+      const float t1 = static_cast<float>(S1), t2 = static_cast<float>(S2);
+      cb = a.fold_use ? t1 * a.inv_count : 0.0f;
+      cc = a.fold_use ? t2 * inv * inv * a.inv_count : 0.0f;
+      if (writer) {
+        a.doffset[c] = t1;
+        a.dscale[c] = t2 * inv;
+        WriteZeros(a.stat_out, c);
+      }
+    }
+    coef[tid] = make_float4(-mean_c, scale_c * inv, cb, cc);
+  }
+  if (tid == group) coef[group] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  ClusterArrive();   // this CTA has read its neighbours' sums
+  __syncthreads();
+  if (n > 0) {
+    const float4 kl = coef[lo], kh = coef[lo + 1];
+    int64_t at = first;
+    int pos = p;
+    for (int j = 0; j < n; ++j) {
+      const uint4 rx = mine[j * kOnChipThreads];
+      float2 xv[kPairs], gv[kPairs], rv[kPairs];
+      WidenPack<kVec>(*reinterpret_cast<const P*>(&rx), xv);
+      if constexpr (kMode == kGrad) {
+        const uint4 rd = mine_dy[j * kOnChipThreads];
+        WidenPack<kVec>(*reinterpret_cast<const P*>(&rd), gv);
+      }
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        const bool lx = 2 * q < before, ly = 2 * q + 1 < before;
+        const float2 d = Add2(xv[q], make_float2(lx ? kl.x : kh.x, ly ? kl.x : kh.x));
+        const float2 A = make_float2(lx ? kl.y : kh.y, ly ? kl.y : kh.y);
+        const float2 B = make_float2(lx ? kl.z : kh.z, ly ? kl.z : kh.z);
+        if constexpr (kMode == kFwd) {
+          rv[q] = Fma2(d, A, B);
+        } else {
+          const float2 C = make_float2(lx ? kl.w : kh.w, ly ? kl.w : kh.w);
+          rv[q] = Mul2(A, Fma2(Neg2(d), C, Add2(gv[q], Neg2(B))));
+        }
+      }
+      P o;
+      NarrowPack<kVec>(rv, o);
+      StoreStream(reinterpret_cast<P*>(out + at), o);
+      Advance(at, pos);
+    }
+  }
+  ClusterWait();   // nobody leaves while a neighbour still reads its sums
+}
+
 // ------------------------------------------------------------ host side --
 
 template <typename T>
@@ -2183,6 +2723,156 @@ inline bool ApplyAddsRows(const Geom& g, int rows) {
   return bytes >= 0 && bytes <= kApplyFoldSmemMax;
 }
 
+// ---- The one-kernel form: which layers take it and how they are cut.
+struct OnChipPlan {
+  int tx = 0;        // channel packs per column block, or channels per group; 0: not this form
+  int cluster = 0;   // CTAs per cluster = pieces of the outer axis
+  int gx = 0;        // column blocks or channel groups
+  int slots = 0;     // 16-byte slots per thread and stream
+  int64_t per_cta = 0;
+  double cost = 0.0;
+};
+
+// Clusters of `cluster` CTAs of `kernel` that are resident at once with all the
+// shared memory the form may take (0: such a launch is not possible).
+template <typename Kernel>
+inline int OnChipClusters(Kernel kernel, std::atomic<int> (*by_device)[kMaxDevices],
+                          int cluster) {
+  int slot = 0;
+  while ((1 << slot) < cluster) ++slot;
+  const int found = PerDevice(by_device[slot], [&] {
+    constexpr int kBytes = kOnChipSlots * kOnChipThreads * 16;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      return -1;
+    }
+    if (cluster == 1) return SmCount();
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    ClusterConfig(&cfg, attr, false, cluster, dim3(1, cluster), dim3(kOnChipThreads), kBytes,
+                  nullptr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return -1;
+    }
+    return n > 0 ? n : -1;
+  });
+  return found > 0 ? found : 0;
+}
+
+// Relative cost of a cut, in slots of 8 KB that a CTA streams in and out (about
+// 0.2 us each): a cluster barrier counts as 3.5 of them (K = 1 against 2 on
+// fp32 [98,2048]: 3.2 and 4.1 us), rows cut into segments of 64 and 32 bytes
+// cost 8 and 25 % (bf16 [25088,256] 10.9 us at 128 bytes, 11.5 at 64).
+inline double OnChipCost(int64_t slots, int k, double segments) {
+  return static_cast<double>(slots) * segments + (k > 1 ? 3.5 : 0.0);
+}
+
+template <typename T>
+inline bool OnChipAllowed(const Geom& g, int streams) {
+  if (GetTuning(kTuneBnOnChipTx) < 0) return false;
+  // A sweep of the chain's own keys wants the chain.
+  if (GetTuning(kTuneBnClusterFold) != 0 || GetTuning(kTuneBnApplyAddsRows) != 64) return false;
+  return g.outer * g.channels * g.inner * static_cast<int64_t>(sizeof(T)) * streams <
+         kOnChipMaxBytes;
+}
+
+// One cut into the plan if it is possible and the best so far: `gx` column
+// blocks, `per` of the outer axis for each of `k` CTAs.
+template <typename Kernel>
+inline void OnChipTry(OnChipPlan* best, Kernel kernel, std::atomic<int> (*by_device)[kMaxDevices],
+                      int tx, int64_t gx, int k, int64_t per, int64_t slots, int streams,
+                      double segments) {
+  if (slots * streams > kOnChipSlots) return;
+  const double cost = OnChipCost(slots * streams, k, segments);
+  if (best->tx != 0 && cost >= best->cost) return;
+  if (gx > OnChipClusters(kernel, by_device, k)) return;
+  *best = OnChipPlan{tx, k, static_cast<int>(gx), static_cast<int>(slots), per, cost};
+}
+
+// Channels-last (the geometry of VectorChain).
+template <typename T, int kMode>
+inline OnChipPlan PlanOnChip(const Geom& g) {
+  static std::atomic<int> by_device[5][kMaxDevices];   // cluster sizes 1, 2, 4, 8, 16
+  OnChipPlan best;
+  constexpr int kStreams = kMode == kFwd ? 1 : 2;
+  if (!OnChipAllowed<T>(g, kStreams)) return best;
+  const int forced_tx = GetTuning(kTuneBnOnChipTx), forced_k = GetTuning(kTuneBnOnChipCluster);
+  const int64_t cv = g.channels / VecWidth<T>::value;
+  const int widest = PlanTx(cv, kOnChipMaxTx);
+  for (int tx = widest; tx >= 1; tx >>= 1) {
+    if (tx == 1 && widest > 1) continue;   // whole 32-byte sectors
+    if (forced_tx > 0 && tx != forced_tx) continue;
+    const int64_t gx = CeilDiv(cv, tx);
+    for (int k = 1; k <= kOnChipMaxCluster; k <<= 1) {
+      if (forced_k > 0 && k != forced_k) continue;
+      const int64_t per = CeilDiv(g.outer, k);
+      const int64_t slots = CeilDiv(per, kOnChipThreads / tx);
+      // Few channels and many rows: too few CTAs to keep up with the chain
+      // (bf16 [100352,64], 64 CTAs of 25 slots: 15.4 us against 11.8;
+      // fp32 [65536,32], 16 slots: 10.2 against 9.2).
+      if (tx < 4 && gx * k < 100 && slots * kStreams > 12) continue;
+      OnChipTry(&best, BnOnChipKernel<T, kMode>, by_device, tx, gx, k, per, slots, kStreams,
+                tx < 4 ? 1.25 : tx < 8 ? 1.08 : 1.0);
+    }
+  }
+  return best;
+}
+
+// Channel-major: groups of channels whose planes are whole packs together.
+template <typename T, int kMode>
+inline OnChipPlan PlanOnChipPlanes(const Geom& g, const void* x, const void* out,
+                                   const void* dy) {
+  static std::atomic<int> by_device[5][kMaxDevices];
+  OnChipPlan best;
+  constexpr int kStreams = kMode == kFwd ? 1 : 2;
+  constexpr int kVec = VecWidth<T>::value;
+  if (g.inner <= 1 || !OnChipAllowed<T>(g, kStreams)) return best;
+  if (!Aligned16(x) || !Aligned16(out) || (dy != nullptr && !Aligned16(dy))) return best;
+  const int forced_tx = GetTuning(kTuneBnOnChipTx), forced_k = GetTuning(kTuneBnOnChipCluster);
+  for (int group = 1; group <= kOnChipMaxGroup; group <<= 1) {
+    if (forced_tx > 0 && group != forced_tx) continue;
+    const int64_t run = group * g.inner / kVec;
+    if (group * g.inner % kVec != 0 || g.channels % group != 0) continue;
+    if (group > 1 && run > kOnChipThreads) continue;
+    // A pack may reach into the next channel, not beyond it.
+    if (g.inner < kVec) continue;
+    for (int k = 1; k <= kOnChipMaxCluster; k <<= 1) {
+      if (forced_k > 0 && k != forced_k) continue;
+      const int64_t per = CeilDiv(g.outer, k);
+      const int64_t slots = group == 1 ? CeilDiv(per * run, kOnChipThreads)
+                                       : CeilDiv(per, kOnChipThreads / run);
+      OnChipTry(&best, BnOnChipPlanesKernel<T, kMode>, by_device, group, g.channels / group, k,
+                per, slots, kStreams, run < 8 ? 1.25 : 1.0);
+    }
+  }
+  return best;
+}
+
+template <typename T, int kMode>
+int LaunchOnChip(const OnChipPlan& p, const T* x, const T* dy, T* out, const ApplyArgs& a,
+                 const Geom& g, cudaStream_t stream) {
+  const size_t smem = static_cast<size_t>(p.slots) * (kMode == kFwd ? 1 : 2) * kOnChipThreads * 16;
+  const bool pdl = GetTuning(kTuneBnPdl) != 0;
+  const dim3 grid(p.gx, p.cluster);
+  cudaError_t err;
+  if (g.inner == 1) {
+    err = LaunchClustered(pdl, p.cluster, BnOnChipKernel<T, kMode>, grid,
+                          dim3(p.tx, kOnChipThreads / p.tx), smem, stream, x, dy, out, a, g.outer,
+                          g.channels / VecWidth<T>::value, g.channels, p.per_cta, p.slots);
+  } else {
+    err = LaunchClustered(pdl, p.cluster, BnOnChipPlanesKernel<T, kMode>, grid,
+                          dim3(kOnChipThreads), smem, stream, x, dy, out, a, g.outer, g.channels,
+                          static_cast<int>(g.inner), p.tx, p.per_cta, p.slots);
+  }
+  if (err != cudaSuccess) cudaGetLastError();
+  return static_cast<int>(err);
+}
+
 template <typename T>
 int FwdTrain(const void* x, const float* scale, const float* offset,
              const float* est_mean, const float* est_var, void* y,
@@ -2227,6 +2917,13 @@ int FwdTrain(const void* x, const float* scale, const float* offset,
   a.mean = saved_mean;
   a.variance = saved_var;
   a.epsilon = epsilon;
+  const OnChipPlan p = VectorChain<T>(g, x, y, nullptr)
+                           ? PlanOnChip<T, kFwd>(g)
+                           : PlanOnChipPlanes<T, kFwd>(g, x, y, nullptr);
+  if (p.tx > 0) {
+    a.stat_out = f;
+    return LaunchOnChip<T, kFwd>(p, xt, nullptr, static_cast<T*>(y), a, g, stream);
+  }
   // (An in-place call, y == x, keeps the finalize kernel: the element-wise
   // kernel would otherwise re-read the first row of x, the shift of the sums,
   // while other CTAs already overwrite it.)
@@ -2316,6 +3013,15 @@ int Grad(const void* dy, const void* x, const float* scale, const float* mean,
   a.sums = is_training ? sums : nullptr;
   a.inv_count = static_cast<float>(1.0 / static_cast<double>(g.rows()));
   const bool vector_chain = VectorChain<T>(g, x, dx, dy);
+  const OnChipPlan p = vector_chain ? PlanOnChip<T, kGrad>(g)
+                                    : PlanOnChipPlanes<T, kGrad>(g, x, dx, dy);
+  if (p.tx > 0) {
+    a.fold_use = is_training;
+    a.dscale = dscale;
+    a.doffset = doffset;
+    a.stat_out = f;
+    return LaunchOnChip<T, kGrad>(p, xt, dyt, static_cast<T*>(dx), a, g, stream);
+  }
   int fold = vector_chain ? GetTuning(kTuneBnClusterFold) : 1;
   const int splits = LaunchStats<T, kGrad>(xt, dyt, mean, partial, g, nullptr, stream, &fold);
   if (splits < 0) return DecodeError(splits);

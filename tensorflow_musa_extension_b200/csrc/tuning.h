@@ -8,7 +8,8 @@ namespace musa_b200 {
 enum TuningKey {
   kTuneAdamCtasPerSm = 0,   // 0: one tile per CTA; k: persistent, k CTAs per SM
   kTuneAdamUnroll = 1,      // packs in flight per thread and stream: 1, 2, 4
-                            // 2, 3: not in use
+  kTuneBnOnChipTx = 2,      // channel packs per column block of the one-kernel form; 0: by rule, -1: off
+  kTuneBnOnChipCluster = 3, // CTAs per cluster of the one-kernel form; 0: by rule
   kTuneBnCtasPerSm = 4,     // CTAs per SM of the BatchNorm statistics grids; 0: what fits
   kTuneBnClusterFold = 5,   // CTAs per cluster of the stats kernel that fold their partial rows on chip
                             // (the element-wise kernel adds the rest: no finalize kernel); 0, 1: off

@@ -653,3 +653,66 @@ def test_outputs_beside_the_statistics(kernel_lib, dtype, shape, layout):
             training, ws.data_ptr(), ws.numel(), st) == 0
         assert all(bool(torch.isfinite(t).all()) for t in outs[:2])
         assert not outs[2].any() and not outs[3].any()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("cluster", [0, 1, 2, 8, 16])
+@pytest.mark.parametrize("shape,layout", [
+    ((1, 8), "NHWC"), ((2, 16), "NHWC"), ((511, 24), "NHWC"), ((1000, 520), "NHWC"),
+    ((6272, 64), "NHWC"), ((12800, 16), "NHWC"), ((12801, 16), "NHWC"),
+    ((1, 16, 7, 7), "NCHW"), ((3, 8, 4, 4), "NCHW"), ((37, 24, 3, 5), "NCHW"),
+    ((64, 32, 14, 14), "NCHW"), ((20, 2, 28, 28), "NCHW"), ((6, 2, 56, 56), "NCHW"), ((3, 5, 8, 11), "NCHW"), ((250, 8, 7, 7), "NCHW"),
+])
+def test_one_kernel_form(kernel_lib, dtype, cluster, shape, layout):
+    """The one-kernel form (inputs held in shared memory, sums met over a
+    cluster) against the oracle and against the chain of kernels, at the edges
+    of its cuts: a single row, partly filled column blocks, CTAs without rows,
+    the last row slot; key 3 forces the cluster size (sizes that cannot hold
+    the layer fall back to the chain), key 2 = -1 turns the form off."""
+    c = shape[-1] if layout == "NHWC" else shape[1]
+    axis = -1 if layout == "NHWC" else 1
+    x, s, o, dy = bn_inputs(70 + c, shape, dtype, 1.0, 3.0, channel_axis=axis)
+    gen = np.random.default_rng(c)
+    rm = gen.standard_normal(c).astype(np.float32)
+    rv = (gen.random(c) + 0.5).astype(np.float32)
+    want = np_ref.fused_batch_norm(x, s, o, rm, rv, epsilon=EPS, exponential_avg_factor=0.25,
+                                   data_format=layout)
+    wg = np_ref.fused_batch_norm_grad(dy, x, s, want[3], want[4], EPS, layout)
+    terms = _rms(dy) * float(np.max(s / np.sqrt(want[4] + EPS)))
+
+    def run():
+        tx = to_torch(x)
+        fwd = raw_ops.FusedBatchNormV3(tx, to_torch(s), to_torch(o), to_torch(rm), to_torch(rv),
+                                       epsilon=EPS, exponential_avg_factor=0.25,
+                                       data_format=layout)
+        args = (to_torch(dy), tx, to_torch(s), fwd.reserve_space_1, fwd.reserve_space_2, None,
+                EPS, layout)
+        grad = raw_ops.FusedBatchNormGradV3(*args)
+        frozen = raw_ops.FusedBatchNormGradV3(*args, is_training=False)
+        torch.cuda.synchronize()
+        return fwd, grad, frozen
+
+    old = kernel_lib.MusaKernelsSetTuning(3, cluster)
+    try:
+        before = kernel_lib.MusaKernelsLaunchCount()
+        fwd, grad, frozen = run()
+        launches = kernel_lib.MusaKernelsLaunchCount() - before
+        again = run()
+    finally:
+        kernel_lib.MusaKernelsSetTuning(3, old)
+    if cluster == 0:
+        assert launches == 3     # every shape of this list takes the form
+    off = kernel_lib.MusaKernelsSetTuning(2, -1)
+    try:
+        chain = run()
+    finally:
+        kernel_lib.MusaKernelsSetTuning(2, off)
+    check_forward(fwd, want, dtype)
+    check_grad(grad, wg, dtype, dx_scale=terms)
+    for a, b in zip((*fwd, *grad, *frozen), (t for out in again for t in out)):
+        assert torch.equal(a, b)
+    for a, b in zip((*fwd[1:], *grad[1:], *frozen[1:]),
+                    (t for out in chain for t in out[1:])):
+        a, b = to_numpy(a).astype(np.float64), to_numpy(b).astype(np.float64)
+        assert np.all(np.abs(a - b) <= 1e-5 * np.abs(b) + 1e-5 * max(_rms(b), 1e-12))
+    check_grad(frozen, tuple(to_numpy(t) for t in chain[2][:3]), dtype, dx_scale=terms)
