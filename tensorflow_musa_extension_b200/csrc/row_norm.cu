@@ -95,6 +95,46 @@ __device__ __forceinline__ float2 GroupSum2(float2 v, float2* smem, int& parity)
   return v;
 }
 
+// Four sums at once (`v`, `w`): one latency for both pairs.  Groups wider than a
+// warp use two scratch rows per call, so successive calls need no parity
+// beyond that of GroupSum2.
+template <int kGroup, int kThreads>
+__device__ __forceinline__ void GroupSum4(float2& v, float2& w, float2* smem, int& parity) {
+  constexpr int kWarpSpan = kGroup < 32 ? kGroup : 32;
+#pragma unroll
+  for (int m = kWarpSpan / 2; m > 0; m >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, m);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, m);
+    w.x += __shfl_xor_sync(0xffffffffu, w.x, m);
+    w.y += __shfl_xor_sync(0xffffffffu, w.y, m);
+  }
+  if constexpr (kGroup > 32) {
+    constexpr int kWarps = kGroup / 32;
+    constexpr int kAll = kThreads / 32;
+    const int warp = threadIdx.x >> 5;
+    const int first = (warp / kWarps) * kWarps;
+    float2* row = smem + parity * kAll;             // first pair
+    float2* row_w = smem + (2 + parity) * kAll;     // second pair
+    parity ^= 1;
+    if ((threadIdx.x & 31) == 0) {
+      row[warp] = v;
+      row_w[warp] = w;
+    }
+    GroupMeet<kGroup, kThreads>();
+    float2 t = make_float2(0.0f, 0.0f), u = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) {
+      const float2 o = row[first + i], q = row_w[first + i];
+      t.x += o.x;
+      t.y += o.y;
+      u.x += q.x;
+      u.y += q.y;
+    }
+    v = t;
+    w = u;
+  }
+}
+
 template <int kGroup, int kThreads>
 __device__ __forceinline__ float GroupSum(float v, float2* smem, int& parity) {
   constexpr int kWarpSpan = kGroup < 32 ? kGroup : 32;
@@ -190,6 +230,15 @@ constexpr int RowMinCtas(int group, int op, int max_packs, int elem_bytes) {
   return 1;
 }
 
+// The LayerNorm gradient takes its two sums over g = dy * gamma in the same
+// round as the second sum over x: two dependent rounds a row instead of three
+// (bf16 [16384,1024] 24.8 -> 22.4 us, [65536,1024] 77.4 -> 68.2, [32768,2048]
+// 88.1 -> 80.8, [8192,8192] 99.0 -> 90.1) - except where the four partial sums
+// spill (256-thread groups of three 16-bit packs: rows of 5120 102 -> 111 us).
+__host__ __device__ constexpr bool RowMergesSums(int group, int max_packs, int elem_bytes) {
+  return !(group == 256 && max_packs == 3 && elem_bytes == 2);
+}
+
 template <typename T, int kGroup, int kMaxPacks, int kOp, bool kFull>
 __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
                                   RowMinCtas(kGroup, kOp, kMaxPacks, sizeof(T)))
@@ -203,7 +252,8 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
   constexpr int kPairs = kVec / 2;
   constexpr int kQuads = kVec / 4;
   using P = Pack<T, kVec>;
-  __shared__ float2 red[2 * (kThreads / 32)];
+  // Two rows by parity; two more for the second pair of GroupSum4.
+  __shared__ float2 red[(kOp == kOpLnGrad ? 4 : 2) * (kThreads / 32)];
   int parity = 0;
   // Ring: [stage][input][pack j][thread], 16 bytes each.  After the ring:
   // gamma (and beta for the LayerNorm forward) widened to fp32 once per CTA,
@@ -254,14 +304,6 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
   GridDepWait();
   GridDepLaunch();
 
-  for (int c = threadIdx.x; c < a.row_size; c += kThreads) {
-    const int e = c % kVec;
-    const int at = ((e / 4) * packs + c / kVec) * 4 + (e & 3);
-    gsm[at] = ToF32(static_cast<const T*>(a.gamma)[c]);
-    if constexpr (kOp == kOpLnFwd) bsm[at] = ToF32(static_cast<const T*>(a.beta)[c]);
-  }
-  __syncthreads();
-
   const int64_t n_blocks = (a.rows + kRows - 1) / kRows;
   // Queues the copies of row block `rb` into ring stage `stage`; always one
   // commit group, empty when there is nothing to copy.
@@ -287,6 +329,15 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
   for (int s = 0; s < kStages - 1; ++s) {
     request(static_cast<int64_t>(blockIdx.x) + static_cast<int64_t>(s) * gridDim.x, s);
   }
+  // gamma / beta while the first rows are on their way (filled before them they
+  // put a memory round trip in front of every launch).
+  for (int c = threadIdx.x; c < a.row_size; c += kThreads) {
+    const int e = c % kVec;
+    const int at = ((e / 4) * packs + c / kVec) * 4 + (e & 3);
+    gsm[at] = ToF32(static_cast<const T*>(a.gamma)[c]);
+    if constexpr (kOp == kOpLnFwd) bsm[at] = ToF32(static_cast<const T*>(a.beta)[c]);
+  }
+  __syncthreads();
 
   int stage = 0;
   for (int64_t rb = blockIdx.x; rb < n_blocks; rb += gridDim.x) {
@@ -339,6 +390,21 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
       const float mean0 = GroupSum<kGroup, kThreads>(s2.x + s2.y, red, parity) * inv_n;
       const float2 nmean0 = Dup(-mean0);
       float2 r2 = make_float2(0.0f, 0.0f), q2 = make_float2(0.0f, 0.0f);
+      // The gradient's sums over g = dy * gamma, pack j: with x_hat = r * inv_std
+      // + shift, sum(g * x_hat) follows from sum(g) and sum(g * r).
+      float2 sg2 = make_float2(0.0f, 0.0f), sgr2 = make_float2(0.0f, 0.0f);
+      const auto GradSums = [&](int j) {
+        float2 gm[kPairs], dv[kPairs];
+        LoadRowVector(gsm, t + j * kGroup, gm);
+        WidenPack<kVec>(cd[j], dv);
+#pragma unroll
+        for (int q = 0; q < kPairs; ++q) {
+          const float2 g = Mul2(dv[q], gm[q]);
+          sg2 = Add2(sg2, g);
+          sgr2 = Fma2(g, xv[j][q], sgr2);
+        }
+      };
+      constexpr bool kMerged = kOp == kOpLnGrad && RowMergesSums(kGroup, kMaxPacks, sizeof(T));
 #pragma unroll
       for (int j = 0; j < kMaxPacks; ++j) {
         if (live && Has(j)) {
@@ -348,10 +414,25 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
             r2 = Add2(r2, xv[j][q]);
             q2 = Fma2(xv[j][q], xv[j][q], q2);
           }
+          if constexpr (kMerged) GradSums(j);
         }
       }
-      const float2 rq = GroupSum2<kGroup, kThreads>(
-          make_float2(r2.x + r2.y, q2.x + q2.y), red, parity);
+      float2 rq = make_float2(r2.x + r2.y, q2.x + q2.y);
+      float2 gs;
+      if constexpr (kMerged) {
+        gs = make_float2(sg2.x + sg2.y, sgr2.x + sgr2.y);
+        GroupSum4<kGroup, kThreads>(rq, gs, red, parity);
+      } else {
+        rq = GroupSum2<kGroup, kThreads>(rq, red, parity);
+        if constexpr (kOp == kOpLnGrad) {
+#pragma unroll
+          for (int j = 0; j < kMaxPacks; ++j) {
+            if (live && Has(j)) GradSums(j);
+          }
+          gs = GroupSum2<kGroup, kThreads>(
+              make_float2(sg2.x + sg2.y, sgr2.x + sgr2.y), red, parity);
+        }
+      }
       const float mean1 = rq.x * inv_n;
       const float mean = mean0 + mean1;
       const float var = fmaxf(fmaf(-mean1, mean1, rq.y * inv_n), 0.0f);
@@ -385,26 +466,8 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
       } else {
         // x_hat = (x - mean) * inv_std; g = dy * gamma
         // dx = inv_std * (g - mean(g) - x_hat * mean(g * x_hat))
-        float2 sg2 = make_float2(0.0f, 0.0f), sgx2 = make_float2(0.0f, 0.0f);
-#pragma unroll
-        for (int j = 0; j < kMaxPacks; ++j) {
-          const int p = t + j * kGroup;
-          if (live && Has(j)) {
-            float2 gm[kPairs], dv[kPairs];
-            LoadRowVector(gsm, p, gm);
-            WidenPack<kVec>(cd[j], dv);
-#pragma unroll
-            for (int q = 0; q < kPairs; ++q) {
-              xv[j][q] = Fma2(xv[j][q], inv2, shift2);  // x_hat from here on
-              const float2 g = Mul2(dv[q], gm[q]);
-              sg2 = Add2(sg2, g);
-              sgx2 = Fma2(g, xv[j][q], sgx2);
-            }
-          }
-        }
-        const float2 gs = GroupSum2<kGroup, kThreads>(
-            make_float2(sg2.x + sg2.y, sgx2.x + sgx2.y), red, parity);
-        const float mg = gs.x * inv_n, mgx = gs.y * inv_n;
+        const float mg = gs.x * inv_n;
+        const float mgx = fmaf(gs.y * inv_n, inv_std, -mean1 * inv_std * mg);
         const float2 nmg = Dup(-mg), nmgx = Dup(-mgx);
         P* op = reinterpret_cast<P*>(a.out) + row * packs;
 #pragma unroll
@@ -416,6 +479,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
             WidenPack<kVec>(cd[j], dv);
 #pragma unroll
             for (int q = 0; q < kPairs; ++q) {
+              xv[j][q] = Fma2(xv[j][q], inv2, shift2);  // x_hat from here on
               const float2 g = Mul2(dv[q], gm[q]);
               o2[q] = Mul2(inv2, Fma2(xv[j][q], nmgx, Add2(g, nmg)));
             }
