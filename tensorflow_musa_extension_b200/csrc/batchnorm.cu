@@ -75,16 +75,17 @@ inline int PlanTx(int64_t cv, int max_tx) {
   return tx > max_tx ? max_tx : tx;
 }
 
-// Channels-last plan.  `cv` = channel packs per row.
+// Channels-last plan.  `cv` = channel packs per row; `cap` = most row splits (0:
+// any number; statistics: what the workspace holds).
 // `resident`: CTAs of this kernel that fit on one SM; the grid is one full
 // wave of them (a second, partly filled wave would idle SMs at the end).
-inline Plan PlanLast(int64_t rows, int64_t channels, int64_t cv, int unroll,
-                     bool cap_by_workspace, int resident, int max_tx = kThreads) {
+inline Plan PlanLast(int64_t rows, int64_t cv, int unroll,
+                     int64_t cap, int resident, int max_tx = kThreads) {
   Plan p;
   p.tx = PlanTx(cv, max_tx);
   p.ty = kThreads / p.tx;
   p.gx = static_cast<int>(CeilDiv(cv, p.tx));
-  int per_sm = GetTuning(cap_by_workspace ? kTuneBnCtasPerSm : kTuneBnApplyCtasPerSm);
+  int per_sm = GetTuning(cap > 0 ? kTuneBnCtasPerSm : kTuneBnApplyCtasPerSm);
   if (per_sm < 1) per_sm = resident > 0 ? resident : 4;
   int64_t target = static_cast<int64_t>(SmCount()) * per_sm / p.gx;
   if (target < 1) target = 1;
@@ -92,10 +93,7 @@ inline Plan PlanLast(int64_t rows, int64_t channels, int64_t cv, int unroll,
   int64_t max_useful = CeilDiv(rows, static_cast<int64_t>(p.ty) * unroll);
   if (max_useful < 1) max_useful = 1;
   int64_t gy = target < max_useful ? target : max_useful;
-  if (cap_by_workspace) {
-    const int64_t cap = MaxSplits(rows, channels);
-    if (gy > cap) gy = cap;
-  }
+  if (cap > 0 && gy > cap) gy = cap;
   if (gy > 65535) gy = 65535;
   p.rows_per_cta = CeilDiv(rows, gy);
   // Keep CTA row ranges a multiple of ty so that lanes stay aligned.
@@ -290,6 +288,15 @@ struct FinalizeArgs {
   // reserve_space_4 / _5).  NULL: none.
   float* zero_scalar;
   float* zero_vec[2];
+  // Rows that are not whole packs (see WrapFactor): the statistics kernel saw
+  // 1 << wrap_log rows as one row, so a partial row holds that many per
+  // channel; the `tail` rows (from element tail_at on) that do not fill such a
+  // row are added here, from x_first (and tail_dy about tail_mean, gradient).
+  int wrap_log;
+  int tail;
+  int64_t tail_at;
+  const void* tail_dy;
+  const float* tail_mean;
 };
 
 __device__ __forceinline__ float LoadAsF32(const void* base, int dtype,
@@ -432,7 +439,8 @@ __global__ void __launch_bounds__(kThreads)
                       const float* __restrict__ mean,
                       float* __restrict__ partial, int64_t rows, int64_t cv,
                       int64_t channels, int64_t rows_per_cta, float keep_fraction,
-                      bool drop_rest, bool interleave, unsigned* epoch_bump, int fold) {
+                      bool drop_rest, bool interleave, unsigned* epoch_bump, int fold,
+                      unsigned wrap_channels) {
   constexpr int kVec = VecWidth<T>::value;
   using P = Pack<T, kVec>;
   GridDepWait();
@@ -481,9 +489,21 @@ __global__ void __launch_bounds__(kThreads)
   if (active) {
     // The shift is requested here and first used (a wait of one memory round
     // trip) after the prologue's copies are on their way.
+    // (wrap_channels: rows of several rows of the tensor, element i belongs to
+    // channel i % wrap_channels.)
     P first;
     float mean_c[kVec];
-    if constexpr (kMode == kFwd) {
+    if (wrap_channels != 0) {
+      const unsigned v = static_cast<unsigned>(col) * kVec;
+#pragma unroll
+      for (int e = 0; e < kVec; ++e) {
+        if constexpr (kMode == kFwd) {
+          first.v[e] = x[(v + e) % wrap_channels];
+        } else {
+          mean_c[e] = __ldg(mean + (v + e) % wrap_channels);
+        }
+      }
+    } else if constexpr (kMode == kFwd) {
       first = LoadKeep(reinterpret_cast<const P*>(x) + col);
     } else {
 #pragma unroll
@@ -974,7 +994,7 @@ __global__ void __launch_bounds__(8 * kLanes) BnFinalizeKernel(FinalizeArgs a) {
   // The threads that finish a channel (first 8 of the CTA) fetch the shift
   // now, so that its latency overlaps the partial-sum loads.
   float shift_k = 0.0f;
-  if (kOut != 2 && tid < 8 && c < a.channels) {
+  if (kOut != 2 && (tid < 8 || py < a.tail) && c < a.channels) {
     shift_k = LoadAsF32(a.x_first, a.x_dtype, c * a.shift_stride);
   }
   // In-kernel exchange: the epoch of this exchange, and the replicas an
@@ -994,13 +1014,19 @@ __global__ void __launch_bounds__(8 * kLanes) BnFinalizeKernel(FinalizeArgs a) {
     // trips otherwise.
     constexpr int kU = 8;
     int p = py;
+    // Entry p of this channel: partial row p >> wrap_log, p's low bits inside it.
+    const int wl = a.wrap_log;
+    const int64_t half = a.channels << wl;   // from a sum of S1 to its S2
+    const auto At = [&](int q) {
+      return ((static_cast<int64_t>(q >> wl) * 2 << wl) + (q & ((1 << wl) - 1))) * a.channels + c;
+    };
     for (; p + (kU - 1) * kLanes < a.splits; p += kU * kLanes) {
       float u1[kU], u2[kU];
 #pragma unroll
       for (int q = 0; q < kU; ++q) {
-        const int64_t row = static_cast<int64_t>(p + q * kLanes) * 2;
-        u1[q] = a.partial[(row + 0) * a.channels + c];
-        u2[q] = a.partial[(row + 1) * a.channels + c];
+        const int64_t at = At(p + q * kLanes);
+        u1[q] = a.partial[at];
+        u2[q] = a.partial[at + half];
       }
 #pragma unroll
       for (int q = 0; q < kU; ++q) {
@@ -1014,15 +1040,28 @@ __global__ void __launch_bounds__(8 * kLanes) BnFinalizeKernel(FinalizeArgs a) {
       v1[q] = 0.0f;
       v2[q] = 0.0f;
       if (p + q * kLanes < a.splits) {
-        const int64_t row = static_cast<int64_t>(p + q * kLanes) * 2;
-        v1[q] = a.partial[(row + 0) * a.channels + c];
-        v2[q] = a.partial[(row + 1) * a.channels + c];
+        const int64_t at = At(p + q * kLanes);
+        v1[q] = a.partial[at];
+        v2[q] = a.partial[at + half];
       }
     }
 #pragma unroll
     for (int q = 0; q < kU - 1; ++q) {
       t1 += static_cast<double>(v1[q]);
       t2 += static_cast<double>(v2[q]);
+    }
+    if (py < a.tail) {
+      const int64_t at = a.tail_at + py * a.channels + c;
+      const float xt = LoadAsF32(a.x_first, a.x_dtype, at);
+      if constexpr (kOut == kTailGrad) {
+        const double g = static_cast<double>(LoadAsF32(a.tail_dy, a.x_dtype, at));
+        t1 += g;
+        t2 += g * static_cast<double>(xt - a.tail_mean[c]);
+      } else {
+        const double d = static_cast<double>(xt - shift_k);
+        t1 += d;
+        t2 += d * d;
+      }
     }
   }
   // A warp holds 4 partial lanes x 8 channels: fold lanes 8 and 16 apart.
@@ -1224,13 +1263,13 @@ struct ApplyArgs {
 // CTAs per SM that the registers are held to: the fp32 gradient fits three
 // (80 registers), the 16-bit forms with their eight channels a thread two, the
 // element form the four that its launch assumes.
-template <typename T, int kVec, int kUnroll, int kMode>
+template <typename T, int kVec, int kUnroll, int kMode, bool kWrap>
 __global__ void __launch_bounds__(kThreads, kVec == 1 ? 4 : sizeof(T) == 4 && kUnroll == 4 ? 3 : 2)
     BnApplyLastKernel(const T* __restrict__ x, const T* __restrict__ dy,
                       T* __restrict__ out, ApplyArgs a, int64_t rows,
                       int64_t cv, int64_t channels, int64_t rows_per_cta,
                       bool reverse, bool last_use, bool early_loads, bool early_inputs,
-                      bool interleave) {
+                      bool interleave, unsigned wrap_channels, int64_t tail_elems) {
   using P = Pack<T, kVec>;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int TX = blockDim.x, TY = blockDim.y;
@@ -1327,6 +1366,13 @@ __global__ void __launch_bounds__(kThreads, kVec == 1 ? 4 : sizeof(T) == 4 && kU
   const bool fold = a.fold_rows != nullptr;
   const bool own_stats = kMode == kFwd && (fold || a.stat_sums != nullptr);
   float scale_c = 0.0f, offset_c = 0.0f, mean_c = 0.0f, var_c = 0.0f, shift_c = 0.0f;
+  // The channel behind column v, and how many there are (kWrap: a row here is
+  // several rows of the tensor; a template parameter, because the same code
+  // behind a run-time test took the whole-pack forward from 33 to 59 us).
+  const int64_t real = kWrap ? static_cast<int64_t>(wrap_channels) : channels;
+  const auto ChannelOf = [&](int64_t v) {
+    return kWrap ? static_cast<int64_t>(static_cast<unsigned>(v) % wrap_channels) : v;
+  };
   auto load_inputs = [&](int64_t c) {
     scale_c = a.scale[c];
     if constexpr (kMode == kFwd) {
@@ -1338,7 +1384,7 @@ __global__ void __launch_bounds__(kThreads, kVec == 1 ? 4 : sizeof(T) == 4 && kU
       var_c = a.variance[c];
     }
   };
-  if (early_inputs && tid < seg) load_inputs(c0 + tid);
+  if (early_inputs && tid < seg) load_inputs(ChannelOf(c0 + tid));
   GridDepWait();
   GridDepLaunch();
   // Second level of the reduction when no finalize kernel ran (fold_rows):
@@ -1381,9 +1427,9 @@ __global__ void __launch_bounds__(kThreads, kVec == 1 ? 4 : sizeof(T) == 4 && kU
   // folded to two (forward) or three (gradient) coefficients and one or two
   // FMAs per element; fp32 keeps the centred form (x - mean) to the end.
   constexpr bool kFold = sizeof(T) == 2;
-  const bool writer = blockIdx.y == 0;
   for (int ch = tid; ch < seg; ch += kThreads) {
-    const int64_t c = c0 + ch;
+    const int64_t c = ChannelOf(c0 + ch);
+    const bool writer = blockIdx.y == 0 && c0 + ch < real;
     if (!early_inputs || ch != tid) load_inputs(c);
     if constexpr (kMode == kFwd) {
       if (own_stats) {
@@ -1395,10 +1441,10 @@ __global__ void __launch_bounds__(kThreads, kVec == 1 ? 4 : sizeof(T) == 4 && kU
           v = s_tot[1][ch] * a.stat_out.inv_count - md * md;
         } else if (a.stat_moments) {
           m = static_cast<double>(a.stat_sums[c]);
-          v = static_cast<double>(a.stat_sums[channels + c]) * a.stat_out.inv_count;
+          v = static_cast<double>(a.stat_sums[real + c]) * a.stat_out.inv_count;
         } else {
           m = static_cast<double>(a.stat_sums[c]) * a.stat_out.inv_count;
-          v = static_cast<double>(a.stat_sums[channels + c]) * a.stat_out.inv_count - m * m;
+          v = static_cast<double>(a.stat_sums[real + c]) * a.stat_out.inv_count - m * m;
         }
         if (v < 0.0) v = 0.0;
         mean_c = static_cast<float>(m);
@@ -1421,7 +1467,7 @@ __global__ void __launch_bounds__(kThreads, kVec == 1 ? 4 : sizeof(T) == 4 && kU
         t2 = static_cast<float>(s_tot[1][ch]);
       } else if (given_sums) {
         t1 = a.sums[c];
-        t2 = a.sums[channels + c];
+        t2 = a.sums[real + c];
       }
       const bool use = fold ? a.fold_use : given_sums;
       cb1 = use ? t1 * a.inv_count : 0.0f;
@@ -1450,6 +1496,27 @@ __global__ void __launch_bounds__(kThreads, kVec == 1 ? 4 : sizeof(T) == 4 && kU
     if constexpr (!kFold) apply_smem[3 * nch + ch] = mean_c;
   }
   __syncthreads();
+  const auto WriteTail = [&] {
+    for (int ch = tid; ch < seg && c0 + ch < tail_elems; ch += kThreads) {
+      const int64_t at = rows * channels + c0 + ch;
+      const float A = apply_smem[ch], B = apply_smem[nch + ch];
+      const float xv = ToF32(x[at]);
+      float r;
+      if constexpr (kMode == kFwd) {
+        r = fmaf(kFold ? xv : xv - apply_smem[3 * nch + ch], A, B);
+      } else {
+        const float g = ToF32(dy[at]), C = apply_smem[2 * nch + ch];
+        r = kFold ? fmaf(g, A, fmaf(xv, B, C))
+                  : A * fmaf(-(xv - apply_smem[3 * nch + ch]), C, g - B);
+      }
+      out[at] = FromF32<T>(r);
+    }
+  };
+  // kWrap: the rows that do not fill a row of this launch, element by element
+  // (before the return of threads beyond the last column would lose some).
+  if constexpr (kWrap) {
+    if (blockIdx.y == gridDim.y - 1) WriteTail();
+  }
   if (!active) return;
   float ca[kVec], cb[kVec], cc[kVec], mean[kVec];
 #pragma unroll
@@ -2257,6 +2324,33 @@ struct Geom {
   int64_t rows() const { return outer * inner; }  // values per channel
 };
 
+// Channels-last rows that are not whole packs (odd channel counts): `factor`
+// neighbouring rows - kVec, or less where the channel count shares a power of
+// two with it - are whole packs together, so the vector kernels run over
+// rows / factor rows of factor * channels columns, column v belonging to
+// channel v % channels.  1: not possible (unaligned, too few rows for one such
+// row, or a workspace that cannot hold a partial row of them).
+// Single elements moved 2 or 4 bytes per access; forward, gradient, inference in
+// us before and after: bf16 [200704,255] 126, 193, 78 -> 58, 89, 44; bf16
+// [20000,100] 16.6, 18.6, 8.4 -> 10.9, 12.1, 4.0; fp32 [60000,1001] 225, 270, 153
+// -> 124, 194, 77 (bf16 [200704,256], whole packs: 47, 77, 33).
+template <typename T>
+inline int WrapFactor(const Geom& g, bool aligned) {
+  constexpr int kVec = VecWidth<T>::value;
+  if (!aligned || g.inner != 1 || g.channels % kVec == 0) return 1;
+  int factor = 2;
+  while (factor * g.channels % kVec != 0) factor *= 2;
+  if (g.outer < factor || MaxSplits(g.outer, g.channels) < factor) return 1;
+  if (g.channels > (1 << 27)) return 1;   // columns are counted in 32 bits
+  return factor;
+}
+
+inline int Log2(int v) {
+  int l = 0;
+  while ((1 << l) < v) ++l;
+  return l;
+}
+
 inline int CheckGeom(const Geom& g) {
   if (g.outer < 0 || g.channels < 0 || g.inner < 0) return MUSA_KERNELS_EINVAL;
   return MUSA_KERNELS_OK;
@@ -2284,8 +2378,8 @@ inline int DecodeError(int rc) { return rc <= -1000 ? -rc - 1000 : rc; }
 // written, or a negative error.
 template <typename T, int kMode, int kStagesT>
 int LaunchStatsPipe(const T* x, const T* dy, const float* mean, float* workspace,
-                    const Geom& g, int64_t cv, unsigned* epoch_bump, cudaStream_t stream,
-                    int* fold_io = nullptr) {
+                    const Geom& g, int64_t cv, int64_t max_splits, int64_t wrap_channels,
+                    unsigned* epoch_bump, cudaStream_t stream, int* fold_io = nullptr) {
   using Cfg = StatsPipe<kMode, kStagesT>;
   auto kernel = BnStatsPipeKernel<T, kMode, kStagesT>;
   static std::atomic<int> resident_by_device[kMaxDevices];
@@ -2310,7 +2404,7 @@ int LaunchStatsPipe(const T* x, const T* dy, const float* mean, float* workspace
   // layers.
   int max_tx = GetTuning(kTuneBnStatsMaxTx);
   if (max_tx <= 0) max_tx = kThreads;
-  const Plan p = PlanLast(g.outer, g.channels, cv, Cfg::kU, true, resident, max_tx);
+  const Plan p = PlanLast(g.outer, cv, Cfg::kU, max_splits, resident, max_tx);
   // What the element-wise pass that follows can find in L2: the budget over
   // the bytes this pass reads (all streams), as the fraction of every
   // thread's rows that is read with the evict-last priority.
@@ -2360,7 +2454,8 @@ int LaunchStatsPipe(const T* x, const T* dy, const float* mean, float* workspace
       GetTuning(kTuneBnPdl) != 0, fold, kernel, dim3(p.gx, gy), dim3(p.tx, p.ty),
       Cfg::kSmemBytes, stream, x, dy, mean, workspace, g.outer, cv, g.channels,
       rows_per_cta, keep_fraction, GetTuning(kTuneBnStatsDropRest) != 0,
-      GetTuning(kTuneBnInterleave) != 0, epoch_bump, fold);
+      GetTuning(kTuneBnInterleave) != 0, epoch_bump, fold,
+      static_cast<unsigned>(wrap_channels));
   if (err != cudaSuccess) {
     cudaGetLastError();
     return EncodeCuda(err);
@@ -2450,20 +2545,27 @@ int LaunchStats(const T* x, const T* dy, const float* mean, float* partial,
   const bool keep = GetTuning(kTuneBnStatsKeep) != 0;
   const bool aligned = Aligned16(x) && (kMode == kFwd || Aligned16(dy));
   if (g.inner == 1) {
+    const int wrap = WrapFactor<T>(g, aligned);
+    const int stages = GetTuning(kTuneBnStatsPipe);
+    const int64_t cap = MaxSplits(g.outer, g.channels);
+    if (wrap > 1 && stages != 0) {
+      const Geom rows{g.outer / wrap, g.channels * wrap, 1};
+      return LaunchStatsPipe<T, kMode, 4>(x, dy, mean, partial, rows, rows.channels / kVec,
+                                          cap / wrap, g.channels, epoch_bump, stream);
+    }
     if (g.channels % kVec == 0 && aligned) {
       const int64_t cv = g.channels / kVec;
-      const int stages = GetTuning(kTuneBnStatsPipe);
       if (stages == 3) {
         *fold_pipe = fold_wanted;
-        return LaunchStatsPipe<T, kMode, 3>(x, dy, mean, partial, g, cv, epoch_bump, stream,
-                                            fold_pipe);
+        return LaunchStatsPipe<T, kMode, 3>(x, dy, mean, partial, g, cv, cap, 0, epoch_bump,
+                                            stream, fold_pipe);
       }
       if (stages != 0) {
         *fold_pipe = fold_wanted;
-        return LaunchStatsPipe<T, kMode, 4>(x, dy, mean, partial, g, cv, epoch_bump, stream,
-                                            fold_pipe);
+        return LaunchStatsPipe<T, kMode, 4>(x, dy, mean, partial, g, cv, cap, 0, epoch_bump,
+                                            stream, fold_pipe);
       }
-      const Plan p = PlanLast(g.outer, g.channels, cv, kUnroll, true, 3);
+      const Plan p = PlanLast(g.outer, cv, kUnroll, cap, 3);
       BnStatsLastKernel<T, kVec, kUnroll, kMode>
           <<<dim3(p.gx, p.gy), dim3(p.tx, p.ty), 0, stream>>>(
               x, dy, mean, partial, g.outer, cv, g.channels, p.rows_per_cta,
@@ -2471,7 +2573,7 @@ int LaunchStats(const T* x, const T* dy, const float* mean, float* partial,
       CountKernelLaunch();
       return p.gy;
     }
-    const Plan p = PlanLast(g.outer, g.channels, g.channels, kUnroll, true, 4);
+    const Plan p = PlanLast(g.outer, g.channels, kUnroll, cap, 4);
     BnStatsLastKernel<T, 1, kUnroll, kMode>
         <<<dim3(p.gx, p.gy), dim3(p.tx, p.ty), 0, stream>>>(
             x, dy, mean, partial, g.outer, g.channels, g.channels,
@@ -2519,6 +2621,23 @@ int LaunchStats(const T* x, const T* dy, const float* mean, float* partial,
   return static_cast<int>(pp.gy);
 }
 
+// What the finalize kernel has to know about the statistics launch before it:
+// `splits` partial rows of x (and dy, about `mean`).
+template <typename T>
+void SetPartials(FinalizeArgs* f, int splits, const Geom& g, const T* x, const T* dy,
+                 const float* mean) {
+  const bool aligned = Aligned16(x) && Aligned16(dy);   // (dy NULL: forward)
+  const int wrap = GetTuning(kTuneBnStatsPipe) != 0 ? WrapFactor<T>(g, aligned) : 1;
+  f->splits = splits * wrap;
+  f->wrap_log = Log2(wrap);
+  f->tail = static_cast<int>(g.outer % wrap);
+  f->tail_at = (g.outer - f->tail) * g.channels;
+  f->x_first = x;
+  f->x_dtype = DtypeCode<T>::value;
+  f->tail_dy = dy;
+  f->tail_mean = mean;
+}
+
 template <int kLanes>
 void LaunchFinalizeAs(int kind, const FinalizeArgs& a, cudaStream_t stream) {
   const int grid = static_cast<int>(CeilDiv(a.channels, 8));
@@ -2556,7 +2675,7 @@ int RunStats(const T* x, const T* dy, const float* mean, float* workspace,
   f.partial = workspace;
   const int splits = LaunchStats<T, kMode>(x, dy, mean, workspace, g, f.xchg_epoch, stream);
   if (splits < 0) return DecodeError(splits);
-  f.splits = splits;
+  SetPartials<T>(&f, splits, g, x, dy, mean);
   LaunchFinalize(kind, f, stream);
   return MUSA_KERNELS_OK;
 }
@@ -2582,11 +2701,12 @@ inline int64_t ApplyFoldBytes(int64_t cv, int fold_n) {
   return static_cast<int64_t>(fold_n) * 2 * tx * kVec * static_cast<int64_t>(sizeof(float));
 }
 
-template <typename T, int kVec, int kU, int kMode>
+template <typename T, int kVec, int kU, int kMode, bool kWrap>
 void LaunchApplyLast(const T* x, const T* dy, T* out, const ApplyArgs& a, const Geom& g,
                      int64_t cv, bool reverse, bool last_use, bool early_loads,
-                     bool early_inputs, cudaStream_t stream) {
-  auto kernel = BnApplyLastKernel<T, kVec, kU, kMode>;
+                     bool early_inputs, int64_t wrap_channels, int64_t tail_elems,
+                     cudaStream_t stream) {
+  auto kernel = BnApplyLastKernel<T, kVec, kU, kMode, kWrap>;
   static std::atomic<int> resident_by_device[kMaxDevices];
   int resident = PerDevice(resident_by_device, [&] {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2609,10 +2729,11 @@ void LaunchApplyLast(const T* x, const T* dy, T* out, const ApplyArgs& a, const 
     const int by_smem = static_cast<int>(233472 / (smem + 4096 + 1024));
     if (by_smem < resident) resident = by_smem > 0 ? by_smem : 1;
   }
-  const Plan p = PlanLast(g.outer, g.channels, cv, kU, false, resident, ApplyMaxTx());
+  const Plan p = PlanLast(g.outer, cv, kU, 0, resident, ApplyMaxTx());
   LaunchChained(GetTuning(kTuneBnPdl) != 0, kernel, dim3(p.gx, p.gy), dim3(p.tx, p.ty), smem,
                 stream, x, dy, out, a, g.outer, cv, g.channels, p.rows_per_cta, reverse,
-                last_use, early_loads, early_inputs, GetTuning(kTuneBnInterleave) != 0);
+                last_use, early_loads, early_inputs, GetTuning(kTuneBnInterleave) != 0,
+                static_cast<unsigned>(wrap_channels), tail_elems);
 }
 
 // How much the element-wise kernel may read before its wait for the kernel it
@@ -2641,28 +2762,31 @@ void LaunchApply(const T* x, const T* dy, T* out, const ApplyArgs& a,
   const bool aligned =
       Aligned16(x) && Aligned16(out) && (kMode == kFwd || Aligned16(dy));
   if (g.inner == 1) {
-    if (g.channels % kVec == 0 && aligned) {
-      const int64_t cv = g.channels / kVec;
-      // The forward pass has one input stream: twice the rows in flight.
+    const int wrap = WrapFactor<T>(g, aligned);
+    if (wrap > 1 || (g.channels % kVec == 0 && aligned)) {
+      const Geom rows{g.outer / wrap, g.channels * wrap, 1};
+      const int64_t cv = rows.channels / kVec;
+      const int64_t wrap_channels = wrap > 1 ? g.channels : 0;
+      const int64_t tail = (g.outer % wrap) * g.channels;
+      // The forward pass has one input stream: twice the rows in flight (whole
+      // packs; the wrapped form then runs at 127 registers and half the rate).
       const bool deep = kMode == kFwd && GetTuning(kTuneBnApplyDeep) != 0;
       const bool tuned_early = GetTuning(kTuneBnApplyEarlyLoads) != 0;
       const bool early = early_reads >= kReadRowsEarly && tuned_early;
       const bool inputs = early_reads == kReadInputsEarly && tuned_early;
-      if (deep) {
-        constexpr int kDeep = kMode == kFwd ? 8 : kUnroll;
-        LaunchApplyLast<T, kVec, kDeep, kMode>(x, dy, out, a, g, cv, reverse, last_use, early,
-                                               inputs, stream);
-      } else {
-        LaunchApplyLast<T, kVec, kUnroll, kMode>(x, dy, out, a, g, cv, reverse, last_use, early,
-                                                 inputs, stream);
-      }
+      constexpr int kDeep = kMode == kFwd ? 8 : kUnroll;
+      const auto launch = wrap > 1 ? LaunchApplyLast<T, kVec, kUnroll, kMode, true>
+                          : deep   ? LaunchApplyLast<T, kVec, kDeep, kMode, false>
+                                   : LaunchApplyLast<T, kVec, kUnroll, kMode, false>;
+      launch(x, dy, out, a, rows, cv, reverse, last_use, early, inputs, wrap_channels, tail,
+             stream);
     } else {
       const Plan p =
-          PlanLast(g.outer, g.channels, g.channels, kUnroll, false, 4);
-      BnApplyLastKernel<T, 1, kUnroll, kMode>
+          PlanLast(g.outer, g.channels, kUnroll, 0, 4);
+      BnApplyLastKernel<T, 1, kUnroll, kMode, false>
           <<<dim3(p.gx, p.gy), dim3(p.tx, p.ty), ApplyCoefBytes(p.tx), stream>>>(
               x, dy, out, a, g.outer, g.channels, g.channels, p.rows_per_cta,
-              reverse, false, false, false, false);
+              reverse, false, false, false, false, 0, 0);
       CountKernelLaunch();
     }
     return;
@@ -2939,7 +3063,7 @@ int FwdTrain(const void* x, const float* scale, const float* offset,
     a.fold_n = splits;
     a.stat_out = f;
   } else {
-    f.splits = splits;
+    SetPartials<T>(&f, splits, g, xt, nullptr, nullptr);
     LaunchFinalize(kTailFwdStats, f, stream);
   }
   LaunchApply<T, kFwd>(xt, nullptr, static_cast<T*>(y), a, g, stream, kReadInputsEarly);
@@ -3034,7 +3158,7 @@ int Grad(const void* dy, const void* x, const float* scale, const float* mean,
     a.doffset = doffset;
     a.stat_out = f;
   } else {
-    f.splits = splits;
+    SetPartials<T>(&f, splits, g, xt, dyt, mean);
     LaunchFinalize(kTailGrad, f, stream);
   }
   LaunchApply<T, kGrad>(xt, dyt, static_cast<T*>(dx), a, g, stream, kReadInputsEarly);

@@ -716,3 +716,66 @@ def test_one_kernel_form(kernel_lib, dtype, cluster, shape, layout):
         a, b = to_numpy(a).astype(np.float64), to_numpy(b).astype(np.float64)
         assert np.all(np.abs(a - b) <= 1e-5 * np.abs(b) + 1e-5 * max(_rms(b), 1e-12))
     check_grad(frozen, tuple(to_numpy(t) for t in chain[2][:3]), dtype, dx_scale=terms)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("rows,c", [(8, 1), (9, 37), (15, 3), (4099, 100), (7001, 6), (2051, 1001),
+                                    (300, 4099), (70001, 5), (9, 70001)])
+def test_rows_that_are_not_whole_packs(kernel_lib, dtype, rows, c):
+    """Odd channel counts: several rows together are whole packs and take the
+    vector kernels, the rows left over are added by the finalize kernel and
+    written element by element.  Against the oracle, and against the element
+    kernels (the same values off a 16-byte boundary): training forward with
+    running statistics, inference, both gradients, the raw sums of the
+    cross-replica form."""
+    x, s, o, dy = bn_inputs(17 + c, (rows, c), dtype, 1.0, 3.0)
+    gen = np.random.default_rng(c)
+    rm = gen.standard_normal(c).astype(np.float32)
+    rv = (gen.random(c) + 0.5).astype(np.float32)
+    want = np_ref.fused_batch_norm(x, s, o, rm, rv, epsilon=EPS, exponential_avg_factor=0.25)
+    wg = np_ref.fused_batch_norm_grad(dy, x, s, want[3], want[4], EPS)
+    terms = _rms(dy) * float(np.max(s / np.sqrt(want[4] + EPS)))
+    ts, to_, tm, tv = to_torch(s), to_torch(o), to_torch(rm), to_torch(rv)
+    st = torch.cuda.current_stream().cuda_stream
+
+    def run(tx, tdy):
+        fwd = raw_ops.FusedBatchNormV3(tx, ts, to_, tm, tv, epsilon=EPS,
+                                       exponential_avg_factor=0.25)
+        infer = raw_ops.FusedBatchNormV3(tx, ts, to_, tm, tv, epsilon=EPS, is_training=False)
+        args = (tdy, tx, ts, fwd.reserve_space_1, fwd.reserve_space_2, None, EPS)
+        grad = raw_ops.FusedBatchNormGradV3(*args)
+        frozen = raw_ops.FusedBatchNormGradV3(*args, is_training=False)
+        sums = torch.empty(2 * c, device="cuda")
+        ws = torch.empty(max(kernel_lib.BnWorkspaceBytes(rows, c, 1), 16), dtype=torch.uint8,
+                         device="cuda")
+        assert kernel_lib.LaunchBnGradStatsSums(
+            raw_ops._DT_CODE[tx.dtype], tdy.data_ptr(), tx.data_ptr(),
+            fwd.reserve_space_1.data_ptr(), sums.data_ptr(), rows, c, 1, ws.data_ptr(),
+            ws.numel(), st) == 0
+        torch.cuda.synchronize()
+        return fwd, infer, grad, frozen, (sums,)
+
+    def unaligned(a):
+        t = to_torch(a)
+        return torch.cat((t.new_zeros(1), t.reshape(-1)))[1:].view(t.shape)
+
+    old = kernel_lib.MusaKernelsSetTuning(2, -1)   # the chain, whatever the size
+    try:
+        got = run(to_torch(x), to_torch(dy))
+        again = run(to_torch(x), to_torch(dy))
+        base = run(unaligned(x), unaligned(dy))
+    finally:
+        kernel_lib.MusaKernelsSetTuning(2, old)
+    check_forward(got[0], want, dtype)
+    check_grad(got[2], wg, dtype, dx_scale=terms)
+    for out, same in zip(got, again):
+        for a, b in zip(out, same):
+            assert torch.equal(a, b)
+    for i, (out, ref) in enumerate(zip(got, base)):
+        for k, (a, b) in enumerate(zip(out, ref)):
+            a, b = to_numpy(a).astype(np.float64), to_numpy(b).astype(np.float64)
+            # Element-wise results: one rounding of T on statistics that agree
+            # to 1e-5; the others are fp32 sums in another order.
+            rt = _rt(dtype) if k == 0 and i < 4 else 1e-5
+            floor = max(_rms(b), terms if i in (2, 3) and k == 0 else 1e-12)
+            assert np.all(np.abs(a - b) <= rt * np.abs(b) + rt * floor), (i, k)
