@@ -164,6 +164,13 @@ __device__ __forceinline__ void AsyncCopy16(void* smem_dst, const void* gmem_src
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(gmem_src)
                : "memory");
 }
+// The first `bytes` (1 .. 16) of a pack; the rest of the slot is zero-filled.
+__device__ __forceinline__ void AsyncCopyPart(void* smem_dst, const void* gmem_src, int bytes) {
+  const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem_src),
+               "r"(bytes)
+               : "memory");
+}
 __device__ __forceinline__ void AsyncCommit() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
@@ -234,12 +241,30 @@ constexpr int RowMinCtas(int group, int op, int max_packs, int elem_bytes) {
 // round as the second sum over x: two dependent rounds a row instead of three
 // (bf16 [16384,1024] 24.8 -> 22.4 us, [65536,1024] 77.4 -> 68.2, [32768,2048]
 // 88.1 -> 80.8, [8192,8192] 99.0 -> 90.1) - except where the four partial sums
-// spill (256-thread groups of three 16-bit packs: rows of 5120 102 -> 111 us).
+// spill (256-thread groups of three 16-bit packs that the row does not fill: rows
+// of 5120 102 -> 111 us; rows of 6144, which fill them, 91.7 -> 85.5).
 __host__ __device__ constexpr bool RowMergesSums(int group, int max_packs, int elem_bytes) {
   return !(group == 256 && max_packs == 3 && elem_bytes == 2);
 }
 
-template <typename T, int kGroup, int kMaxPacks, int kOp, bool kFull>
+// How the rows lie against the 128-bit packs.
+//   kRowsPacked  whole packs (row_size a multiple of the pack width)
+//   kRowsFull    the same, and they fill the layout: no per-pack checks
+//   kRowsShifted any row_size: a row starts `shift` elements into a pack.  Its
+//                first and last pack may hold elements of the neighbouring rows,
+//                which are read as zeros and not written.  A thread's rows are a
+//                multiple of the pack width apart (the launch sees to it), so
+//                its shift, and with it the columns it meets, never changes.
+enum RowLayout { kRowsPacked = 0, kRowsFull = 1, kRowsShifted = 2 };
+
+// The fp32 copies of gamma / beta for shifted rows: column c at c + kVec, spread
+// by one word in 32 (neighbouring lanes read words a pack apart), zeros around.
+__host__ __device__ constexpr int ShiftedWord(int i) { return i + (i >> 5); }
+__host__ __device__ constexpr int ShiftedWords(int row_size, int vec) {
+  return ShiftedWord(row_size + 2 * vec) + 1;
+}
+
+template <typename T, int kGroup, int kMaxPacks, int kOp, int kLayout>
 __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
                                   RowMinCtas(kGroup, kOp, kMaxPacks, sizeof(T)))
     RowNormKernel(RowArgs a) {
@@ -260,14 +285,52 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
   // in quads (see Quad below).
   extern __shared__ uint4 ring[];
   float* gsm = reinterpret_cast<float*>(ring + kStages * kInputs * kMaxPacks * kThreads);
-  float* bsm = gsm + a.row_size;
+  constexpr bool kFull = kLayout == kRowsFull;
+  constexpr bool kShifted = kLayout == kRowsShifted;
+  float* bsm = gsm + (kShifted ? ShiftedWords(a.row_size, kVec) : a.row_size);
   // LayerNorm gradient, after the last row: one slab [2][kVec / 4][packs][4]
   // of column sums per row lane, laid over the ring.
   float* slab = reinterpret_cast<float*>(ring);
 
   const int t = threadIdx.x % kGroup;
   const int lane_row = threadIdx.x / kGroup;
-  const int packs = a.row_size / kVec;
+  // Shifted rows: elements of the first pack that belong to the row before
+  // (the same for all rows of this thread), and the packs that hold the row.
+  int shift = 0;
+  if constexpr (kShifted) {
+    const int64_t row0 = static_cast<int64_t>(blockIdx.x) * kRows + lane_row;
+    shift = static_cast<int>((row0 % kVec) * (a.row_size % kVec) % kVec);
+  }
+  const int packs = kShifted ? (a.row_size + shift + kVec - 1) / kVec : a.row_size / kVec;
+  // First pack of a row in units of packs from the tensor's start.
+  const auto RowPack = [&](int64_t row) {
+    return kShifted ? (row * a.row_size - shift) / kVec : row * packs;
+  };
+  // Pack p holds elements of other rows too; element e of it belongs to the row.
+  const auto Edge = [&](int p) { return kShifted && (p == 0 || p == packs - 1); };
+  const auto Inside = [&](int p, int e) {
+    return static_cast<unsigned>(p * kVec + e - shift) < static_cast<unsigned>(a.row_size);
+  };
+  const auto Mask = [&](int p, float2 (&v)[kPairs]) {
+    if (Edge(p)) {
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        if (!Inside(p, 2 * q)) v[q].x = 0.0f;
+        if (!Inside(p, 2 * q + 1)) v[q].y = 0.0f;
+      }
+    }
+  };
+  const auto StorePack = [&](P* base, int p, const P& v) {
+    if (Edge(p)) {
+      T* at = reinterpret_cast<T*>(base + p);
+#pragma unroll
+      for (int e = 0; e < kVec; ++e) {
+        if (Inside(p, e)) at[e] = v.v[e];
+      }
+    } else {
+      StoreStream(base + p, v);
+    }
+  };
   const float inv_n = 1.0f / static_cast<float>(a.row_size);
   float* my_slab = slab + static_cast<size_t>(lane_row) * 2 * a.row_size;
   uint4* const mine = ring + threadIdx.x;
@@ -280,6 +343,15 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
     return *reinterpret_cast<const float4*>(base + (h * packs + p) * 4);
   };
   const auto LoadRowVector = [&](const float* base, int p, float2 (&out)[kPairs]) {
+    if constexpr (kShifted) {
+      const int first = (p + 1) * kVec - shift;
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        out[q] = make_float2(base[ShiftedWord(first + 2 * q)],
+                             base[ShiftedWord(first + 2 * q + 1)]);
+      }
+      return;
+    }
 #pragma unroll
     for (int h = 0; h < kQuads; ++h) {
       const float4 v = Quad(base, h, p);
@@ -310,15 +382,22 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
   auto request = [&](int64_t rb, int stage) {
     const int64_t row = rb * kRows + lane_row;
     if (rb < n_blocks && row < a.rows) {
-      const P* xp = reinterpret_cast<const P*>(a.x) + row * packs;
-      const P* dp = reinterpret_cast<const P*>(a.dy) + row * packs;
+      const P* xp = reinterpret_cast<const P*>(a.x) + RowPack(row);
+      const P* dp = reinterpret_cast<const P*>(a.dy) + RowPack(row);
 #pragma unroll
       for (int j = 0; j < kMaxPacks; ++j) {
         const int p = t + j * kGroup;
         if (Has(j)) {
-          AsyncCopy16(mine + ((stage * kInputs + 0) * kMaxPacks + j) * kThreads, xp + p);
-          if constexpr (kGrad) {
-            AsyncCopy16(mine + ((stage * kInputs + 1) * kMaxPacks + j) * kThreads, dp + p);
+          uint4* const to_x = mine + ((stage * kInputs + 0) * kMaxPacks + j) * kThreads;
+          uint4* const to_d = mine + ((stage * kInputs + 1) * kMaxPacks + j) * kThreads;
+          if (kShifted && p == packs - 1 && row == a.rows - 1) {
+            // The tensor's last pack: no byte beyond its end is read.
+            const int bytes = (a.row_size + shift - p * kVec) * static_cast<int>(sizeof(T));
+            AsyncCopyPart(to_x, xp + p, bytes);
+            if constexpr (kGrad) AsyncCopyPart(to_d, dp + p, bytes);
+          } else {
+            AsyncCopy16(to_x, xp + p);
+            if constexpr (kGrad) AsyncCopy16(to_d, dp + p);
           }
         }
       }
@@ -331,11 +410,22 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
   }
   // gamma / beta while the first rows are on their way (filled before them they
   // put a memory round trip in front of every launch).
-  for (int c = threadIdx.x; c < a.row_size; c += kThreads) {
-    const int e = c % kVec;
-    const int at = ((e / 4) * packs + c / kVec) * 4 + (e & 3);
-    gsm[at] = ToF32(static_cast<const T*>(a.gamma)[c]);
-    if constexpr (kOp == kOpLnFwd) bsm[at] = ToF32(static_cast<const T*>(a.beta)[c]);
+  if constexpr (kShifted) {
+    for (int i = threadIdx.x; i < a.row_size + 2 * kVec; i += kThreads) {
+      const int c = i - kVec;
+      const bool in = c >= 0 && c < a.row_size;
+      gsm[ShiftedWord(i)] = in ? ToF32(static_cast<const T*>(a.gamma)[c]) : 0.0f;
+      if constexpr (kOp == kOpLnFwd) {
+        bsm[ShiftedWord(i)] = in ? ToF32(static_cast<const T*>(a.beta)[c]) : 0.0f;
+      }
+    }
+  } else {
+    for (int c = threadIdx.x; c < a.row_size; c += kThreads) {
+      const int e = c % kVec;
+      const int at = ((e / 4) * packs + c / kVec) * 4 + (e & 3);
+      gsm[at] = ToF32(static_cast<const T*>(a.gamma)[c]);
+      if constexpr (kOp == kOpLnFwd) bsm[at] = ToF32(static_cast<const T*>(a.beta)[c]);
+    }
   }
   __syncthreads();
 
@@ -369,6 +459,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
     for (int j = 0; j < kMaxPacks; ++j) {
       if (live && Has(j)) {
         WidenPack<kVec>(cx[j], xv[j]);
+        Mask(t + j * kGroup, xv[j]);
       } else {
 #pragma unroll
         for (int q = 0; q < kPairs; ++q) xv[j][q] = make_float2(0.0f, 0.0f);
@@ -397,6 +488,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
         float2 gm[kPairs], dv[kPairs];
         LoadRowVector(gsm, t + j * kGroup, gm);
         WidenPack<kVec>(cd[j], dv);
+        Mask(t + j * kGroup, dv);
 #pragma unroll
         for (int q = 0; q < kPairs; ++q) {
           const float2 g = Mul2(dv[q], gm[q]);
@@ -404,13 +496,16 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
           sgr2 = Fma2(g, xv[j][q], sgr2);
         }
       };
-      constexpr bool kMerged = kOp == kOpLnGrad && RowMergesSums(kGroup, kMaxPacks, sizeof(T));
+      constexpr bool kMerged =
+          kOp == kOpLnGrad && (kFull || RowMergesSums(kGroup, kMaxPacks, sizeof(T)));
 #pragma unroll
       for (int j = 0; j < kMaxPacks; ++j) {
         if (live && Has(j)) {
 #pragma unroll
+          for (int q = 0; q < kPairs; ++q) xv[j][q] = Add2(xv[j][q], nmean0);
+          Mask(t + j * kGroup, xv[j]);
+#pragma unroll
           for (int q = 0; q < kPairs; ++q) {
-            xv[j][q] = Add2(xv[j][q], nmean0);
             r2 = Add2(r2, xv[j][q]);
             q2 = Fma2(xv[j][q], xv[j][q], q2);
           }
@@ -446,7 +541,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
           if (a.mean_out != nullptr) a.mean_out[row] = mean;
           if (a.inv_std_out != nullptr) a.inv_std_out[row] = inv_std;
         }
-        P* yp = reinterpret_cast<P*>(a.out) + row * packs;
+        P* yp = reinterpret_cast<P*>(a.out) + RowPack(row);
 #pragma unroll
         for (int j = 0; j < kMaxPacks; ++j) {
           const int p = t + j * kGroup;
@@ -460,7 +555,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
             }
             P o;
             NarrowPack<kVec>(o2, o);
-            StoreStream(yp + p, o);
+            StorePack(yp, p, o);
           }
         }
       } else {
@@ -469,7 +564,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
         const float mg = gs.x * inv_n;
         const float mgx = fmaf(gs.y * inv_n, inv_std, -mean1 * inv_std * mg);
         const float2 nmg = Dup(-mg), nmgx = Dup(-mgx);
-        P* op = reinterpret_cast<P*>(a.out) + row * packs;
+        P* op = reinterpret_cast<P*>(a.out) + RowPack(row);
 #pragma unroll
         for (int j = 0; j < kMaxPacks; ++j) {
           const int p = t + j * kGroup;
@@ -477,6 +572,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
             float2 gm[kPairs], dv[kPairs], o2[kPairs];
             LoadRowVector(gsm, p, gm);
             WidenPack<kVec>(cd[j], dv);
+            Mask(p, dv);
 #pragma unroll
             for (int q = 0; q < kPairs; ++q) {
               xv[j][q] = Fma2(xv[j][q], inv2, shift2);  // x_hat from here on
@@ -485,7 +581,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
             }
             P o;
             NarrowPack<kVec>(o2, o);
-            StoreStream(op + p, o);
+            StorePack(op, p, o);
             // Column sums: dgamma += dy * x_hat, dbeta += dy.
 #pragma unroll
             for (int q = 0; q < kPairs; ++q) {
@@ -505,8 +601,8 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
       const float inv = 1.0f / sqrtf(ms + a.epsilon);
       const float2 inv2 = Dup(inv);
       if (live && t == 0) static_cast<T*>(a.stat_t)[row] = FromF32<T>(inv);
-      P* yp = reinterpret_cast<P*>(a.out) + row * packs;
-      P* np = reinterpret_cast<P*>(a.out2) + row * packs;
+      P* yp = reinterpret_cast<P*>(a.out) + RowPack(row);
+      P* np = reinterpret_cast<P*>(a.out2) + RowPack(row);
 #pragma unroll
       for (int j = 0; j < kMaxPacks; ++j) {
         const int p = t + j * kGroup;
@@ -521,8 +617,8 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
           P o, nrm;
           NarrowPack<kVec>(n2, nrm);
           NarrowPack<kVec>(o2, o);
-          StoreStream(np + p, nrm);
-          StoreStream(yp + p, o);
+          StorePack(np, p, nrm);
+          StorePack(yp, p, o);
         }
       }
     } else {  // kOpRmsGrad
@@ -535,6 +631,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
           float2 gm[kPairs], dv[kPairs];
           LoadRowVector(gsm, p, gm);
           WidenPack<kVec>(cd[j], dv);
+          Mask(p, dv);
 #pragma unroll
           for (int q = 0; q < kPairs; ++q) {
             gv[j][q] = Mul2(dv[q], gm[q]);
@@ -546,7 +643,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
       const float inv = live ? ToF32(static_cast<const T*>(a.inv_in)[row]) : 0.0f;
       const float2 inv2 = Dup(inv);
       const float2 ncoeff = Dup(-(dot * inv * inv * inv * inv_n));
-      P* op = reinterpret_cast<P*>(a.out) + row * packs;
+      P* op = reinterpret_cast<P*>(a.out) + RowPack(row);
 #pragma unroll
       for (int j = 0; j < kMaxPacks; ++j) {
         const int p = t + j * kGroup;
@@ -558,7 +655,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
           }
           P o;
           NarrowPack<kVec>(o2, o);
-          StoreStream(op + p, o);
+          StorePack(op, p, o);
         }
       }
     }
@@ -575,7 +672,16 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
 #pragma unroll
     for (int j = 0; j < kMaxPacks; ++j) {
       const int p = t + j * kGroup;
-      if (Has(j)) {
+      if (kShifted && Has(j)) {
+        // Plain [2][row_size] slabs: the row lanes' shifts differ.
+#pragma unroll
+        for (int e = 0; e < kVec; ++e) {
+          if (!Inside(p, e)) continue;
+          const int c = p * kVec + e - shift;
+          my_slab[c] = (e & 1) ? ag[j][e / 2].y : ag[j][e / 2].x;
+          my_slab[a.row_size + c] = (e & 1) ? ab[j][e / 2].y : ab[j][e / 2].x;
+        }
+      } else if (Has(j)) {
 #pragma unroll
         for (int h = 0; h < kQuads; ++h) {
           *reinterpret_cast<float4*>(my_slab + (h * packs + p) * 4) = make_float4(
@@ -591,7 +697,8 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
       const int half = c / a.row_size;
       const int col = c - half * a.row_size;
       const int e = col % kVec;
-      const int at = ((half * kQuads + e / 4) * packs + col / kVec) * 4 + (e & 3);
+      const int at =
+          kShifted ? c : ((half * kQuads + e / 4) * packs + col / kVec) * 4 + (e & 3);
       float s = slab[at];
       for (int l = 1; l < kRows; ++l) s += slab[static_cast<size_t>(l) * 2 * a.row_size + at];
       out[c] = s;
@@ -748,19 +855,22 @@ inline int MaxGradCtas() { return SmCount() * kMaxGradCtasPerSm; }
 // of a CTA (2 * row_size floats per row lane) are never larger than two
 // stages of the two-input ring.
 template <int kOp>
-size_t RowSmemBytes(int group, int elem_bytes, int threads, int max_packs, int row_size) {
+size_t RowSmemBytes(int group, int elem_bytes, int threads, int max_packs, int row_size,
+                    bool shifted) {
   size_t bytes = static_cast<size_t>(RowStages(kOp, group, elem_bytes)) * RowPipe<kOp>::kInputs *
                  max_packs * threads * 16;
-  bytes += static_cast<size_t>(kOp == kOpLnFwd ? 2 : 1) * row_size * sizeof(float);
+  const int words = shifted ? ShiftedWords(row_size, 16 / elem_bytes) : row_size;
+  bytes += static_cast<size_t>(kOp == kOpLnFwd ? 2 : 1) * words * sizeof(float);
   return bytes;
 }
 
-template <typename T, int kGroup, int kMaxPacks, int kOp, bool kFull>
+template <typename T, int kGroup, int kMaxPacks, int kOp, int kLayout>
 int LaunchGroupAs(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
   constexpr int kThreads = RowThreads(kGroup, kOp);
   constexpr int kRows = kThreads / kGroup;
-  auto kernel = RowNormKernel<T, kGroup, kMaxPacks, kOp, kFull>;
-  size_t smem = RowSmemBytes<kOp>(kGroup, sizeof(T), kThreads, kMaxPacks, a.row_size);
+  auto kernel = RowNormKernel<T, kGroup, kMaxPacks, kOp, kLayout>;
+  size_t smem = RowSmemBytes<kOp>(kGroup, sizeof(T), kThreads, kMaxPacks, a.row_size,
+                                  kLayout == kRowsShifted);
   // Function attributes and occupancy are per-device state; both are cached
   // per device for this instantiation.  The shared-memory size depends on the
   // row length, so the attribute is raised when a longer row arrives and the
@@ -808,6 +918,11 @@ int LaunchGroupAs(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
   if (per_sm > kCap) per_sm = kCap;
   const int64_t need = CeilDiv(a.rows, kRows);
   int64_t grid = static_cast<int64_t>(SmCount()) * per_sm;
+  if (kLayout == kRowsShifted && grid < need) {
+    // Consecutive rows of a thread a multiple of the pack width apart.
+    constexpr int kStep = VecWidth<T>::value > kRows ? VecWidth<T>::value / kRows : 1;
+    grid -= grid % kStep;
+  }
   if (grid > need) grid = need;
   *ctas_out = static_cast<int>(grid);
   return static_cast<int>(LaunchChained(true, kernel, dim3(static_cast<unsigned>(grid)),
@@ -816,16 +931,19 @@ int LaunchGroupAs(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
 
 template <typename T, int kGroup, int kMaxPacks, int kOp>
 int LaunchGroup(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
+  if (a.row_size % VecWidth<T>::value != 0) {
+    return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, kRowsShifted>(a, ctas_out, stream);
+  }
   // Rows that fill the layout need no per-pack presence checks.  Only the
   // LayerNorm gradient gains from the specialised form (fp32 rows of 1024:
   // +8 %); the forward kernels measured the same or, where the compiler then
   // spills under their register cap, slower.
   if constexpr (kOp == kOpLnGrad) {
     if (a.row_size / VecWidth<T>::value == kGroup * kMaxPacks) {
-      return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, true>(a, ctas_out, stream);
+      return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, kRowsFull>(a, ctas_out, stream);
     }
   }
-  return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, false>(a, ctas_out, stream);
+  return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, kRowsPacked>(a, ctas_out, stream);
 }
 
 template <typename T, int kOp>
@@ -839,14 +957,22 @@ int LaunchLoop(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
                                         stream, a));
 }
 
+// Packs that a row can touch, wherever it starts.
+template <typename T>
+inline int RowPacks(int row_size) {
+  constexpr int kVec = VecWidth<T>::value;
+  return row_size % kVec == 0 ? row_size / kVec : (row_size + 2 * kVec - 2) / kVec;
+}
+
 template <typename T, int kOp, int kMaxPacks>
 int DispatchPacks(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
-  constexpr int kVec = VecWidth<T>::value;
-  const int packs = a.row_size / kVec;
+  const int packs = RowPacks<T>(a.row_size);
+  const bool shifted = a.row_size % VecWidth<T>::value != 0;
   const auto fits = [&](int group) {
     if (packs > group * kMaxPacks) return false;
     const int threads = RowThreads(group, kOp);
-    return RowSmemBytes<kOp>(group, sizeof(T), threads, kMaxPacks, a.row_size) <= 200 * 1024;
+    return RowSmemBytes<kOp>(group, sizeof(T), threads, kMaxPacks, a.row_size, shifted) <=
+           200 * 1024;
   };
   if (fits(8)) return LaunchGroup<T, 8, kMaxPacks, kOp>(a, ctas_out, stream);
   if (fits(32)) return LaunchGroup<T, 32, kMaxPacks, kOp>(a, ctas_out, stream);
@@ -864,8 +990,17 @@ int DispatchPacks(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
 
 template <typename T, int kOp>
 int Dispatch(const RowArgs& a, bool aligned, int* ctas_out, cudaStream_t stream) {
-  constexpr int kVec = VecWidth<T>::value;
-  if (aligned && a.row_size % kVec == 0) {
+  // Rows that are not whole packs take the same layouts (kRowsShifted).  Us
+  // against the element form, LayerNorm forward / gradient, RMSNorm forward /
+  // gradient: bf16 [65536,1001] 241, 626, 144, 159 -> 78, 146, 84, 81; fp32
+  // [32768,1001] 113, 368, 86, 85 -> 62, 93, 74, 77; bf16 [8192,771] 30, 72, 18, 19
+  // -> 13, 27, 12, 13.  The two ops with one store per load lose where a handful
+  // of long rows each fill an SM (fp32 [500,5001]: 9.2 -> 10.2 and 8.6 -> 9.1; the
+  // element form runs them all at once): those keep it.
+  const bool few_long_rows = a.row_size % VecWidth<T>::value != 0 && RowPacks<T>(a.row_size) > 1024 &&
+                             a.rows <= static_cast<int64_t>(SmCount()) * kMaxCtasPerSm &&
+                             (kOp == kOpLnFwd || kOp == kOpRmsGrad);
+  if (aligned && !few_long_rows) {
     // Packs per thread.  Four keep short rows inside one warp (shuffle-only
     // sums) and measured best for rows that fill the layout.  Rows of 3 * 2^k
     // packs (768, 1536, 3072 ... bf16 columns) take three: the layout is then
@@ -879,7 +1014,7 @@ int Dispatch(const RowArgs& a, bool aligned, int* ctas_out, cudaStream_t stream)
     int want = GetTuning(kTuneRowNormPacks);
     if (want < 1 || want > 4) {
       want = 4;
-      const int packs = a.row_size / kVec;
+      const int packs = RowPacks<T>(a.row_size);
       int group = 512;
       for (int g : {8, 32, 64, 128, 256}) {
         if (g == 64 && sizeof(T) != 2) continue;  // as in DispatchPacks

@@ -267,3 +267,46 @@ def test_every_register_layout_gives_the_same_answers(kernel_lib, packs, n):
         assert_close(to_numpy(ry), np_ref.rms_norm(x, gamma)[0], rt, at, "rms y")
         assert_close(to_numpy(rdx), np_ref.rms_norm_grad_dx(x, to_numpy(rinv), gamma, dy),
                      rt * 5, at * 5 + 1e-5, "rms dx")
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("rows,n", [(1, 3), (2, 9), (7, 17), (3000, 31), (5, 257), (1500, 1001),
+                                    (900, 2050), (700, 3333), (400, 4099), (301, 8190)])
+def test_rows_that_start_inside_a_pack(kernel_lib, rows, n, dtype):
+    """Row lengths that are not whole packs: rows start anywhere inside a
+    128-bit pack, the first and last pack hold elements of the neighbouring
+    rows.  All four ops against the element form (the same values off a 16-byte
+    boundary), with huge values beside every row's ends: a neighbour that leaked
+    into a row would show."""
+    rng = np.random.default_rng(rows + n)
+    d = {"float32": torch.float32, "float16": torch.float16, "bfloat16": torch.bfloat16}[dtype]
+    x = rng.standard_normal((rows, n)) + 0.5
+    dy = rng.standard_normal((rows, n)) * 0.1
+    x[::3] *= 100.0       # neighbours of another scale
+    dy[::3] *= 100.0
+    x, dy = (torch.from_numpy(t).to(d).cuda() for t in (x, dy))
+    g, b = (torch.from_numpy(rng.standard_normal(n)).to(d).cuda() for _ in range(2))
+
+    def unaligned(t):
+        return torch.cat((t.new_zeros(1), t.reshape(-1)))[1:].view(t.shape)
+
+    def run(x, dy):
+        out = [raw_ops.MusaLayerNorm(x, g, b), *raw_ops.MusaLayerNormGrad(dy, x, g, b)]
+        if d != torch.float16:
+            f = raw_ops.MusaRmsNorm(x, g)
+            out += [*f, raw_ops.MusaRmsNormGradDx(x, f.inv_rms, g, dy)]
+        torch.cuda.synchronize()
+        return out
+
+    got, again, want = run(x, dy), run(x, dy), run(unaligned(x), unaligned(dy))
+    # fp32 sums in another order (a few hundred ulps of the largest term for the
+    # column sums), one rounding of T in the 16-bit results.
+    rt = 1e-5 if d == torch.float32 else 2.0 ** (-9 if d == torch.float16 else -6)
+    for i, (a, same, ref) in enumerate(zip(got, again, want)):
+        assert torch.equal(a, same), i
+        a, ref = a.double(), ref.double()
+        if i in (2, 3):    # dgamma, dbeta: sums over rows of very different scale
+            scale = dy.double().abs().max() * max(rows, 1) ** 0.5 * (4 if i == 2 else 1)
+        else:
+            scale = ref.abs().amax(-1, keepdim=True).clamp_min(1e-12)
+        assert bool(((a - ref).abs() <= rt * ref.abs() + rt * scale).all()), i
