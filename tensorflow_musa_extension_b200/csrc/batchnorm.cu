@@ -854,8 +854,8 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Channel-major planes whose length is not a whole number of packs (7x7,
-// 5x5, 3x3 ...): single planes cannot be read with 128-bit accesses, but a
+// Channel-major planes of up to 2816 elements.  Where a plane is not a whole
+// number of packs (7x7, 5x5, 3x3 ...) it cannot be read with 128-bit accesses, but a
 // GROUP of kVec neighbouring channels can - its kVec * inner elements are
 // `inner` whole packs, and the group starts on a 16-byte boundary for every n.
 // A CTA owns one group and a split of the outer axis; thread t reads pack t of
@@ -864,8 +864,8 @@ __global__ void __launch_bounds__(kThreads)
 // a thread's pack always covers the same one or two channels: the first
 // `before` elements belong to channel lo, the rest to lo + 1.
 // Packs of a run per thread: inner <= 11 * 256, whose per-pack sums (16 bytes
-// each) fit the shared memory of a plain launch.  bf16 [64,64,33,33] with single
-// elements instead: 26.6 us forward, 32.8 gradient (new figures below).
+// each) fit the shared memory of a plain launch.  bf16 [64,64,33,33], single
+// elements -> this form: forward 26.6 -> 20.8 us, gradient 32.8 -> 20.5.
 constexpr int kGroupSlots = 11;
 constexpr int kGroupUnroll = 4;  // values of n in flight per thread
 
@@ -2540,12 +2540,16 @@ inline int PlaneVec(int64_t inner, bool aligned) {
   return 1;
 }
 
-// The channel-group form applies to planes that are not whole packs, when the
-// groups tile the channel axis and a thread has at most kGroupSlots packs.
+// The channel-group form applies when the groups tile the channel axis and a
+// thread has at most kGroupSlots packs; a CTA reads runs of whole groups (6 KB of
+// 14x14 planes) where the warp-per-channel form reads single planes.  Forward,
+// gradient, inference in us, warp per channel -> groups: fp32 [256,512,14,14] 84,
+// 89, 39 -> 56, 90, 38; fp32 [256,128,28,28] 90, 94, 42 -> 59, 94, 38; bf16
+// [256,128,28,28] 34, 53, 16.3 -> 31, 53, 14.9.
 template <typename T>
 inline bool UseChannelGroups(const Geom& g, bool aligned) {
   constexpr int kG = VecWidth<T>::value;
-  return aligned && g.inner % kG != 0 && g.inner >= kG &&
+  return aligned && g.inner >= kG &&
          g.inner <= static_cast<int64_t>(kGroupSlots) * kThreads && g.channels % kG == 0;
 }
 struct GroupPlan {
@@ -2557,8 +2561,10 @@ inline GroupPlan PlanGroups(const Geom& g) {
   constexpr int kG = VecWidth<T>::value;
   GroupPlan p;
   p.gx = g.channels / kG;
-  const int64_t t = (g.inner + 31) / 32 * 32;
-  p.threads = static_cast<int>(t < kThreads ? t : kThreads);
+  // The run of `inner` packs in as few equal slots as 256 threads allow (784 packs
+  // are 4 x 196, not 3 x 256 + 16).
+  const int64_t per_slot = CeilDiv(g.inner, CeilDiv(g.inner, kThreads));
+  p.threads = static_cast<int>((per_slot + 31) / 32 * 32);
   const int64_t per_sm = GroupCtas(kMode, sizeof(T)) * kThreads / p.threads;   // one wave
   int64_t target = static_cast<int64_t>(SmCount()) * per_sm / (p.gx > 0 ? p.gx : 1);
   if (target < 1) target = 1;
