@@ -614,6 +614,7 @@ int LaunchApplyAdamGroupHostTable(int state_dtype, int grad_dtype, void* const* 
   if (count < 0) return MUSA_KERNELS_EINVAL;
   if (count == 0) return MUSA_KERNELS_OK;
   if (!var || !m || !v || !grad || !sizes) return MUSA_KERNELS_EINVAL;
+  try {   // (host tables of the overlap check)
 #define MUSA_ADAM_GROUP(S, G)                                                              \
   return LaunchAdamGroup<S, G>(var, m, v, grad, sizes, count, lr_t, beta1, beta2, epsilon, \
                                use_nesterov, stream)
@@ -626,6 +627,9 @@ int LaunchApplyAdamGroupHostTable(int state_dtype, int grad_dtype, void* const* 
     if (state_dtype == MUSA_DT_BF16) MUSA_ADAM_GROUP(__nv_bfloat16, __nv_bfloat16);
   }
 #undef MUSA_ADAM_GROUP
+  } catch (const std::bad_alloc&) {
+    return MUSA_KERNELS_ETOOLARGE;
+  }
   return MUSA_KERNELS_EUNSUPPORTED;
 }
 
