@@ -1,4 +1,5 @@
-"""Builds libmusa_plugin_kernels.so (the sm_100a launcher layer) in-tree.
+"""Builds libmusa_plugin_kernels.so (the sm_100a launcher layer) and _native_ops.so
+(the native host path of the ops, host code against the installed torch) in-tree.
 
     python -m tensorflow_musa_extension_b200.build [--force] [--verbose]
 
