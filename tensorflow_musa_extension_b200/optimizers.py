@@ -32,7 +32,8 @@ def apply_adam_mixed(var, m, v, beta1_power, beta2_power, lr, beta1, beta2,
 
 class MusaAdam:
     """Adam over device tensors: one fused launch for neighbouring variables of
-    one state and gradient type."""
+    one state and gradient type where the pairs come as a list or tuple, else
+    one per variable."""
 
     _LOWP_GRAD_DTYPES = (torch.float32, torch.bfloat16, torch.float16)
 
@@ -72,7 +73,12 @@ class MusaAdam:
 
     def apply_gradients(self, grads_and_vars):
         """One step over (grad, var) pairs; returns the new iteration count.
-        Neighbouring variables of one kind are updated by one launch."""
+        Neighbouring variables of one kind in a list or tuple are updated by
+        one launch.  Any other iterable may make a pair when it is asked for it
+        (refill one gradient buffer, read a variable that the pair before has
+        updated, switch streams), so each of its pairs is updated before the
+        next one is asked for."""
+        together = type(grads_and_vars) in (list, tuple)
         step = self.iterations + 1
         b1p = self.beta_1 ** step
         b2p = self.beta_2 ** step
@@ -103,6 +109,8 @@ class MusaAdam:
                         flush()
                         kind = this
                     group.append((t, m, v, grad))
+                    if not together:
+                        flush()
                     continue
                 flush()
                 if t.dtype == torch.float32:
