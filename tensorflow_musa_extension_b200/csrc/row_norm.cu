@@ -19,6 +19,7 @@
 // cancel.  Rows that do not fit the register form (very long, or not a whole
 // number of aligned packs) take a CTA-per-row kernel with element accesses.
 #include "common.cuh"
+#include "row_layout.h"
 #include "trace.h"
 #include "tuning.h"
 #include "../../include/musa_plugin_kernels.h"
@@ -287,6 +288,8 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
   float* gsm = reinterpret_cast<float*>(ring + kStages * kInputs * kMaxPacks * kThreads);
   constexpr bool kFull = kLayout == kRowsFull;
   constexpr bool kShifted = kLayout == kRowsShifted;
+  // Rows shorter than a pack (at most two packs) always come to groups of 8.
+  constexpr int kTailRows = kGroup == 8 ? kVec : 1;
   float* bsm = gsm + (kShifted ? ShiftedWords(a.row_size, kVec) : a.row_size);
   // LayerNorm gradient, after the last row: one slab [2][kVec / 4][packs][4]
   // of column sums per row lane, laid over the ring.
@@ -298,13 +301,12 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
   // (the same for all rows of this thread), and the packs that hold the row.
   int shift = 0;
   if constexpr (kShifted) {
-    const int64_t row0 = static_cast<int64_t>(blockIdx.x) * kRows + lane_row;
-    shift = static_cast<int>((row0 % kVec) * (a.row_size % kVec) % kVec);
+    shift = RowShift<kVec>(static_cast<int64_t>(blockIdx.x) * kRows + lane_row, a.row_size);
   }
-  const int packs = kShifted ? (a.row_size + shift + kVec - 1) / kVec : a.row_size / kVec;
+  const int packs = kShifted ? ShiftedPacks<kVec>(a.row_size, shift) : a.row_size / kVec;
   // First pack of a row in units of packs from the tensor's start.
   const auto RowPack = [&](int64_t row) {
-    return kShifted ? (row * a.row_size - shift) / kVec : row * packs;
+    return kShifted ? ShiftedRowPack<kVec>(row, a.row_size, shift) : row * packs;
   };
   // Pack p holds elements of other rows too; element e of it belongs to the row.
   const auto Edge = [&](int p) { return kShifted && (p == 0 || p == packs - 1); };
@@ -390,9 +392,10 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
         if (Has(j)) {
           uint4* const to_x = mine + ((stage * kInputs + 0) * kMaxPacks + j) * kThreads;
           uint4* const to_d = mine + ((stage * kInputs + 1) * kMaxPacks + j) * kThreads;
-          if (kShifted && p == packs - 1 && row == a.rows - 1) {
+          if (kShifted && MayEndTensor<kTailRows>(row, a.rows, p, packs)) {
             // The tensor's last pack: no byte beyond its end is read.
-            const int bytes = (a.row_size + shift - p * kVec) * static_cast<int>(sizeof(T));
+            const int bytes = PackElements<kVec, kTailRows>(row, a.rows, a.row_size, shift, p) *
+                              static_cast<int>(sizeof(T));
             AsyncCopyPart(to_x, xp + p, bytes);
             if constexpr (kGrad) AsyncCopyPart(to_d, dp + p, bytes);
           } else {
