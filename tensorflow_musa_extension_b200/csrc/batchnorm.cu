@@ -2985,10 +2985,14 @@ inline OnChipPlan PlanOnChip(const Geom& g) {
       if (forced_k > 0 && k != forced_k) continue;
       const int64_t per = CeilDiv(g.outer, k);
       const int64_t slots = CeilDiv(per, kOnChipThreads / tx);
-      // Few channels and many rows: too few CTAs to keep up with the chain
-      // (bf16 [100352,64], 64 CTAs of 25 slots: 15.4 us against 11.8;
-      // fp32 [65536,32], 16 slots: 10.2 against 9.2).
-      if (tx < 4 && gx * k < 100 && slots * kStreams > 12) continue;
+      // Few channels and many rows: too few CTAs to keep up with the chain.
+      // Segments of 32 bytes: bf16 [100352,64], 64 CTAs of 25 slots: 15.4 us
+      // against 11.8; fp32 [65536,32], 16 slots: 10.2 against 9.2.  Wider ones (48
+      // CTAs of whole 64-byte segments): bf16 [50176,64], 32 CTAs of 25 slots:
+      // 11.3 against 9.5; bf16 [50176,32], 16 CTAs: 10.3 against 8.8; fp16
+      // [50176,72], 48 CTAs, a third of them a quarter full: 13.8 against
+      // 11.3; but fp32 [50176,48], 48 CTAs: 9.5 against 9.9.
+      if ((tx < 4 ? gx * k < 100 : cv * k < 48 * 4) && slots * kStreams > 12) continue;
       OnChipTry(&best, BnOnChipKernel<T, kMode>, by_device, tx, gx, k, per, slots, kStreams,
                 tx < 4 ? 1.25 : tx < 8 ? 1.08 : 1.0);
     }

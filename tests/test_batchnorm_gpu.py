@@ -779,3 +779,21 @@ def test_rows_that_are_not_whole_packs(kernel_lib, dtype, rows, c):
             rt = _rt(dtype) if k == 0 and i < 4 else 1e-5
             floor = max(_rms(b), terms if i in (2, 3) and k == 0 else 1e-12)
             assert np.all(np.abs(a - b) <= rt * np.abs(b) + rt * floor), (i, k)
+
+
+@pytest.mark.parametrize("dtype,rows,c,one_kernel", [
+    ("bfloat16", 49152, 64, True),      # 64 CTAs of 12 slots
+    ("bfloat16", 49153, 64, False),     # 13 slots, or 32 CTAs of 25
+    ("float16", 51200, 64, False), ("bfloat16", 50176, 32, False), ("float32", 50176, 32, False),
+    ("bfloat16", 49153, 40, False), ("float16", 50176, 72, False),
+    ("float32", 50176, 48, True)])      # 48 CTAs of 25
+def test_long_narrow_layers(kernel_lib, dtype, rows, c, one_kernel):
+    """A forward of few channels and many rows leaves the one-kernel form where its
+    cuts are too few CTAs, whichever way the columns are cut."""
+    x, s, o, dy = bn_inputs(rows + c, (rows, c), dtype, 1.0, 3.0)
+    tx, e = to_torch(x), torch.empty(0, device="cuda")
+    before = kernel_lib.MusaKernelsLaunchCount()
+    fwd = raw_ops.FusedBatchNormV3(tx, to_torch(s), to_torch(o), e, e, epsilon=EPS)
+    launches = kernel_lib.MusaKernelsLaunchCount() - before
+    assert (launches == 1) == one_kernel
+    check_forward(fwd, np_ref.fused_batch_norm(x, s, o, epsilon=EPS), dtype)
