@@ -2540,18 +2540,6 @@ inline int PlaneVec(int64_t inner, bool aligned) {
   return 1;
 }
 
-// The channel-group form applies when the groups tile the channel axis and a
-// thread has at most kGroupSlots packs; a CTA reads runs of whole groups (6 KB of
-// 14x14 planes) where the warp-per-channel form reads single planes.  Forward,
-// gradient, inference in us, warp per channel -> groups: fp32 [256,512,14,14] 84,
-// 89, 39 -> 56, 90, 38; fp32 [256,128,28,28] 90, 94, 42 -> 59, 94, 38; bf16
-// [256,128,28,28] 34, 53, 16.3 -> 31, 53, 14.9.
-template <typename T>
-inline bool UseChannelGroups(const Geom& g, bool aligned) {
-  constexpr int kG = VecWidth<T>::value;
-  return aligned && g.inner >= kG &&
-         g.inner <= static_cast<int64_t>(kGroupSlots) * kThreads && g.channels % kG == 0;
-}
 struct GroupPlan {
   int64_t gx, gy, per;
   int threads;
@@ -2565,17 +2553,100 @@ inline GroupPlan PlanGroups(const Geom& g) {
   // are 4 x 196, not 3 x 256 + 16).
   const int64_t per_slot = CeilDiv(g.inner, CeilDiv(g.inner, kThreads));
   p.threads = static_cast<int>((per_slot + 31) / 32 * 32);
-  const int64_t per_sm = GroupCtas(kMode, sizeof(T)) * kThreads / p.threads;   // one wave
-  int64_t target = static_cast<int64_t>(SmCount()) * per_sm / (p.gx > 0 ? p.gx : 1);
-  if (target < 1) target = 1;
-  int64_t gy = target < g.outer ? target : g.outer;
+  const int64_t wave = static_cast<int64_t>(SmCount()) *
+                       (GroupCtas(kMode, sizeof(T)) * kThreads / p.threads);
   const int64_t cap = MaxSplits(g.outer, g.channels);
-  if (gy > cap) gy = cap;
-  if (gy > 65535) gy = 65535;
-  if (gy < 1) gy = 1;
-  p.per = CeilDiv(g.outer, gy);
-  p.gy = CeilDiv(g.outer, p.per);
+  // The outer axis in as many pieces as one to six whole waves hold, whichever
+  // takes the fewest images one after the other; the start and end of a CTA count
+  // as four.  (One wave alone, rounded down, is 58 % full at 256 groups of three
+  // CTAs an SM: fp32 [128,1024,14,14] gradient 96.8 us, in three waves, and the
+  // statistics by planes, 82.7.)
+  int64_t best = 0;
+  for (int w = 1; w <= 6; ++w) {
+    int64_t gy = w * wave / (p.gx > 0 ? p.gx : 1);
+    // Beyond eight CTAs an SM only pieces of four images or more: CTAs of two or
+    // three warps with an image each are all start and end (fp32 inference of
+    // [32,320,7,7] 3.1 us with 17 an SM, 2.1 with eight).
+    const int64_t fours = CeilDiv(g.outer, 4), eight = 8 * SmCount() / (p.gx > 0 ? p.gx : 1);
+    if (gy > fours && gy > eight) gy = fours > eight ? fours : eight;
+    if (gy > g.outer) gy = g.outer;
+    if (gy > cap) gy = cap;
+    if (gy > 65535) gy = 65535;
+    if (gy < 1) gy = 1;
+    const int64_t per = CeilDiv(g.outer, gy);
+    gy = CeilDiv(g.outer, per);
+    const int64_t cost = CeilDiv(p.gx * gy, wave) * (per + 4);
+    if (w == 1 || cost < best) {
+      best = cost;
+      p.per = per;
+      p.gy = gy;
+    }
+  }
   return p;
+}
+
+// Whether a pass takes the channel-group kernel, and how it is cut.  The form is
+// possible when the groups tile the channel axis and a thread has at most
+// kGroupSlots packs.  A CTA then reads runs of whole groups where the
+// warp-per-channel kernels read single planes, with the widest access that
+// divides them (`access` bytes): better than those at 2 and 4 bytes and, at 8
+// and 16, where a thread has several images in flight (`per` images a CTA) to
+// pay for walking its `slots` one after the other.  Inputs beyond L2 are read
+// as fast by plain planes.  Us, warp per channel -> groups:
+//   statistics   fp32 [256,64,28,28] (six images a CTA) 48 -> 39, [8,512,28,28]
+//   (forward)    (two) 18.9 -> 19.5, [4,512,15,15] (one) 7.7 -> 9.1; bf16
+//                [64,512,20,20] 22 -> 20, [64,512,32,32] 38.7 -> 40.2 (hence 896),
+//                [16,512,30,30] (8-byte accesses, two) 19 -> 21, 64 images 48 -> 46,
+//                [4,512,29,29] (2-byte, one) 13.6 -> 14.7, 64 images 60 -> 35
+//   elements     fp32 [16,64,28,28] (one) 3.5 -> 5.0, 128 images (three) 13.8 ->
+//   (forward)    10.7; bf16 [16,64,28,28] 2.6 -> 4.1, [64,512,28,28] 19.2 -> 19.5,
+//                [16,64,30,30] (8-byte, one) 3.2 -> 4.6, [64,512,30,30] 29.7 -> 23.0,
+//                [64,512,21,21] (2-byte) 30 -> 12
+//   statistics   fp32 [32,512,14,14] 16.8 -> 15.8, [128,512,14,14] 45 -> 50,
+//   (gradient)   [16,512,28,28] 24.6 -> 29.2, [64,512,21,21] (4-byte) level,
+//                [32,512,29,29] 51 -> 53; bf16 [32,512,24,24] 22.0 -> 21.3,
+//                [64,512,28,28] 48.5 -> 50.3, [64,512,30,30] (8-byte) 52 -> 57,
+//                [32,512,29,29] (2-byte) 42 -> 32
+//   elements     fp32 [64,64,28,28] (three) 16.8 -> 15.7, [4,512,28,28] (two) 11.7 ->
+//   (gradient)   12.0; bf16 [32,512,24,24] 24.3 -> 22.0, [4,512,28,28] 9.3 -> 11.5
+template <typename T, int kMode, bool kStats>
+inline bool UseChannelGroups(const Geom& g, bool aligned, GroupPlan* plan) {
+  constexpr int kG = VecWidth<T>::value;
+  constexpr bool k32 = sizeof(T) == 4;
+  if (!aligned || g.inner < kG || g.inner > static_cast<int64_t>(kGroupSlots) * kThreads ||
+      g.channels % kG != 0 || g.channels / kG > 0x7fffffffLL) {
+    return false;
+  }
+  *plan = PlanGroups<T, kMode>(g);
+  const int access = PlaneVec<T>(g.inner, aligned) * static_cast<int>(sizeof(T));
+  const int64_t slots = CeilDiv(g.inner, kThreads);
+  const int64_t per = plan->per;
+  const int64_t elements = g.outer * g.channels * g.inner;
+  if (kStats && kMode == kFwd) {
+    if (k32) {
+      if (g.inner <= 128) return true;
+      return per >= (slots == 1 && access == 16 ? 2 : 3) &&
+             slots <= (access == 4 ? kGroupSlots : access == 8 ? 5 : 7);
+    }
+    return slots == 1 || (per >= 2 && (access <= 4 || slots <= (access == 8 ? 2 : 3))) ||
+           (per >= 4 && (access == 8 ? slots <= 4 : g.inner <= 896));
+  }
+  if (kMode == kFwd) {
+    if (access <= 4 || (k32 && access == 8)) return true;
+    if (access == 8) return slots <= 2 || per >= 2;
+    return elements < (int64_t{1} << 25) && (slots <= 2 || per >= 2) && (k32 || slots <= 3);
+  }
+  if (kStats) {
+    if (g.inner <= 128) return true;
+    if (k32) {
+      return per >= 4 && ((access == 4 && slots <= 2) ||
+                          (access == 16 && slots == 1 && elements < (int64_t{1} << 22)));
+    }
+    return per >= 2 && (access == 2 || slots <= (access == 4 ? 4 : access == 8 ? 1 : 3));
+  }
+  if (access <= 4 || (k32 && access == 8)) return true;
+  if (access == 8) return slots <= 2 || per >= 3;
+  return slots == 1 || (k32 ? per >= 3 : slots <= 3 && per >= 2);
 }
 
 // Stats launch: fills partial[splits][2][C]; returns splits or a negative
@@ -2630,8 +2701,8 @@ int LaunchStats(const T* x, const T* dy, const float* mean, float* partial,
     CountKernelLaunch();
     return p.gy;
   }
-  if (UseChannelGroups<T>(g, aligned) && g.channels / kVec <= 0x7fffffffLL) {
-    const GroupPlan gp = PlanGroups<T, kMode>(g);
+  GroupPlan gp;
+  if (UseChannelGroups<T, kMode, true>(g, aligned, &gp)) {
     BnStatsGroupKernel<T, kMode>
         <<<dim3(static_cast<unsigned>(gp.gx), static_cast<unsigned>(gp.gy)), gp.threads,
            static_cast<size_t>(g.inner) * sizeof(float4), stream>>>(
@@ -2841,8 +2912,8 @@ void LaunchApply(const T* x, const T* dy, T* out, const ApplyArgs& a,
     return;
   }
   const bool pdl = GetTuning(kTuneBnPdl) != 0;
-  if (UseChannelGroups<T>(g, aligned) && g.channels / kVec <= 0x7fffffffLL) {
-    const GroupPlan gp = PlanGroups<T, kMode>(g);
+  GroupPlan gp;
+  if (UseChannelGroups<T, kMode, false>(g, aligned, &gp)) {
     LaunchChained(pdl, BnApplyGroupKernel<T, kMode>,
                   dim3(static_cast<unsigned>(gp.gx), static_cast<unsigned>(gp.gy)),
                   dim3(gp.threads), 0, stream, x, dy, out, a, g.outer, g.channels,
