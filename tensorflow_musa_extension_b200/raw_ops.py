@@ -15,6 +15,7 @@ library they raise.
 """
 import collections
 import ctypes
+import logging
 import threading
 
 import numpy as np
@@ -32,6 +33,8 @@ except Exception:  # pragma: no cover
     _NP_BF16 = None
 
 ACT_IDENTITY, ACT_RELU, ACT_SWISH, ACT_SIGMOID = 0, 1, 2, 3
+
+logger = logging.getLogger(__name__)
 
 _SUFFIX = {torch.float32: "F32", torch.float16: "F16", torch.bfloat16: "BF16",
            torch.float64: "F64", torch.int32: "I32", torch.int64: "I64"}
@@ -51,18 +54,44 @@ def _lib():
     return _bound
 
 
+class _NoNativePath:
+    """Stands in for `_native_ops` where it cannot be loaded: declines every call."""
+
+    @staticmethod
+    def adam_kind(*args):
+        return -1
+
+    def __getattr__(self, name):
+        return self._decline
+
+    @staticmethod
+    def _decline(*args):
+        return None
+
+
 def _native():
     """The native host path: one C++ function per op that checks, allocates and
     launches.  It answers None for every call that is not contiguous device
     tensors of the op's types (host buffers, conversions, errors); the op then
-    takes its general path below."""
+    takes its general path below.  So do all calls where the extension module is
+    missing or was built against another torch (the kernels come from the kernel
+    library in any case)."""
     global _bound_native
     if _bound_native is None:
         _require_cuda()
         lib = _lib()
-        from . import _native_ops
-        _native_ops.bind(lib._handle)
-        _bound_native = _native_ops
+        with _bind_lock:
+            if _bound_native is None:
+                try:
+                    from . import _native_ops as native
+                    native.bind(lib._handle)
+                except ImportError as e:
+                    native = _NoNativePath()
+                    logger.warning(
+                        "The native host path of the ops cannot be loaded (%s): calls go through "
+                        "the slower Python path. Build it with `python -m "
+                        "tensorflow_musa_extension_b200.build`.", e)
+                _bound_native = native
     return _bound_native
 
 
