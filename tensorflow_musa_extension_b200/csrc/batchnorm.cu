@@ -3019,8 +3019,6 @@ inline double OnChipCost(int64_t slots, int k, double segments) {
 template <typename T>
 inline bool OnChipAllowed(const Geom& g, int streams) {
   if (GetTuning(kTuneBnOnChipTx) < 0) return false;
-  // A sweep of the chain's own keys wants the chain.
-  if (GetTuning(kTuneBnClusterFold) != 0 || GetTuning(kTuneBnApplyAddsRows) != 64) return false;
   return g.outer * g.channels * g.inner * static_cast<int64_t>(sizeof(T)) * streams <
          kOnChipMaxBytes;
 }

@@ -16,14 +16,15 @@ std::once_flag g_tuning_once;
 void InitTuningOnce() {
   std::call_once(g_tuning_once, [] {
     static const int defaults[kTuneCount] = {
-        /*AdamCtasPerSm*/ 0, /*AdamUnroll*/ 2, /*BnOnChipTx*/ 0,
-        /*BnOnChipCluster*/ 0, /*BnCtasPerSm*/ 0, /*BnClusterFold*/ 0,
+        /*AdamCtasPerSm*/ 0, /*AdamUnroll*/ 2, /*unused*/ 0,
+        /*unused*/ 0, /*BnCtasPerSm*/ 0, /*BnClusterFold*/ 0,
         /*BnApplyReverse*/ 1, /*BnStatsKeep*/ 1, /*BnStatsPipe*/ 4,
         /*BnApplyDeep*/ 1, /*BnPdl*/ 1, /*BnL2KeepMb*/ 64, /*RowNormPacks*/ 0,
         /*BnApplyAddsRows*/ 64, /*BnStatsMaxTx*/ 16, /*BnL2KeepPartial*/ 1,
         /*BnStatsDropRest*/ 1, /*BnApplyDropAll*/ 0, /*BnApplyEarlyLoads*/ 1,
         /*BnFinalizeLanes*/ 128, /*BnApplyCtasPerSm*/ 0, /*BnInterleave*/ 1,
-        /*BnApplyMaxTx*/ 16, /*BnFullWave*/ 1};
+        /*BnApplyMaxTx*/ 16, /*BnFullWave*/ 1,
+        /*BnOnChipTx*/ 0, /*BnOnChipCluster*/ 0};
     for (int i = 0; i < kTuneCount; ++i) g_tuning[i].store(defaults[i]);
   });
 }

@@ -8,8 +8,8 @@ namespace musa_b200 {
 enum TuningKey {
   kTuneAdamCtasPerSm = 0,   // 0: one tile per CTA; k: persistent, k CTAs per SM
   kTuneAdamUnroll = 1,      // packs in flight per thread and stream: 1, 2, 4
-  kTuneBnOnChipTx = 2,      // channel packs per column block of the one-kernel form; 0: by rule, -1: off
-  kTuneBnOnChipCluster = 3, // CTAs per cluster of the one-kernel form; 0: by rule
+  // 2 and 3: not used (the bias chains' grid and unroll of earlier builds; a number is
+  // not given a second meaning)
   kTuneBnCtasPerSm = 4,     // CTAs per SM of the BatchNorm statistics grids; 0: what fits
   kTuneBnClusterFold = 5,   // CTAs per cluster of the stats kernel that fold their partial rows on chip
                             // (the element-wise kernel adds the rest: no finalize kernel); 0, 1: off
@@ -32,7 +32,10 @@ enum TuningKey {
   kTuneBnInterleave = 21,   // 1: CTAs take row tiles round-robin instead of one contiguous range
   kTuneBnApplyMaxTx = 22,   // channel packs per column block of the element-wise kernel; 0: the row
   kTuneBnFullWave = 23,     // 1: with interleaved row tiles the grid keeps the full wave (no shrink to whole row ranges)
-  kTuneCount = 24
+  kTuneBnOnChipTx = 24,     // channel packs per column block (channel-major: channels per group) of the
+                            // one-kernel form; 0: by rule, -1: off (the chain of kernels at every size)
+  kTuneBnOnChipCluster = 25,  // CTAs per cluster of the one-kernel form; 0: by rule
+  kTuneCount = 26
 };
 
 int GetTuning(int key);

@@ -523,6 +523,7 @@ def test_chain_without_finalize_kernel(kernel_lib, fold, dtype, rows, c):
         torch.cuda.synchronize()
         return fwd, grad, infer
 
+    form = kernel_lib.MusaKernelsSetTuning(24, -1)   # the chain, whatever the size
     old_rows = kernel_lib.MusaKernelsSetTuning(13, 0)
     try:
         base = run()
@@ -538,6 +539,7 @@ def test_chain_without_finalize_kernel(kernel_lib, fold, dtype, rows, c):
     finally:
         kernel_lib.MusaKernelsSetTuning(5, old)
         kernel_lib.MusaKernelsSetTuning(13, old_rows)
+        kernel_lib.MusaKernelsSetTuning(24, form)
     check_forward(got[0], want, dtype)
     check_grad(got[1], wg, dtype, dx_scale=terms)
     check_grad(got[2], wi, dtype, dx_scale=terms)
@@ -667,8 +669,8 @@ def test_one_kernel_form(kernel_lib, dtype, cluster, shape, layout):
     """The one-kernel form (inputs held in shared memory, sums met over a
     cluster) against the oracle and against the chain of kernels, at the edges
     of its cuts: a single row, partly filled column blocks, CTAs without rows,
-    the last row slot; key 3 forces the cluster size (sizes that cannot hold
-    the layer fall back to the chain), key 2 = -1 turns the form off."""
+    the last row slot; key 25 forces the cluster size (sizes that cannot hold
+    the layer fall back to the chain), key 24 = -1 turns the form off."""
     c = shape[-1] if layout == "NHWC" else shape[1]
     axis = -1 if layout == "NHWC" else 1
     x, s, o, dy = bn_inputs(70 + c, shape, dtype, 1.0, 3.0, channel_axis=axis)
@@ -692,21 +694,21 @@ def test_one_kernel_form(kernel_lib, dtype, cluster, shape, layout):
         torch.cuda.synchronize()
         return fwd, grad, frozen
 
-    old = kernel_lib.MusaKernelsSetTuning(3, cluster)
+    old = kernel_lib.MusaKernelsSetTuning(25, cluster)
     try:
         before = kernel_lib.MusaKernelsLaunchCount()
         fwd, grad, frozen = run()
         launches = kernel_lib.MusaKernelsLaunchCount() - before
         again = run()
     finally:
-        kernel_lib.MusaKernelsSetTuning(3, old)
+        kernel_lib.MusaKernelsSetTuning(25, old)
     if cluster == 0:
         assert launches == 3     # every shape of this list takes the form
-    off = kernel_lib.MusaKernelsSetTuning(2, -1)
+    off = kernel_lib.MusaKernelsSetTuning(24, -1)
     try:
         chain = run()
     finally:
-        kernel_lib.MusaKernelsSetTuning(2, off)
+        kernel_lib.MusaKernelsSetTuning(24, off)
     check_forward(fwd, want, dtype)
     check_grad(grad, wg, dtype, dx_scale=terms)
     for a, b in zip((*fwd, *grad, *frozen), (t for out in again for t in out)):
@@ -759,13 +761,13 @@ def test_rows_that_are_not_whole_packs(kernel_lib, dtype, rows, c):
         t = to_torch(a)
         return torch.cat((t.new_zeros(1), t.reshape(-1)))[1:].view(t.shape)
 
-    old = kernel_lib.MusaKernelsSetTuning(2, -1)   # the chain, whatever the size
+    old = kernel_lib.MusaKernelsSetTuning(24, -1)   # the chain, whatever the size
     try:
         got = run(to_torch(x), to_torch(dy))
         again = run(to_torch(x), to_torch(dy))
         base = run(unaligned(x), unaligned(dy))
     finally:
-        kernel_lib.MusaKernelsSetTuning(2, old)
+        kernel_lib.MusaKernelsSetTuning(24, old)
     check_forward(got[0], want, dtype)
     check_grad(got[2], wg, dtype, dx_scale=terms)
     for out, same in zip(got, again):
@@ -797,3 +799,25 @@ def test_long_narrow_layers(kernel_lib, dtype, rows, c, one_kernel):
     launches = kernel_lib.MusaKernelsLaunchCount() - before
     assert (launches == 1) == one_kernel
     check_forward(fwd, np_ref.fused_batch_norm(x, s, o, epsilon=EPS), dtype)
+
+
+def test_retired_tuning_numbers_have_no_effect(kernel_lib):
+    """Keys 2 and 3 were the bias chains' launch shape: a program that still
+    sets them gets the same kernels as one that does not."""
+    x, s, o, dy = bn_inputs(3, (1000, 64), "float32", 1.0, 3.0)
+
+    def launches():
+        before = kernel_lib.MusaKernelsLaunchCount()
+        out = run_both(x, s, o, dy, "NHWC")
+        return kernel_lib.MusaKernelsLaunchCount() - before, out
+
+    want = launches()
+    old = [kernel_lib.MusaKernelsSetTuning(k, v) for k, v in ((2, -1), (3, 8))]
+    try:
+        got = launches()
+    finally:
+        for k, v in zip((2, 3), old):
+            kernel_lib.MusaKernelsSetTuning(k, v)
+    assert got[0] == want[0]
+    for a, b in zip((t for out in got[1] for t in out), (t for out in want[1] for t in out)):
+        assert torch.equal(a, b)

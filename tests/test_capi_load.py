@@ -82,6 +82,9 @@ def test_tuning_hook_round_trip(kernel_lib):
     assert kernel_lib.MusaKernelsGetTuning(1) == 4
     kernel_lib.MusaKernelsSetTuning(1, old)
     assert kernel_lib.MusaKernelsSetTuning(999, 1) == -1
+    # The one-kernel BatchNorm form has numbers of its own (24, 25), by rule at first.
+    assert kernel_lib.MusaKernelsSetTuning(24, 0) == 0
+    assert kernel_lib.MusaKernelsSetTuning(25, 0) == 0
 
 
 def test_loader_reports_search_locations(monkeypatch, tmp_path):
