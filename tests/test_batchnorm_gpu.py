@@ -1,5 +1,6 @@
 """FusedBatchNorm forward / gradient on the GPU (through the C ABI) against the
 CPU oracle and the committed golden vectors."""
+import contextlib
 import ctypes
 
 import numpy as np
@@ -63,6 +64,55 @@ def run_both(x, scale, offset, dy, fmt):
                                         fwd.reserve_space_3, epsilon=EPS, data_format=fmt,
                                         is_training=True)
     return fwd, grad
+
+
+@contextlib.contextmanager
+def tuned(lib, *pairs):
+    """Tuning keys set for the length of the block; (24, -1) is the chain of kernels
+    at every size."""
+    old = [(k, lib.MusaKernelsSetTuning(k, v)) for k, v in pairs]
+    try:
+        yield
+    finally:
+        for k, v in reversed(old):
+            lib.MusaKernelsSetTuning(k, v)
+
+
+def launch_ops(lib, x, scale, offset, dy, fmt="NHWC", est=None, factor=1.0, scratch=0xA5):
+    """Training forward, training gradient and frozen gradient (about the running
+    statistics `est` where given, else the batch's) through the C entry points,
+    with scratch and outputs that arrive holding arbitrary bytes."""
+    tx, tdy, ts, to_ = (to_torch(a) for a in (x, dy, scale, offset))
+    c = tx.shape[-1] if fmt == "NHWC" else tx.shape[1]
+    outer, inner = (tx.numel() // c, 1) if fmt == "NHWC" else (tx.shape[0], tx[0, 0].numel())
+    code, st = raw_ops._DT_CODE[tx.dtype], torch.cuda.current_stream().cuda_stream
+    need = max(lib.BnWorkspaceBytes(outer, c, inner), 16)
+
+    def ptrs(ts_):
+        return [t.data_ptr() for t in ts_]
+
+    def dirty():
+        return torch.full((need,), scratch, dtype=torch.uint8, device="cuda")
+
+    def outputs():
+        return [torch.full_like(tx, 999.0)] + [torch.full((c,), 999.0, device="cuda")
+                                               for _ in range(4)]
+
+    run = [to_torch(a) for a in est] if est is not None else None
+    out, r3, ws = outputs(), torch.full((), 999.0, device="cuda"), dirty()
+    assert lib.LaunchBnFwdTrainOp(code, *ptrs((tx, ts, to_)), *(ptrs(run) if run else (None, None)),
+                                  *ptrs(out), r3.data_ptr(), outer, c, inner, EPS, factor,
+                                  ws.data_ptr(), ws.numel(), st) == 0
+    fwd = raw_ops.FusedBatchNormV3Output(*out, r3)
+    results = [fwd]
+    for training in (True, False):
+        stats = (fwd.reserve_space_1, fwd.reserve_space_2) if training or not run else run
+        out, ws = outputs(), dirty()
+        assert lib.LaunchBnGradOp(code, *ptrs((tdy, tx, ts, *stats)), *ptrs(out), outer, c, inner,
+                                  EPS, training, ws.data_ptr(), ws.numel(), st) == 0
+        results.append(raw_ops.FusedBatchNormGradV3Output(*out))
+    torch.cuda.synchronize()
+    return results
 
 
 def test_golden_vectors(golden, kernel_lib):
@@ -252,26 +302,24 @@ def test_dirty_workspace_and_launch_shapes(kernel_lib, dtype, rows, c):
     x, s, o, dy = bn_inputs(300 + rows, (rows, c), dtype, 1.0, 3.0)
     want = np_ref.fused_batch_norm(x, s, o, epsilon=EPS)
     wg = np_ref.fused_batch_norm_grad(dy, x, s, want[3], want[4], EPS)
-    need = kernel_lib.BnWorkspaceBytes(rows, c, 1)
-    ws = raw_ops._workspace(need, torch.device("cuda", 0))
-    ws.fill_(0xA5)
-    fwd, grad = run_both(x, s, o, dy, "NHWC")
-    fwd2, grad2 = run_both(x, s, o, dy, "NHWC")
-    torch.cuda.synchronize()
-    for a, b in zip(list(fwd)[:5] + list(grad)[:3], list(fwd2)[:5] + list(grad2)[:3]):
-        assert torch.equal(a, b)
-    check_forward(fwd, want, dtype)
     terms = _rms(dy) * float(np.max(s / np.sqrt(want[4] + EPS)))
-    check_grad(grad, wg, dtype, dx_scale=terms)
+
+    def run(*pairs, scratch=0xA5):
+        with tuned(kernel_lib, *pairs):
+            return launch_ops(kernel_lib, x, s, o, dy, scratch=scratch)
+
+    chain = (24, -1)    # the keys below are the chain's
+    for pairs in ((), (chain,)):
+        fwd, grad, _ = run(*pairs)
+        fwd2, grad2, _ = run(*pairs, scratch=0x5A)
+        for a, b in zip(list(fwd)[:5] + list(grad)[:3], list(fwd2)[:5] + list(grad2)[:3]):
+            assert torch.equal(a, b)
+        check_forward(fwd, want, dtype)
+        check_grad(grad, wg, dtype, dx_scale=terms)
     for key, value in ((14, 256), (14, 8), (19, 32), (22, 0), (22, 8),
                        (21, 1 - kernel_lib.MusaKernelsGetTuning(21)),
                        (23, 1 - kernel_lib.MusaKernelsGetTuning(23))):
-        old = kernel_lib.MusaKernelsSetTuning(key, value)
-        try:
-            fwd3, grad3 = run_both(x, s, o, dy, "NHWC")
-            torch.cuda.synchronize()
-        finally:
-            kernel_lib.MusaKernelsSetTuning(key, old)
+        fwd3, grad3, _ = run(chain, (key, value))
         check_forward(fwd3, want, dtype)
         check_grad(grad3, wg, dtype, dx_scale=terms)
         assert_close(to_numpy(fwd.batch_mean), to_numpy(fwd3.batch_mean), 1e-5, 1e-6)
@@ -511,35 +559,13 @@ def test_chain_without_finalize_kernel(kernel_lib, fold, dtype, rows, c):
     wi = np_ref.fused_batch_norm_grad(dy, x, s, rm, rv, EPS, is_training=False)
     terms = _rms(dy) * float(np.max(s / np.sqrt(want[4] + EPS)))
 
-    def run():
-        tx = to_torch(x)
-        fwd = raw_ops.FusedBatchNormV3(tx, to_torch(s), to_torch(o), to_torch(rm), to_torch(rv),
-                                       epsilon=EPS, exponential_avg_factor=0.25)
-        grad = raw_ops.FusedBatchNormGradV3(to_torch(dy), tx, to_torch(s), fwd.reserve_space_1,
-                                            fwd.reserve_space_2, fwd.reserve_space_3,
-                                            epsilon=EPS)
-        infer = raw_ops.FusedBatchNormGradV3(to_torch(dy), tx, to_torch(s), to_torch(rm),
-                                             to_torch(rv), None, epsilon=EPS, is_training=False)
-        torch.cuda.synchronize()
-        return fwd, grad, infer
+    def run(*pairs, scratch=0x5A):
+        with tuned(kernel_lib, (24, -1), *pairs):
+            return launch_ops(kernel_lib, x, s, o, dy, est=(rm, rv), factor=0.25, scratch=scratch)
 
-    form = kernel_lib.MusaKernelsSetTuning(24, -1)   # the chain, whatever the size
-    old_rows = kernel_lib.MusaKernelsSetTuning(13, 0)
-    try:
-        base = run()
-    finally:
-        kernel_lib.MusaKernelsSetTuning(13, old_rows)
-    old = kernel_lib.MusaKernelsSetTuning(5, fold)
-    kernel_lib.MusaKernelsSetTuning(13, 4096)
-    try:
-        need = kernel_lib.BnWorkspaceBytes(rows, c, 1)
-        raw_ops._workspace(need, torch.device("cuda", 0)).fill_(0x5A)
-        got = run()
-        again = run()
-    finally:
-        kernel_lib.MusaKernelsSetTuning(5, old)
-        kernel_lib.MusaKernelsSetTuning(13, old_rows)
-        kernel_lib.MusaKernelsSetTuning(24, form)
+    base = run((13, 0))
+    got = run((13, 4096), (5, fold))
+    again = run((13, 4096), (5, fold), scratch=0xA5)
     check_forward(got[0], want, dtype)
     check_grad(got[1], wg, dtype, dx_scale=terms)
     check_grad(got[2], wi, dtype, dx_scale=terms)
@@ -637,24 +663,29 @@ def test_outputs_beside_the_statistics(kernel_lib, dtype, shape, layout):
     def ptrs(ts_):
         return [t.data_ptr() for t in ts_]
 
-    y, stats, r3 = torch.empty_like(tx), fresh(4), torch.full((), float("nan"), device="cuda")
-    assert kernel_lib.LaunchBnFwdInferOp(
-        code, *ptrs((tx, ts, to_, rm, rv, y, *stats, r3)), outer, c, inner, EPS, st) == 0
-    for got, want in zip(stats, (rm, rv, rm, rv)):
-        assert torch.equal(got, want)
-    assert float(r3) == 0.0
-    stats, r3 = fresh(4), torch.full((), float("nan"), device="cuda")
-    assert kernel_lib.LaunchBnFwdTrainOp(
-        code, *ptrs((tx, ts, to_)), None, None, *ptrs((y, *stats, r3)), outer, c, inner, EPS, 1.0,
-        ws.data_ptr(), ws.numel(), st) == 0
-    assert float(r3) == 0.0 and all(bool(torch.isfinite(t).all()) for t in stats)
-    for training in (True, False):
-        dx, outs = torch.empty_like(tx), fresh(4)
-        assert kernel_lib.LaunchBnGradOp(
-            code, *ptrs((tdy, tx, ts, stats[2], stats[3], dx, *outs)), outer, c, inner, EPS,
-            training, ws.data_ptr(), ws.numel(), st) == 0
-        assert all(bool(torch.isfinite(t).all()) for t in outs[:2])
-        assert not outs[2].any() and not outs[3].any()
+    def run_all():
+        y, stats, r3 = torch.empty_like(tx), fresh(4), torch.full((), float("nan"), device="cuda")
+        assert kernel_lib.LaunchBnFwdInferOp(
+            code, *ptrs((tx, ts, to_, rm, rv, y, *stats, r3)), outer, c, inner, EPS, st) == 0
+        for got, want in zip(stats, (rm, rv, rm, rv)):
+            assert torch.equal(got, want)
+        assert float(r3) == 0.0
+        stats, r3 = fresh(4), torch.full((), float("nan"), device="cuda")
+        assert kernel_lib.LaunchBnFwdTrainOp(
+            code, *ptrs((tx, ts, to_)), None, None, *ptrs((y, *stats, r3)), outer, c, inner, EPS, 1.0,
+            ws.data_ptr(), ws.numel(), st) == 0
+        assert float(r3) == 0.0 and all(bool(torch.isfinite(t).all()) for t in stats)
+        for training in (True, False):
+            dx, outs = torch.empty_like(tx), fresh(4)
+            assert kernel_lib.LaunchBnGradOp(
+                code, *ptrs((tdy, tx, ts, stats[2], stats[3], dx, *outs)), outer, c, inner, EPS,
+                training, ws.data_ptr(), ws.numel(), st) == 0
+            assert all(bool(torch.isfinite(t).all()) for t in outs[:2])
+            assert not outs[2].any() and not outs[3].any()
+
+    for pairs in ((), ((24, -1),)):      # by rule (mostly one kernel), and the chain
+        with tuned(kernel_lib, *pairs):
+            run_all()
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
