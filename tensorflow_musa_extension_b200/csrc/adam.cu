@@ -326,7 +326,14 @@ int LaunchAdamGroup(void* const* var, void* const* m, void* const* v,
     total += sizes[i];
   }
   MUSA_TRACE("LaunchApplyAdamGroup", (6 * sizeof(StateT) + sizeof(GradT)) * total);
-  if (AdamGroupOverlaps(var, m, v, grad, sizes, count, sizeof(StateT), sizeof(GradT))) {
+  bool one_by_one;
+  try {
+    one_by_one =
+        AdamGroupOverlaps(var, m, v, grad, sizes, count, sizeof(StateT), sizeof(GradT));
+  } catch (const std::bad_alloc&) {
+    one_by_one = true;   // no host memory for the check: right without it
+  }
+  if (one_by_one) {
     for (int i = 0; i < count; ++i) {
       LaunchAdam<StateT, GradT>(static_cast<StateT*>(var[i]), static_cast<StateT*>(m[i]),
                                 static_cast<StateT*>(v[i]), static_cast<const GradT*>(grad[i]),
@@ -614,7 +621,6 @@ int LaunchApplyAdamGroupHostTable(int state_dtype, int grad_dtype, void* const* 
   if (count < 0) return MUSA_KERNELS_EINVAL;
   if (count == 0) return MUSA_KERNELS_OK;
   if (!var || !m || !v || !grad || !sizes) return MUSA_KERNELS_EINVAL;
-  try {   // (host tables of the overlap check)
 #define MUSA_ADAM_GROUP(S, G)                                                              \
   return LaunchAdamGroup<S, G>(var, m, v, grad, sizes, count, lr_t, beta1, beta2, epsilon, \
                                use_nesterov, stream)
@@ -627,9 +633,6 @@ int LaunchApplyAdamGroupHostTable(int state_dtype, int grad_dtype, void* const* 
     if (state_dtype == MUSA_DT_BF16) MUSA_ADAM_GROUP(__nv_bfloat16, __nv_bfloat16);
   }
 #undef MUSA_ADAM_GROUP
-  } catch (const std::bad_alloc&) {
-    return MUSA_KERNELS_ETOOLARGE;
-  }
   return MUSA_KERNELS_EUNSUPPORTED;
 }
 

@@ -1,9 +1,13 @@
 """MusaAdam.apply_gradients takes any iterable of (grad, var) pairs.  One that makes
 its pairs on demand sees every update before the next pair is asked for; a list
 or tuple, whose pairs all exist before the call, shares launches."""
+import subprocess
+import sys
+
 import pytest
 import torch
 
+from conftest import ROOT
 from tensorflow_musa_extension_b200 import optimizers, raw_ops
 
 
@@ -88,3 +92,29 @@ def test_pairs_made_on_demand(kernel_lib, kind):
         raw_ops.MusaResourceApplyAdamMixed(var, m, v, 0.9, 0.999, 1e-3, 0.9, 0.999, 1e-7, grad)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+WITHOUT_MEMORY = """
+import ctypes, resource, sys
+sys.path.insert(0, %r)
+import tensorflow_musa_extension_b200 as package
+from tensorflow_musa_extension_b200 import _capi
+lib = _capi.bind(package.get_library())
+count = 1 << 22                     # the overlap check asks for 96 bytes of each
+null = (ctypes.c_void_p * count)()
+sizes = (ctypes.c_int64 * count)()  # empty variables: nothing to launch
+pages = int(open("/proc/self/statm").read().split()[0])
+limit = pages * resource.getpagesize() + (64 << 20)
+resource.setrlimit(resource.RLIMIT_AS, (limit, limit))
+sys.exit(lib.LaunchApplyAdamGroupHostTable(0, 0, null, null, null, null, sizes, count, 1e-3, 0.9,
+                                           0.999, 1e-7, False, None))
+"""
+
+
+def test_group_launcher_without_host_memory(kernel_lib):
+    """The check for variables that share memory needs a host table; without the
+    memory for it the update is still made, variable by variable."""
+    got = subprocess.run([sys.executable, "-c", WITHOUT_MEMORY % ROOT], capture_output=True,
+                         text=True)
+    # 35 and 100: the CUDA runtime's own answers on a machine without a device.
+    assert got.returncode in (0, 35, 100), (got.returncode, got.stderr)
