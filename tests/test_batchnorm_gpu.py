@@ -852,3 +852,55 @@ def test_retired_tuning_numbers_have_no_effect(kernel_lib):
     assert got[0] == want[0]
     for a, b in zip((t for out in got[1] for t in out), (t for out in want[1] for t in out)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("shape", [
+    # Planes of the channel-group kernels beyond four packs a thread (1025 .. 2816
+    # elements), several images a CTA: 5, 6, 7, 10 and 11 packs a thread, planes of
+    # single elements, of 4-byte, 8-byte and whole packs.
+    (16, 512, 33, 33), (16, 512, 34, 33), (16, 512, 40, 40), (24, 256, 47, 51), (12, 512, 44, 64),
+    # The longest plane, and the first that is too long; one image a CTA.
+    (2, 16, 44, 64), (2, 16, 1, 2817), (1, 8, 50, 50),
+    # One to four packs a thread, whole and not.
+    (40, 256, 14, 14), (9, 64, 18, 18), (24, 128, 24, 24), (33, 64, 28, 28), (17, 64, 32, 32),
+    (33, 64, 29, 31), (5, 2048, 7, 14)])
+def test_channel_major_chain(kernel_lib, dtype, shape):
+    """Channel-major planes through the chain of kernels (group and plane kernels as
+    the rule has it for each pass), inference too, against the oracle."""
+    c = shape[1]
+    x, s, o, dy = bn_inputs(500 + c + shape[3], shape, dtype, 1.0, 3.0, channel_axis=1)
+    want = np_ref.fused_batch_norm(x, s, o, epsilon=EPS, data_format="NCHW")
+    wg = np_ref.fused_batch_norm_grad(dy, x, s, want[3], want[4], EPS, "NCHW")
+    terms = _rms(dy) * float(np.max(s / np.sqrt(want[4] + EPS)))
+    with tuned(kernel_lib, (24, -1)):
+        fwd, grad, _ = launch_ops(kernel_lib, x, s, o, dy, "NCHW")
+    check_forward(fwd, want, dtype)
+    check_grad(grad, wg, dtype, dx_scale=terms)
+    infer = raw_ops.FusedBatchNormV3(to_torch(x), to_torch(s), to_torch(o), fwd.reserve_space_1,
+                                     fwd.reserve_space_2, epsilon=EPS, data_format="NCHW",
+                                     is_training=False)
+    rt = _rt(dtype)
+    assert_close(to_numpy(infer.y), want[0], rt, rt * _rms(want[0]), "inference")
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("rows,parts", [(4099, 1), (4096, 4), (4099, 4)])
+@pytest.mark.parametrize("fused", [False, True, "moments"])
+@pytest.mark.parametrize("c", [37, 101])
+def test_split_api_with_odd_channel_counts(kernel_lib, dtype, rows, parts, fused, c):
+    """The cross-replica forms where several rows make one whole-pack row: the rows
+    left over (4099 = 4096 + 3) are added by the finalize kernel of every form; row
+    blocks that start inside a pack take the element kernels."""
+    x, s, o, dy = bn_inputs(18 + c, (rows, c), dtype, 0.0, 1.0)
+    got = _split_forward_and_grad(kernel_lib, to_torch(x), to_torch(dy), to_torch(s),
+                                  to_torch(o), parts, fused)
+    want = np_ref.fused_batch_norm(x, s, o, epsilon=EPS)
+    wg = np_ref.fused_batch_norm_grad(dy, x, s, want[3], want[4], EPS)
+    rt = _rt(dtype)
+    assert_close(to_numpy(got[0]), want[0], rt, rt * _rms(want[0]), "y")
+    for i in range(1, 5):
+        assert_close(to_numpy(got[i]), want[i], 1e-4, 1e-4 * max(_rms(want[i]), 1e-6))
+    assert_close(to_numpy(got[5]), wg[0], rt, rt * _rms(wg[0]), "dx")
+    assert_close(to_numpy(got[6]), wg[1], 1e-4, 1e-4 * _rms(wg[1]), "dscale")
+    assert_close(to_numpy(got[7]), wg[2], 1e-4, 1e-4 * _rms(wg[2]), "doffset")

@@ -113,7 +113,7 @@ def test_single_replica_handle_round_trip(kernel_lib):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,c", [(4096, 64), (777, 520), (5000, 2048)])
+@pytest.mark.parametrize("rows,c", [(4096, 64), (777, 520), (5000, 2048), (779, 37), (4099, 1001)])
 def test_finalize_kernel_runs_the_exchange_itself(kernel_lib, dtype, rows, c):
     """LaunchBnStatsMomentsExchange / LaunchBnGradStatsSumsExchange with a
     one-replica handle return what the two-step forms return, call after call

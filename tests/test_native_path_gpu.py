@@ -1,6 +1,8 @@
 """The native host path of the ops against their general Python path: the same
 bits for every call that the native path takes, the same answers and errors for
 those that it leaves."""
+import threading
+
 import pytest
 import torch
 
@@ -124,3 +126,70 @@ def test_adam_step(monkeypatch, kernel_lib, state, grad):
         opt.apply_gradients(pairs)
         return tuple(t for v in vs for t in (v, opt.get_slot(v, "m"), opt.get_slot(v, "v")))
     _same(*_both(monkeypatch, step))
+
+
+def _train_step(x, dy, s, o):
+    e = torch.empty(0, device="cuda")
+    f = raw_ops.FusedBatchNormV3(x, s, o, e, e, 1e-3)
+    g = raw_ops.FusedBatchNormGradV3(dy, x, s, f.reserve_space_1, f.reserve_space_2, None, 1e-3)
+    b = s.to(x.dtype)
+    return (*f, *g, raw_ops.MusaLayerNorm(x, b, b), *raw_ops.MusaLayerNormGrad(dy, x, b, b),
+            raw_ops.MusaBiasAddRelu(x, b))
+
+
+def _step_inputs(seed, c):
+    # The first size fits the one-kernel form, the second takes the chain and its scratch.
+    rows = 700 if c == 48 else 70000
+    return (_rand((rows, c), BF16, seed), _rand((rows, c), BF16, seed + 1),
+            _rand((c,), F32, seed + 2), _rand((c,), F32, seed + 3))
+
+
+@pytest.mark.parametrize("c", [48, 256])
+@pytest.mark.parametrize("own_stream", [False, True])
+def test_several_threads(kernel_lib, c, own_stream):
+    """Calls of four threads at once, on one stream or on one each: the bits of
+    the same calls made one after the other (scratch is private to a call)."""
+    inputs = [_step_inputs(10 * i, c) for i in range(4)]
+    want = [_train_step(*a) for a in inputs]
+    torch.cuda.synchronize()
+    got, failed = [None] * 4, []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream() if own_stream
+                                   else torch.cuda.default_stream()):
+                for _ in range(20):
+                    got[i] = _train_step(*inputs[i])
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:   # reported by the assertion below
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+    for a, b in zip(got, want):
+        for u, v in zip(a, b):
+            assert torch.equal(u, v)
+
+
+@pytest.mark.parametrize("c", [48, 256])
+def test_graph_capture(kernel_lib, c):
+    """A captured step (outputs and scratch from the graph's pool) replayed on new
+    inputs: the bits of the eager calls."""
+    buffers, other = _step_inputs(3, c), _step_inputs(50, c)
+    _train_step(*buffers)      # per-device set-up
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = _train_step(*buffers)
+    for values in (other, _step_inputs(90, c)):
+        for t, v in zip(buffers, values):
+            t.copy_(v)
+        graph.replay()
+        torch.cuda.synchronize()
+        for u, v in zip(out, _train_step(*values)):
+            assert torch.equal(u, v)
+    del graph

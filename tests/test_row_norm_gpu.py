@@ -276,14 +276,16 @@ def test_rows_that_start_inside_a_pack(kernel_lib, rows, n, dtype):
     """Row lengths that are not whole packs: rows start anywhere inside a
     128-bit pack, the first and last pack hold elements of the neighbouring
     rows.  All four ops against the element form (the same values off a 16-byte
-    boundary), with huge values beside every row's ends: a neighbour that leaked
-    into a row would show."""
+    boundary), every third row with huge values at its ends, next to the ends of the
+    rows beside it: a neighbour that leaked into a row would show.  The column sums
+    against 64-bit sums of the same inputs."""
     rng = np.random.default_rng(rows + n)
     d = {"float32": torch.float32, "float16": torch.float16, "bfloat16": torch.bfloat16}[dtype]
     x = rng.standard_normal((rows, n)) + 0.5
     dy = rng.standard_normal((rows, n)) * 0.1
-    x[::3] *= 100.0       # neighbours of another scale
-    dy[::3] *= 100.0
+    ends = np.unique(np.r_[0:min(8, n), max(0, n - 8):n])
+    for t in (x, dy):     # the elements that can share a pack with the next row's
+        t[::3, ends] *= 100.0
     x, dy = (torch.from_numpy(t).to(d).cuda() for t in (x, dy))
     g, b = (torch.from_numpy(rng.standard_normal(n)).to(d).cuda() for _ in range(2))
 
@@ -299,14 +301,46 @@ def test_rows_that_start_inside_a_pack(kernel_lib, rows, n, dtype):
         return out
 
     got, again, want = run(x, dy), run(x, dy), run(unaligned(x), unaligned(dy))
-    # fp32 sums in another order (a few hundred ulps of the largest term for the
-    # column sums), one rounding of T in the 16-bit results.
+    # fp32 sums in another order, one rounding of T in the 16-bit results.
     rt = 1e-5 if d == torch.float32 else 2.0 ** (-9 if d == torch.float16 else -6)
+    # dgamma and dbeta in 64 bits from the same inputs: one rounding of T, and 1e-5
+    # of the terms' magnitudes for fp32 terms whose x_hat is off by up to a few
+    # 1e-6 (an ulp of the row's largest value).
+    x64, dy64 = x.double(), dy.double()
+    mean = x64.mean(-1, keepdim=True)
+    xhat = (x64 - mean) / ((x64 - mean).square().mean(-1, keepdim=True) + 1e-5).sqrt()
+    column_sums = {2: dy64 * xhat, 3: dy64}
+    ulp = {torch.float32: 2.0 ** -23, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[d]
     for i, (a, same, ref) in enumerate(zip(got, again, want)):
         assert torch.equal(a, same), i
         a, ref = a.double(), ref.double()
-        if i in (2, 3):    # dgamma, dbeta: sums over rows of very different scale
-            scale = dy.double().abs().max() * max(rows, 1) ** 0.5 * (4 if i == 2 else 1)
-        else:
-            scale = ref.abs().amax(-1, keepdim=True).clamp_min(1e-12)
+        if i in column_sums:
+            terms = column_sums[i]
+            bound = ulp * terms.sum(0).abs() + 1e-5 * (terms.abs() + dy64.abs()).sum(0)
+            assert bool(((a - terms.sum(0)).abs() <= bound).all()), i
+            continue
+        scale = ref.abs().amax(-1, keepdim=True).clamp_min(1e-12)
         assert bool(((a - ref).abs() <= rt * ref.abs() + rt * scale).all()), i
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("n", [8, 24, 1000, 1024, 3072, 5120, 6144, 8192])
+@pytest.mark.parametrize("mean", [0.0, 1000.0])
+def test_gradient_sums_of_a_row(kernel_lib, n, dtype, mean):
+    """The gradient takes its sums over dy * gamma beside the second sum over x (in
+    all layouts but one: 16-bit rows of 5120) and corrects them by what the
+    first mean was off: rows of a large mean, where that correction counts."""
+    rng = np.random.default_rng(n)
+    dt = np_dtype(dtype)
+    x = (rng.standard_normal((40, n)) * (8 if dtype == "bfloat16" else 1) + mean).astype(dt)
+    dy = rng.standard_normal((40, n)).astype(dt)
+    g = rng.uniform(0.5, 1.5, n).astype(dt)
+    dx, dgamma, dbeta = raw_ops.MusaLayerNormGrad(*(to_torch(a) for a in (dy, x, g, g)))
+    want = np_ref.layer_norm_grad(dy, x, g)
+    # x minus the first mean is exact (values of one binade) and the correction takes
+    # out the rest: fp32 terms of size 1, 40 of them in a column; bf16 one rounding
+    # of each side.
+    rt = 2.0 ** -7 if dtype == "bfloat16" else 1e-5
+    assert_close(to_numpy(dx), want[0], rt, 2e-5, "dx")
+    assert_close(to_numpy(dgamma), want[1], rt, 2e-4, "dgamma")
+    assert_close(to_numpy(dbeta), want[2], rt, 1e-4, "dbeta")
