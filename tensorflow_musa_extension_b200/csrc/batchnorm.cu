@@ -864,8 +864,8 @@ __global__ void __launch_bounds__(kThreads)
 // a thread's pack always covers the same one or two channels: the first
 // `before` elements belong to channel lo, the rest to lo + 1.
 // Packs of a run per thread: inner <= 11 * 256, whose per-pack sums (16 bytes
-// each) fit the shared memory of a plain launch.  bf16 [64,64,33,33], single
-// elements -> this form: forward 26.6 -> 20.8 us, gradient 32.8 -> 20.5.
+// each) fit the shared memory of a plain launch.  bf16
+// [128,64,33,33], single elements -> this form: gradient 41.5 -> 23.9 us.
 constexpr int kGroupSlots = 11;
 constexpr int kGroupUnroll = 4;  // values of n in flight per thread
 
@@ -1826,7 +1826,7 @@ __global__ void __launch_bounds__(kThreads, GroupCtas(kMode, sizeof(T)))
 
 // ------------------------------------------------- one kernel per op ----
 //
-// Layers that fit the shared memory of the SMs (up to about 25 MB of inputs)
+// Layers whose inputs are below 16 MiB and fit the shared memory of the clusters
 // need no second pass over memory and no kernel boundary: a CLUSTER of up to
 // 16 CTAs owns a block of `tx` channel packs and all rows, each CTA keeps its
 // row range of x (and dy) in shared memory, the CTAs' sums meet through
@@ -1839,9 +1839,10 @@ __global__ void __launch_bounds__(kThreads, GroupCtas(kMode, sizeof(T)))
 // gradient 6.1 -> 4.4; bf16 [1568,2048] 8.6 -> 6.0 and 9.5 -> 6.7; bf16
 // [6272,1024] forward 11.7 -> 7.9; channel-major bf16 [64,512,7,7] 10.8 -> 6.6
 // and 12.3 -> 7.0, [64,512,14,14] forward 18.4 -> 8.9, fp32 [8,64,14,14]
-// 8.3 -> 4.0.  The limit on the inputs is where the form stops fitting: 64 to
-// 128 CTAs hold 13 to 25 MB, and near that the two are level (fp32
-// [25088,128], 12.8 MB: 10.8 against 9.4-10.2).
+// 8.3 -> 4.0.  The limit of 16 MiB is not where the form stops fitting - 64 to
+// 128 CTAs hold 13 to 25 MB, fp32 [100352,64] would fit - but where it was
+// measured: near it the gain is small (fp32 [25088,128], 12.8 MB: 9.7 -> 9.2)
+// and larger inputs keep the chain.
 constexpr int kOnChipThreads = 512;
 constexpr int kOnChipWarps = kOnChipThreads / 32;
 constexpr int kOnChipMaxTx = 8;

@@ -9,6 +9,9 @@ the same hyper-parameters, slot names ("m", "v") and dispatch:
   fp32 variable + grad in {fp32, fp16, bf16}  -> MusaResourceApplyAdamMixed
   fp16/bf16 variable with a same-dtype grad    -> ResourceApplyAdam (16-bit
                                                   state, fp32 arithmetic)
+                (device tensors in the form of the kernels take these ops' update
+                 through the group launcher, LaunchApplyAdamGroupHostTable, and
+                 get the same bits; the rest goes through the ops themselves)
   amsgrad=True                                 -> rejected (the reference falls
                                                   back to stock Keras there)
 """
