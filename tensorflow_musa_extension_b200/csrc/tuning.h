@@ -35,7 +35,8 @@ enum TuningKey {
   kTuneBnOnChipTx = 24,     // channel packs per column block (channel-major: channels per group) of the
                             // one-kernel form; 0: by rule, -1: off (the chain of kernels at every size)
   kTuneBnOnChipCluster = 25,  // CTAs per cluster of the one-kernel form; 0: by rule
-  kTuneCount = 26
+  kTuneBnGrid = 26,         // grid-wide one-kernel form of large layers: 0 by rule, 1 at every size, -1 off
+  kTuneCount = 27
 };
 
 int GetTuning(int key);
