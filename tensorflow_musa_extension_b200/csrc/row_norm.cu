@@ -43,7 +43,8 @@ struct RowArgs {
   void* stat_t;          // RMSNorm forward: inv_rms, type T
   float* mean_out;       // LayerNorm forward, optional fp32 [rows]
   float* inv_std_out;    // LayerNorm forward, optional fp32 [rows]
-  float* partial;        // LayerNorm gradient: [ctas][2][row_size]
+  float* partial;        // LayerNorm gradient: [ctas][2][row_size], columns in slab order
+                         // where rows are whole packs
   int64_t rows;
   int row_size;
   float epsilon;
@@ -673,7 +674,7 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
   if constexpr (kOp == kOpLnGrad) {
     // One partial row (dgamma part, dbeta part) per CTA: the slabs of the row
     // lanes added in lane order.  Column c of half s sits at
-    // ((s * kQuads + (c % kVec) / 4) * packs + c / kVec) * 4 + c % 4.
+    // ((s * kQuads + (c % kVec) / 4) * packs + c / kVec) * 4 + c % 4 of a slab.
     // The ring is free once every thread has left the loop: the slabs of the
     // row lanes go there.
     AsyncWait<0>();
@@ -701,16 +702,31 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
       }
     }
     __syncthreads();
+    // Whole packs: in the slabs' own order, four columns at a time (column by column, with
+    // the divisions that takes, this tail was 1.5 us of the call; LnGradFinalizeKernel
+    // knows the order).
     float* out = a.partial + static_cast<int64_t>(blockIdx.x) * 2 * a.row_size;
-    for (int c = threadIdx.x; c < 2 * a.row_size; c += kThreads) {
-      const int half = c / a.row_size;
-      const int col = c - half * a.row_size;
-      const int e = col % kVec;
-      const int at =
-          kShifted ? c : ((half * kQuads + e / 4) * packs + col / kVec) * 4 + (e & 3);
-      float s = slab[at];
-      for (int l = 1; l < kRows; ++l) s += slab[static_cast<size_t>(l) * 2 * a.row_size + at];
-      out[c] = s;
+    if constexpr (kShifted) {
+      for (int c = threadIdx.x; c < 2 * a.row_size; c += kThreads) {
+        float s = slab[c];
+        for (int l = 1; l < kRows; ++l) s += slab[static_cast<size_t>(l) * 2 * a.row_size + c];
+        out[c] = s;
+      }
+    } else {
+      const int quads = 2 * kQuads * packs;
+      const float4* const from = reinterpret_cast<const float4*>(slab);
+      for (int q = threadIdx.x; q < quads; q += kThreads) {
+        float4 s = from[q];
+#pragma unroll
+        for (int l = 1; l < kRows; ++l) {
+          const float4 v = from[l * quads + q];
+          s.x += v.x;
+          s.y += v.y;
+          s.z += v.z;
+          s.w += v.w;
+        }
+        reinterpret_cast<float4*>(out)[q] = s;
+      }
     }
   }
 }
@@ -813,42 +829,83 @@ __global__ void __launch_bounds__(256) RowNormLoopKernel(RowArgs a) {
   }
 }
 
-// dgamma / dbeta = sum over the CTAs' partial rows, fixed order, fp64.
-template <typename T>
+// dgamma / dbeta = sum over the CTAs' partial rows, fixed order.  A CTA adds 16
+// columns; kQuads: the rows are in the order of RowNormKernel's slabs and come four
+// columns a load.  Bound by latency: one memory round trip with all loads of a
+// thread in flight, a tree over those five (single columns: ten) rows in fp32 and
+// fp64 from there on.  (Every partial widened by itself is 4096 conversions to fp64
+// per SM at 16 a cycle: bf16 [16384,1024], a call of 20.4 us without this kernel,
+// takes 22.8 us that way and 22.3 so; two loads at a time, 8 columns a CTA and a
+// serial last step took 23.5.  [1024,1024]: 7.3, 6.8 and 8.3.)
+template <typename T, bool kQuads>
 __global__ void __launch_bounds__(256)
     LnGradFinalizeKernel(const float* __restrict__ partial, int n_partial,
                          int row_size, T* __restrict__ dgamma,
                          T* __restrict__ dbeta) {
-  constexpr int kCh = 8, kLanes = 32;
-  __shared__ double red[256];
-  const int tc = threadIdx.x % kCh;
-  const int tl = threadIdx.x / kCh;
-  const int c = blockIdx.x * kCh + tc;  // column of the [2 * row_size] row
+  constexpr int kColumns = 16, kWarps = 8, kLoads = kQuads ? 5 : 10;
+  constexpr int kWide = kQuads ? 4 : 1;            // columns per load
+  constexpr int kUnits = kColumns / kWide;         // loads per partial row and CTA
+  constexpr int kLanes = kWarps * 32 / kUnits;     // partial rows at once
+  using P = Pack<float, kWide>;
+  __shared__ double red[kWarps][kColumns];
+  const int tid = threadIdx.x;
+  const int64_t unit = static_cast<int64_t>(blockIdx.x) * kUnits + tid % kUnits;
+  // The column that thread tid < 16 writes: of [dgamma, dbeta].
+  const int64_t at = static_cast<int64_t>(blockIdx.x) * kColumns + tid;
+  const bool writer = tid < kColumns && at < 2 * static_cast<int64_t>(row_size);
+  int column = static_cast<int>(at % row_size);
+  const bool beta = at >= row_size;
+  if constexpr (kQuads) {
+    constexpr int kVec = VecWidth<T>::value;
+    const int packs = row_size / kVec;
+    const int quad = column / 4;   // of its half: [kVec / 4][packs]
+    column = quad % packs * kVec + quad / packs * 4 + column % 4;
+  }
   GridDepWait();
   GridDepLaunch();
-  double s0 = 0.0, s1 = 0.0;
-  if (c < 2 * row_size) {
-    int p = tl;
-    for (; p + kLanes < n_partial; p += 2 * kLanes) {
-      const float v0 = partial[static_cast<int64_t>(p) * 2 * row_size + c];
-      const float v1 = partial[static_cast<int64_t>(p + kLanes) * 2 * row_size + c];
-      s0 += v0;
-      s1 += v1;
-    }
-    for (; p < n_partial; p += kLanes) {
-      s0 += partial[static_cast<int64_t>(p) * 2 * row_size + c];
+  double s[kWide];
+#pragma unroll
+  for (int w = 0; w < kWide; ++w) s[w] = 0.0;
+  if (unit * kWide < 2 * static_cast<int64_t>(row_size)) {
+    const float* const from = partial + unit * kWide;
+    for (int p = tid / kUnits; p < n_partial; p += kLoads * kLanes) {
+      P v[kLoads];
+#pragma unroll
+      for (int i = 0; i < kLoads; ++i) {
+        const int r = p + i * kLanes;
+#pragma unroll
+        for (int w = 0; w < kWide; ++w) v[i].v[w] = 0.0f;
+        if (r < n_partial) {
+          v[i] = *reinterpret_cast<const P*>(from + static_cast<int64_t>(r) * 2 * row_size);
+        }
+      }
+#pragma unroll
+      for (int m = 1; m < kLoads; m *= 2) {
+#pragma unroll
+        for (int i = 0; i + m < kLoads; i += 2 * m) {
+#pragma unroll
+          for (int w = 0; w < kWide; ++w) v[i].v[w] += v[i + m].v[w];
+        }
+      }
+#pragma unroll
+      for (int w = 0; w < kWide; ++w) s[w] += static_cast<double>(v[0].v[w]);
     }
   }
-  double s = s0 + s1;
-  red[threadIdx.x] = s;
+#pragma unroll
+  for (int m = 16; m >= kUnits; m >>= 1) {
+#pragma unroll
+    for (int w = 0; w < kWide; ++w) s[w] += __shfl_xor_sync(0xffffffffu, s[w], m);
+  }
+  if ((tid & 31) < kUnits) {
+#pragma unroll
+    for (int w = 0; w < kWide; ++w) red[tid >> 5][(tid & 31) * kWide + w] = s[w];
+  }
   __syncthreads();
-  if (tl == 0 && c < 2 * row_size) {
-    for (int l = 1; l < kLanes; ++l) s += red[l * kCh + tc];
-    if (c < row_size) {
-      dgamma[c] = FromF32<T>(static_cast<float>(s));
-    } else {
-      dbeta[c - row_size] = FromF32<T>(static_cast<float>(s));
-    }
+  if (writer) {
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) sum += red[w][tid];
+    (beta ? dbeta : dgamma)[column] = FromF32<T>(static_cast<float>(sum));
   }
 }
 
@@ -856,6 +913,12 @@ __global__ void __launch_bounds__(256)
 
 constexpr int kMaxCtasPerSm = 8;
 constexpr int kMaxGradCtasPerSm = 4;  // bounds the partial rows of the gradient
+
+// Partial rows that a launch leaves (LayerNorm gradient), and whether in slab order.
+struct GradRows {
+  int count;
+  bool quads;
+};
 
 inline int MaxGradCtas() { return SmCount() * kMaxGradCtasPerSm; }
 
@@ -874,7 +937,7 @@ size_t RowSmemBytes(int group, int elem_bytes, int threads, int max_packs, int r
 }
 
 template <typename T, int kGroup, int kMaxPacks, int kOp, int kLayout>
-int LaunchGroupAs(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
+int LaunchGroupAs(const RowArgs& a, GradRows* rows_out, cudaStream_t stream) {
   constexpr int kThreads = RowThreads(kGroup, kOp);
   constexpr int kRows = kThreads / kGroup;
   auto kernel = RowNormKernel<T, kGroup, kMaxPacks, kOp, kLayout>;
@@ -926,6 +989,22 @@ int LaunchGroupAs(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
   constexpr int kCap = kOp == kOpLnGrad ? kMaxGradCtasPerSm : kMaxCtasPerSm;
   if (per_sm > kCap) per_sm = kCap;
   const int64_t need = CeilDiv(a.rows, kRows);
+  const int tuned = GetTuning(kTuneRowCtas);
+  if (tuned > 0) {
+    if (per_sm > tuned) per_sm = tuned;
+  } else if (kOp == kOpLnGrad) {
+    // Every CTA leaves a partial row for the second kernel, so fewer are better where
+    // the others do not wait for them: fp32 needs no more than 96 KB of ring on an SM
+    // (four CTAs against two: [16384,512] 22.3 -> 19.6 us, [16384,2048] 75 -> 65), and a
+    // few row blocks per CTA no more than two (bf16 [4096,512] 11.3 -> 8.3, [16384,128]
+    // 9.7 -> 7.8).
+    constexpr int kRing = RowStages(kOp, kGroup, sizeof(T)) * RowPipe<kOp>::kInputs * kMaxPacks *
+                          kThreads * 16;
+    constexpr int kFit = 96 * 1024 / kRing;
+    constexpr int kMost = kFit > 2 ? kFit : 2;
+    if (sizeof(T) == 4 && per_sm > kMost) per_sm = kMost;
+    if (need < 8 * static_cast<int64_t>(SmCount()) && per_sm > 2) per_sm = 2;
+  }
   int64_t grid = static_cast<int64_t>(SmCount()) * per_sm;
   if (kLayout == kRowsShifted && grid < need) {
     // Consecutive rows of a thread a multiple of the pack width apart.
@@ -933,15 +1012,15 @@ int LaunchGroupAs(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
     grid -= grid % kStep;
   }
   if (grid > need) grid = need;
-  *ctas_out = static_cast<int>(grid);
+  *rows_out = GradRows{static_cast<int>(grid), kLayout != kRowsShifted};
   return static_cast<int>(LaunchChained(true, kernel, dim3(static_cast<unsigned>(grid)),
                                         dim3(kThreads), smem, stream, a));
 }
 
 template <typename T, int kGroup, int kMaxPacks, int kOp>
-int LaunchGroup(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
+int LaunchGroup(const RowArgs& a, GradRows* rows_out, cudaStream_t stream) {
   if (a.row_size % VecWidth<T>::value != 0) {
-    return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, kRowsShifted>(a, ctas_out, stream);
+    return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, kRowsShifted>(a, rows_out, stream);
   }
   // Rows that fill the layout need no per-pack presence checks.  Only the
   // LayerNorm gradient gains from the specialised form (fp32 rows of 1024:
@@ -949,18 +1028,18 @@ int LaunchGroup(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
   // spills under their register cap, slower.
   if constexpr (kOp == kOpLnGrad) {
     if (a.row_size / VecWidth<T>::value == kGroup * kMaxPacks) {
-      return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, kRowsFull>(a, ctas_out, stream);
+      return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, kRowsFull>(a, rows_out, stream);
     }
   }
-  return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, kRowsPacked>(a, ctas_out, stream);
+  return LaunchGroupAs<T, kGroup, kMaxPacks, kOp, kRowsPacked>(a, rows_out, stream);
 }
 
 template <typename T, int kOp>
-int LaunchLoop(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
+int LaunchLoop(const RowArgs& a, GradRows* rows_out, cudaStream_t stream) {
   int64_t grid = static_cast<int64_t>(SmCount()) *
                  (kOp == kOpLnGrad ? kMaxGradCtasPerSm : kMaxCtasPerSm);
   if (grid > a.rows) grid = a.rows;
-  *ctas_out = static_cast<int>(grid);
+  *rows_out = GradRows{static_cast<int>(grid), false};
   return static_cast<int>(LaunchChained(true, RowNormLoopKernel<T, kOp>,
                                         dim3(static_cast<unsigned>(grid)), dim3(256), 0,
                                         stream, a));
@@ -974,7 +1053,7 @@ inline int RowPacks(int row_size) {
 }
 
 template <typename T, int kOp, int kMaxPacks>
-int DispatchPacks(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
+int DispatchPacks(const RowArgs& a, GradRows* rows_out, cudaStream_t stream) {
   const int packs = RowPacks<T>(a.row_size);
   const bool shifted = a.row_size % VecWidth<T>::value != 0;
   const auto fits = [&](int group) {
@@ -983,22 +1062,22 @@ int DispatchPacks(const RowArgs& a, int* ctas_out, cudaStream_t stream) {
     return RowSmemBytes<kOp>(group, sizeof(T), threads, kMaxPacks, a.row_size, shifted) <=
            200 * 1024;
   };
-  if (fits(8)) return LaunchGroup<T, 8, kMaxPacks, kOp>(a, ctas_out, stream);
-  if (fits(32)) return LaunchGroup<T, 32, kMaxPacks, kOp>(a, ctas_out, stream);
+  if (fits(8)) return LaunchGroup<T, 8, kMaxPacks, kOp>(a, rows_out, stream);
+  if (fits(32)) return LaunchGroup<T, 32, kMaxPacks, kOp>(a, rows_out, stream);
   // Two-warp groups: measured better than a half-filled 128-thread group for
   // 16-bit rows (bf16 rows of 2048: LayerNorm 5.6 against 3.8 TB/s), worse for
   // fp32 rows of the same byte length.
   if constexpr (kMaxPacks == 2 || kMaxPacks == 3 || sizeof(T) == 2) {
-    if (fits(64)) return LaunchGroup<T, 64, kMaxPacks, kOp>(a, ctas_out, stream);
+    if (fits(64)) return LaunchGroup<T, 64, kMaxPacks, kOp>(a, rows_out, stream);
   }
-  if (fits(128)) return LaunchGroup<T, 128, kMaxPacks, kOp>(a, ctas_out, stream);
-  if (fits(256)) return LaunchGroup<T, 256, kMaxPacks, kOp>(a, ctas_out, stream);
-  if (fits(512)) return LaunchGroup<T, 512, kMaxPacks, kOp>(a, ctas_out, stream);
+  if (fits(128)) return LaunchGroup<T, 128, kMaxPacks, kOp>(a, rows_out, stream);
+  if (fits(256)) return LaunchGroup<T, 256, kMaxPacks, kOp>(a, rows_out, stream);
+  if (fits(512)) return LaunchGroup<T, 512, kMaxPacks, kOp>(a, rows_out, stream);
   return -1;  // no register layout holds this row
 }
 
 template <typename T, int kOp>
-int Dispatch(const RowArgs& a, bool aligned, int* ctas_out, cudaStream_t stream) {
+int Dispatch(const RowArgs& a, bool aligned, GradRows* rows_out, cudaStream_t stream) {
   // Rows that are not whole packs take the same layouts (kRowsShifted).  Us
   // against the element form, LayerNorm forward / gradient, RMSNorm forward /
   // gradient: bf16 [65536,1001] 241, 626, 144, 159 -> 78, 146, 84, 81; fp32
@@ -1039,13 +1118,13 @@ int Dispatch(const RowArgs& a, bool aligned, int* ctas_out, cudaStream_t stream)
       }
     }
     int rc = -1;
-    if (want == 1) rc = DispatchPacks<T, kOp, 1>(a, ctas_out, stream);
-    if (want == 2) rc = DispatchPacks<T, kOp, 2>(a, ctas_out, stream);
-    if (want == 3) rc = DispatchPacks<T, kOp, 3>(a, ctas_out, stream);
-    if (rc == -1) rc = DispatchPacks<T, kOp, 4>(a, ctas_out, stream);
+    if (want == 1) rc = DispatchPacks<T, kOp, 1>(a, rows_out, stream);
+    if (want == 2) rc = DispatchPacks<T, kOp, 2>(a, rows_out, stream);
+    if (want == 3) rc = DispatchPacks<T, kOp, 3>(a, rows_out, stream);
+    if (rc == -1) rc = DispatchPacks<T, kOp, 4>(a, rows_out, stream);
     if (rc != -1) return rc;
   }
-  return LaunchLoop<T, kOp>(a, ctas_out, stream);
+  return LaunchLoop<T, kOp>(a, rows_out, stream);
 }
 
 inline bool BadRows(int64_t rows, int64_t row_size) {
@@ -1072,9 +1151,9 @@ int LayerNormFwd(const void* x, const void* gamma, const void* beta, void* y,
   a.rows = rows;
   a.row_size = static_cast<int>(row_size);
   a.epsilon = epsilon;
-  int ctas = 0;
+  GradRows partial = {};
   const bool aligned = Aligned16(x) && Aligned16(gamma) && Aligned16(beta) && Aligned16(y);
-  const int rc = Dispatch<T, kOpLnFwd>(a, aligned, &ctas, stream);
+  const int rc = Dispatch<T, kOpLnFwd>(a, aligned, &partial, stream);
   return rc != 0 ? rc : static_cast<int>(cudaGetLastError());
 }
 
@@ -1109,14 +1188,14 @@ int LayerNormGrad(const void* dy, const void* x, const void* gamma, void* dx,
   a.rows = rows;
   a.row_size = static_cast<int>(row_size);
   a.epsilon = epsilon;
-  int ctas = 0;
+  GradRows partial = {};
   const bool aligned = Aligned16(x) && Aligned16(dy) && Aligned16(gamma) && Aligned16(dx);
-  int rc = Dispatch<T, kOpLnGrad>(a, aligned, &ctas, stream);
+  int rc = Dispatch<T, kOpLnGrad>(a, aligned, &partial, stream);
   if (rc != 0) return rc;
   rc = static_cast<int>(LaunchChained(
-      true, LnGradFinalizeKernel<T>,
-      dim3(static_cast<unsigned>(CeilDiv(2 * row_size, 8))), dim3(256), 0, stream,
-      static_cast<const float*>(a.partial), ctas, a.row_size, static_cast<T*>(dgamma),
+      true, partial.quads ? LnGradFinalizeKernel<T, true> : LnGradFinalizeKernel<T, false>,
+      dim3(static_cast<unsigned>(CeilDiv(2 * row_size, 16))), dim3(256), 0, stream,
+      static_cast<const float*>(a.partial), partial.count, a.row_size, static_cast<T*>(dgamma),
       static_cast<T*>(dbeta)));
   return rc != 0 ? rc : static_cast<int>(cudaGetLastError());
 }
@@ -1136,10 +1215,10 @@ void RmsNormFwd(const void* x, const void* gamma, void* y, void* normalized,
   a.rows = rows;
   a.row_size = static_cast<int>(row_size);
   a.epsilon = epsilon;
-  int ctas = 0;
+  GradRows partial = {};
   const bool aligned =
       Aligned16(x) && Aligned16(gamma) && Aligned16(y) && Aligned16(normalized);
-  Dispatch<T, kOpRmsFwd>(a, aligned, &ctas, stream);
+  Dispatch<T, kOpRmsFwd>(a, aligned, &partial, stream);
 }
 
 template <typename T>
@@ -1157,9 +1236,9 @@ void RmsNormGradDx(const void* x, const void* inv_rms, const void* gamma,
   a.out = dx;
   a.rows = rows;
   a.row_size = static_cast<int>(row_size);
-  int ctas = 0;
+  GradRows partial = {};
   const bool aligned = Aligned16(x) && Aligned16(gamma) && Aligned16(dy) && Aligned16(dx);
-  Dispatch<T, kOpRmsGrad>(a, aligned, &ctas, stream);
+  Dispatch<T, kOpRmsGrad>(a, aligned, &partial, stream);
 }
 
 }  // namespace

@@ -36,7 +36,8 @@ enum TuningKey {
                             // one-kernel form; 0: by rule, -1: off (the chain of kernels at every size)
   kTuneBnOnChipCluster = 25,  // CTAs per cluster of the one-kernel form; 0: by rule
   kTuneBnGrid = 26,         // grid-wide one-kernel form of large layers: 0 by rule, 1 at every size, -1 off
-  kTuneCount = 27
+  kTuneRowCtas = 27,        // most CTAs per SM of the row kernels; 0: by rule
+  kTuneCount = 28
 };
 
 int GetTuning(int key);
