@@ -1094,11 +1094,13 @@ int Dispatch(const RowArgs& a, bool aligned, GradRows* rows_out, cudaStream_t st
     // packs (768, 1536, 3072 ... bf16 columns) take three: the layout is then
     // full again, with three quarters of the registers and of the ring (bf16
     // LayerNorm gradient of 768 columns: 5.6 against 4.5 TB/s).  Rows that
-    // fill less than half of the four-pack layout of their group take two
-    // (fp32 rows of 768: LayerNorm 5.5 against 4.6 TB/s); the LayerNorm
-    // gradient, whose column sums live in registers, also at exactly half
-    // (fp32 rows of 1024: 5.6 against 5.1 - the other ops measured the same
-    // or slower there).  Tuning values 1 .. 4 force a layout.
+    // fill no more than half of the four-pack layout of their group take two
+    // (fp32 rows of 768: LayerNorm 5.5 against 4.6 TB/s; bf16 [65536,512], exactly
+    // half: LayerNorm 33.5 -> 25.9 us, RMSNorm gradient 38.9 -> 34.0; bf16 rows of 500 and
+    // fp32 rows of 250 gain 10 to 28 %) - but the forward LayerNorm of large fp32
+    // tensors of whole packs, at exactly half, wants the deeper ring ([65536,1024] 91 us
+    // with four, 98 with two; [16384,1024] 25.7 and 23.2).  Tuning values 1 .. 4
+    // force a layout.
     int want = GetTuning(kTuneRowNormPacks);
     if (want < 1 || want > 4) {
       want = 4;
@@ -1111,7 +1113,10 @@ int Dispatch(const RowArgs& a, bool aligned, GradRows* rows_out, cudaStream_t st
           break;
         }
       }
-      if (packs < 2 * group || (packs == 2 * group && kOp == kOpLnGrad)) {
+      const bool deep = sizeof(T) == 4 && kOp == kOpLnFwd && packs == 2 * group &&
+                        a.row_size % VecWidth<T>::value == 0 &&
+                        a.rows * a.row_size > (int64_t{1} << 24);
+      if (packs <= 2 * group && !deep) {
         want = 2;
       } else if (packs <= 3 * group && packs > 2 * group) {
         want = 3;
