@@ -4,7 +4,7 @@
 // A FusedBatchNormV3 + FusedBatchNormGradV3 pair cost 85 us of host time in
 // Python (30 attribute reads, 13 tensor allocations, two context managers,
 // ctypes conversions of 18 arguments) for 19 us of device work on [8,14,14,64],
-// 25 us here; the functions here take the calls that need no conversion -
+// 25 us here with every tensor allocated through the dispatcher and 12 without; the functions here take the calls that need no conversion -
 // strided, contiguous tensors of the right types on one CUDA device - and return
 // None for every other call, which the Python path then converts or refuses as
 // it always did.  So what is accepted, refused and returned does not depend on
@@ -19,8 +19,10 @@
 #include <torch/csrc/utils/pybind.h>
 
 #include <ATen/ATen.h>
+#include <ATen/EmptyTensor.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -90,14 +92,54 @@ bool IsF32Vector(const at::Tensor* t, int64_t c, const at::Tensor& like) {
          t->device() == like.device();
 }
 
-at::Tensor Vector(int64_t c, const at::Tensor& like, at::ScalarType dtype = at::kFloat) {
-  return at::empty({c}, like.options().dtype(dtype));
+// Outputs and scratch come from torch's caching allocator on the current device and
+// stream, without the dispatcher's way there: it has nothing left to decide for a
+// plain CUDA tensor.
+constexpr c10::DispatchKeySet kCudaKey(c10::DispatchKey::CUDA);
+
+c10::Allocator* Allocator() { return c10::cuda::CUDACachingAllocator::get(); }
+
+at::Tensor EmptyLike(const at::Tensor& t) {
+  if (t.has_names()) return at::empty_like(t);
+  return at::detail::empty_strided_generic(t.sizes(), t.strides(), Allocator(), kCudaKey,
+                                           t.scalar_type());
 }
 
-at::Tensor Scratch(size_t bytes, const at::Tensor& like) {
-  return at::empty({static_cast<int64_t>(bytes < 16 ? 16 : bytes)},
-                   like.options().dtype(at::kByte));
+at::Tensor Empty(at::IntArrayRef sizes, at::ScalarType dtype) {
+  return at::detail::empty_generic(sizes, Allocator(), kCudaKey, dtype, std::nullopt);
 }
+
+// The small float outputs of one call: tensors of their own that share one allocation,
+// each on a 512-byte boundary as the allocator's are.
+class FloatBlock {
+ public:
+  FloatBlock(int64_t vectors, int64_t length) : step_((length + 127) / 128 * 128) {
+    const size_t bytes = static_cast<size_t>(vectors * step_) * sizeof(float);
+    storage_ = c10::Storage(c10::make_intrusive<c10::StorageImpl>(
+        c10::StorageImpl::use_byte_size_t(), bytes, Allocator()->allocate(bytes), Allocator(),
+        /*resizable=*/true));
+  }
+  at::Tensor Next(at::IntArrayRef sizes) {
+    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(
+        c10::Storage(storage_), kCudaKey, c10::scalarTypeToTypeMeta(at::kFloat));
+    c10::TensorImpl* impl = t.unsafeGetTensorImpl();
+    impl->set_storage_offset(used_++ * step_);
+    impl->set_sizes_contiguous(sizes);
+    return t;
+  }
+
+ private:
+  c10::Storage storage_;
+  int64_t step_, used_ = 0;
+};
+
+// Scratch of at least `bytes`, for the length of the call.
+struct Scratch {
+  explicit Scratch(size_t bytes)
+      : size(bytes < 16 ? 16 : bytes), data(Allocator()->allocate(size)) {}
+  size_t size;
+  c10::DataPtr data;
+};
 
 // [outer, channels, inner] of a shape; false: not a layout name or too few axes.
 bool Geometry(const at::Tensor& x, PyObject* format, int64_t* outer, int64_t* c, int64_t* inner) {
@@ -190,20 +232,20 @@ PyObject* BnForward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
   }
   const c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor y = at::empty_like(x);
-  at::Tensor s0 = Vector(c, x), s1 = Vector(c, x), s2 = Vector(c, x), s3 = Vector(c, x);
-  at::Tensor r3 = at::empty({}, x.options().dtype(at::kFloat));
+  at::Tensor y = EmptyLike(x);
+  FloatBlock block(5, c);
+  at::Tensor s0 = block.Next(c), s1 = block.Next(c), s2 = block.Next(c), s3 = block.Next(c);
+  at::Tensor r3 = block.Next({});
   const auto F = [](const at::Tensor& t) { return static_cast<float*>(t.data_ptr()); };
   int rc;
   if (training) {
-    const size_t bytes = g_api.BnWorkspaceBytes(outer, c, inner);
-    at::Tensor ws = Scratch(bytes, x);
+    const Scratch ws(g_api.BnWorkspaceBytes(outer, c, inner));
     pybind11::gil_scoped_release nogil;
     rc = g_api.LaunchBnFwdTrainOp(
         code, x.data_ptr(), F(*scale), F(*offset), have_est ? F(*mean) : nullptr,
         have_est ? F(*var) : nullptr, y.data_ptr(), F(s0), F(s1), F(s2), F(s3), F(r3), outer, c,
-        inner, static_cast<float>(eps), static_cast<float>(factor), ws.data_ptr(),
-        static_cast<size_t>(ws.numel()), StreamOf(x));
+        inner, static_cast<float>(eps), static_cast<float>(factor), ws.data.get(), ws.size,
+        StreamOf(x));
   } else {
     pybind11::gil_scoped_release nogil;
     rc = g_api.LaunchBnFwdInferOp(code, x.data_ptr(), F(*scale), F(*offset), F(*mean), F(*var),
@@ -235,17 +277,18 @@ PyObject* BnGradient(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
   }
   const c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor dx = at::empty_like(x);
-  at::Tensor ds = Vector(c, x), db = Vector(c, x), r4 = Vector(c, x), r5 = Vector(c, x);
+  at::Tensor dx = EmptyLike(x);
+  FloatBlock block(4, c);
+  at::Tensor ds = block.Next(c), db = block.Next(c), r4 = block.Next(c), r5 = block.Next(c);
   const auto F = [](const at::Tensor& t) { return static_cast<float*>(t.data_ptr()); };
   int rc;
   {
-    at::Tensor ws = Scratch(g_api.BnWorkspaceBytes(outer, c, inner), x);
+    const Scratch ws(g_api.BnWorkspaceBytes(outer, c, inner));
     pybind11::gil_scoped_release nogil;
     rc = g_api.LaunchBnGradOp(code, dy.data_ptr(), x.data_ptr(), F(*scale), F(*mean), F(*var),
                               dx.data_ptr(), F(ds), F(db), F(r4), F(r5), outer, c, inner,
-                              static_cast<float>(eps), training, ws.data_ptr(),
-                              static_cast<size_t>(ws.numel()), StreamOf(x));
+                              static_cast<float>(eps), training, ws.data.get(), ws.size,
+                              StreamOf(x));
   }
   return Results(rc, {dx, ds, db, r4, r5});
   END_HANDLE_TH_ERRORS
@@ -267,7 +310,7 @@ PyObject* BiasAct(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   const int act = static_cast<int>(PyLong_AsLong(a[3]));
   const c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor y = at::empty_like(x);
+  at::Tensor y = EmptyLike(x);
   int rc;
   {
     pybind11::gil_scoped_release nogil;
@@ -294,17 +337,17 @@ PyObject* BiasReluGrad(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
   }
   const c10::cuda::CUDAGuard guard(g.device());
-  at::Tensor dx = at::empty_like(g);
-  at::Tensor db = Vector(c, g, g.scalar_type());
+  at::Tensor dx = EmptyLike(g);
+  at::Tensor db = Empty(c, g.scalar_type());
   int rc;
   {
-    at::Tensor ws = Scratch(g_api.BiasGradWorkspaceBytes(outer, c, inner,
-                                                         static_cast<int>(g.element_size())), g);
+    const Scratch ws(
+        g_api.BiasGradWorkspaceBytes(outer, c, inner, static_cast<int>(g.element_size())));
     pybind11::gil_scoped_release nogil;
     rc = ByDtype(code, g_api.LaunchBiasAddReluGrad_F32, g_api.LaunchBiasAddReluGrad_F16,
                  g_api.LaunchBiasAddReluGrad_BF16)(
-        g.data_ptr(), f.data_ptr(), dx.data_ptr(), db.data_ptr(), outer, c, inner, ws.data_ptr(),
-        static_cast<size_t>(ws.numel()), StreamOf(g));
+        g.data_ptr(), f.data_ptr(), dx.data_ptr(), db.data_ptr(), outer, c, inner, ws.data.get(),
+        ws.size, StreamOf(g));
   }
   return Results(rc, {dx, db});
   END_HANDLE_TH_ERRORS
@@ -328,7 +371,7 @@ PyObject* LayerNorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t last = x.size(-1);
   if (code < 0 || !RowVector(g, x, last) || !RowVector(b, x, last)) Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor y = at::empty_like(x);
+  at::Tensor y = EmptyLike(x);
   int rc;
   {
     pybind11::gil_scoped_release nogil;
@@ -356,17 +399,16 @@ PyObject* LayerNormGrad(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
   }
   const c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor dx = at::empty_like(x), dg = at::empty_like(*g), db = at::empty_like(*b);
+  at::Tensor dx = EmptyLike(x), dg = EmptyLike(*g), db = EmptyLike(*b);
   const int64_t rows = x.numel() / last;
   int rc;
   {
-    at::Tensor ws = Scratch(g_api.LayerNormGradWorkspaceBytes(rows, last), x);
+    const Scratch ws(g_api.LayerNormGradWorkspaceBytes(rows, last));
     pybind11::gil_scoped_release nogil;
     rc = ByDtype(code, g_api.LaunchLayerNormGrad_F32, g_api.LaunchLayerNormGrad_F16,
                  g_api.LaunchLayerNormGrad_BF16)(
         dy.data_ptr(), x.data_ptr(), g->data_ptr(), dx.data_ptr(), dg.data_ptr(), db.data_ptr(),
-        rows, last, static_cast<float>(eps), ws.data_ptr(), static_cast<size_t>(ws.numel()),
-        StreamOf(x));
+        rows, last, static_cast<float>(eps), ws.data.get(), ws.size, StreamOf(x));
   }
   return Results(rc, {dx, dg, db});
   END_HANDLE_TH_ERRORS
@@ -384,10 +426,10 @@ PyObject* RmsNorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t last = x.size(-1);
   if ((!f32 && x.scalar_type() != at::kBFloat16) || !RowVector(g, x, last)) Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor y = at::empty_like(x), normalized = at::empty_like(x);
+  at::Tensor y = EmptyLike(x), normalized = EmptyLike(x);
   auto shape = x.sizes().vec();
   shape.back() = 1;
-  at::Tensor inv = at::empty(shape, x.options());
+  at::Tensor inv = Empty(shape, x.scalar_type());
   const int64_t rows = x.numel() / last;
   {
     pybind11::gil_scoped_release nogil;
@@ -424,7 +466,7 @@ PyObject* RmsNormGradDx(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
   }
   const c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor dx = at::empty_like(x);
+  at::Tensor dx = EmptyLike(x);
   const int64_t rows = x.numel() / last;
   {
     pybind11::gil_scoped_release nogil;

@@ -184,7 +184,7 @@ def _native_result(out, kind, what):
     output); an int is the launcher's error code."""
     if type(out) is int:
         _check(out, what)
-    return out[0] if kind is None else kind._make(out)
+    return out[0] if kind is None else tuple.__new__(kind, out)
 
 
 _ws_cache = {}
