@@ -1885,8 +1885,8 @@ __global__ void __launch_bounds__(kOnChipThreads, 1)
 // any length) is walked as one flattened sequence of packs, 512 apart.
 constexpr int kOnChipMaxGroup = 16;
 
-template <typename T, int kMode>
-__global__ void __launch_bounds__(kOnChipThreads, 1)
+template <typename T, int kMode, int kPerSm>
+__global__ void __launch_bounds__(kOnChipThreads, kPerSm)
     BnOnChipPlanesKernel(const T* x, const T* dy, T* out, ApplyArgs a, int64_t outer,
                          int64_t channels, int inner, int group, int64_t outer_per_cta,
                          int slots) {
@@ -2719,6 +2719,7 @@ struct OnChipPlan {
   int slots = 0;     // 16-byte slots per thread and stream
   int64_t per_cta = 0;
   double cost = 0.0;
+  bool waves = false;   // more channels than CTAs that are resident at once
 };
 
 // Clusters of `cluster` CTAs of `kernel` that are resident at once with all the
@@ -2777,7 +2778,7 @@ inline void OnChipTry(OnChipPlan* best, Kernel kernel, std::atomic<int> (*by_dev
   const double cost = OnChipCost(slots * streams, k, segments);
   if (best->tx != 0 && cost >= best->cost) return;
   if (gx > OnChipClusters(kernel, by_device, k)) return;
-  *best = OnChipPlan{tx, k, static_cast<int>(gx), static_cast<int>(slots), per, cost};
+  *best = OnChipPlan{tx, k, static_cast<int>(gx), static_cast<int>(slots), per, cost, false};
 }
 
 // Channels-last (the geometry of VectorChain).
@@ -2836,11 +2837,64 @@ inline OnChipPlan PlanOnChipPlanes(const Geom& g, const void* x, const void* out
       const int64_t per = CeilDiv(g.outer, k);
       const int64_t slots = group == 1 ? CeilDiv(per * run, kOnChipThreads)
                                        : CeilDiv(per, kOnChipThreads / run);
-      OnChipTry(&best, BnOnChipPlanesKernel<T, kMode>, by_device, group, g.channels / group, k,
+      OnChipTry(&best, BnOnChipPlanesKernel<T, kMode, 1>, by_device, group, g.channels / group, k,
                 per, slots, kStreams, run < 8 ? 1.25 : 1.0);
     }
   }
   return best;
+}
+
+// Channel-major layers beyond that, where one CTA holds a channel (planes of whole packs):
+// the same kernel in waves of single CTAs.  Every value is read once; a CTA takes no more
+// than half an SM's shared memory, so that two share the SM and one loads while the
+// other writes.  A wave costs about 4 us beside its bytes, so CTAs have to be well filled
+// (7 to 12 slots) and waves too - two thirds where the chain walks long planes, nine
+// tenths where its channel-group kernels take short ones.  Us, chain -> this form: bf16
+// [64,500,24,24] forward 29.9 -> 20.3, [16,512,28,28] gradient 20.3 -> 15.1, [20,1000,28,28]
+// 32.4 -> 27.9; fp32 [10,640,40,40] forward 37.7 -> 21.5, [32,512,20,20] 19.6 -> 16.0,
+// [100,2000,10,10] gradient 68.4 -> 54.8.  Beyond the lines: bf16 [128,2048,8,8] forward, 2 slots,
+// 21.7 -> 35.6; fp32 [100,2000,10,10] forward, 5 slots, 43.5 -> 45.7; bf16 [256,1024,8,8]
+// gradient, waves filled to 0.86, 28.1 -> 29.3.  Channels over clusters of four and more
+// (bf16 [64,512,28,28] gradient 49.6 -> 56.9) and groups of channels whose planes share packs
+// ([256,2048,7,7] 30.9 -> 38.3: the choices per element bound it) keep the chain.
+constexpr int kOnChipWaveSlots = 12;   // of all streams
+
+template <typename T, int kMode>
+inline OnChipPlan PlanOnChipWaves(const Geom& g, const void* x, const void* out,
+                                  const void* dy) {
+  OnChipPlan p;
+  constexpr int kStreams = kMode == kFwd ? 1 : 2;
+  constexpr int kVec = VecWidth<T>::value;
+  const int tuned = GetTuning(kTuneBnGrid);
+  if (tuned < 0 || GetTuning(kTuneBnOnChipTx) < 0) return p;
+  if (g.inner <= 1 || g.inner % kVec != 0 || g.channels > 0x7fffffffLL) return p;
+  if (!Aligned16(x) || !Aligned16(out) || (dy != nullptr && !Aligned16(dy))) return p;
+  const int64_t packs = g.outer * (g.inner / kVec);   // of a channel
+  const int64_t slots = CeilDiv(packs, static_cast<int64_t>(kOnChipThreads));
+  if (slots * kStreams > kOnChipWaveSlots) return p;
+  static std::atomic<int> by_device[kMaxDevices];
+  const int64_t resident = PerDevice(by_device, [] {
+    constexpr int kBytes = kOnChipWaveSlots * kOnChipThreads * 16;
+    auto kernel = BnOnChipPlanesKernel<T, kMode, 2>;
+    int n = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kOnChipThreads, kBytes) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      return -1;
+    }
+    return n > 0 ? n * SmCount() : -1;
+  });
+  if (resident < 0) return p;
+  const int64_t room = CeilDiv(g.channels, resident) * resident;
+  const double full = g.inner >= 400 ? 0.66 : 0.9;
+  if (tuned == 0 &&
+      (slots * kStreams < 7 || static_cast<double>(g.channels) < full * static_cast<double>(room))) {
+    return p;
+  }
+  return OnChipPlan{1, 1, static_cast<int>(g.channels), static_cast<int>(slots), g.outer, 0.0,
+                    true};
 }
 
 template <typename T, int kMode>
@@ -2855,9 +2909,11 @@ int LaunchOnChip(const OnChipPlan& p, const T* x, const T* dy, T* out, const App
                           dim3(p.tx, kOnChipThreads / p.tx), smem, stream, x, dy, out, a, g.outer,
                           g.channels / VecWidth<T>::value, g.channels, p.per_cta, p.slots);
   } else {
-    err = LaunchClustered(pdl, p.cluster, BnOnChipPlanesKernel<T, kMode>, grid,
-                          dim3(kOnChipThreads), smem, stream, x, dy, out, a, g.outer, g.channels,
-                          static_cast<int>(g.inner), p.tx, p.per_cta, p.slots);
+    const auto kernel =
+        p.waves ? BnOnChipPlanesKernel<T, kMode, 2> : BnOnChipPlanesKernel<T, kMode, 1>;
+    err = LaunchClustered(pdl, p.cluster, kernel, grid, dim3(kOnChipThreads), smem, stream, x, dy,
+                          out, a, g.outer, g.channels, static_cast<int>(g.inner), p.tx, p.per_cta,
+                          p.slots);
   }
   if (err != cudaSuccess) cudaGetLastError();
   return static_cast<int>(err);
@@ -2917,9 +2973,9 @@ int FwdTrain(const void* x, const float* scale, const float* offset,
       if (rc != cudaErrorCooperativeLaunchTooLarge) return rc;
     }
   }
-  const OnChipPlan p = VectorChain<T>(g, x, y, nullptr)
-                           ? PlanOnChip<T, kFwd>(g)
-                           : PlanOnChipPlanes<T, kFwd>(g, x, y, nullptr);
+  OnChipPlan p = VectorChain<T>(g, x, y, nullptr) ? PlanOnChip<T, kFwd>(g)
+                                                  : PlanOnChipPlanes<T, kFwd>(g, x, y, nullptr);
+  if (p.tx == 0) p = PlanOnChipWaves<T, kFwd>(g, x, y, nullptr);
   if (p.tx > 0) {
     a.stat_out = f;
     return LaunchOnChip<T, kFwd>(p, xt, nullptr, static_cast<T*>(y), a, g, stream);
@@ -3026,8 +3082,9 @@ int Grad(const void* dy, const void* x, const float* scale, const float* mean,
       if (rc != cudaErrorCooperativeLaunchTooLarge) return rc;
     }
   }
-  const OnChipPlan p = vector_chain ? PlanOnChip<T, kGrad>(g)
-                                    : PlanOnChipPlanes<T, kGrad>(g, x, dx, dy);
+  OnChipPlan p = vector_chain ? PlanOnChip<T, kGrad>(g)
+                              : PlanOnChipPlanes<T, kGrad>(g, x, dx, dy);
+  if (p.tx == 0) p = PlanOnChipWaves<T, kGrad>(g, x, dx, dy);
   if (p.tx > 0) {
     a.fold_use = is_training;
     a.dscale = dscale;

@@ -35,7 +35,8 @@ enum TuningKey {
   kTuneBnOnChipTx = 24,     // channel packs per column block (channel-major: channels per group) of the
                             // one-kernel form; 0: by rule, -1: off (the chain of kernels at every size)
   kTuneBnOnChipCluster = 25,  // CTAs per cluster of the one-kernel form; 0: by rule
-  kTuneBnGrid = 26,         // grid-wide one-kernel form of large layers: 0 by rule, 1 at every size, -1 off
+  kTuneBnGrid = 26,         // one-kernel forms of large layers (grid-wide; channel-major in
+                            // waves): 0 by rule, 1 wherever possible, -1 off
   kTuneRowCtas = 27,        // most CTAs per SM of the row kernels; 0: by rule
   kTuneCount = 28
 };
