@@ -4,11 +4,11 @@
 // A FusedBatchNormV3 + FusedBatchNormGradV3 pair cost 85 us of host time in
 // Python (30 attribute reads, 13 tensor allocations, two context managers,
 // ctypes conversions of 18 arguments) for 19 us of device work on [8,14,14,64],
-// 25 us here with every tensor allocated through the dispatcher and 12 without; the functions here take the calls that need no conversion -
-// strided, contiguous tensors of the right types on one CUDA device - and return
-// None for every other call, which the Python path then converts or refuses as
-// it always did.  So what is accepted, refused and returned does not depend on
-// this file.
+// 25 us here with every tensor allocated through the dispatcher and 15 without; the
+// functions here take the calls that need no conversion - strided, contiguous
+// tensors of the right types on one CUDA device - and return None for every other
+// call, which the Python path then converts or refuses as it always did.  So what
+// is accepted, refused and returned does not depend on this file.
 //
 // Scratch comes from the caching allocator for the length of the call: it is
 // ordered by the current stream, private to the call (several threads may run
@@ -109,29 +109,9 @@ at::Tensor Empty(at::IntArrayRef sizes, at::ScalarType dtype) {
   return at::detail::empty_generic(sizes, Allocator(), kCudaKey, dtype, std::nullopt);
 }
 
-// The small float outputs of one call: tensors of their own that share one allocation,
-// each on a 512-byte boundary as the allocator's are.
-class FloatBlock {
- public:
-  FloatBlock(int64_t vectors, int64_t length) : step_((length + 127) / 128 * 128) {
-    const size_t bytes = static_cast<size_t>(vectors * step_) * sizeof(float);
-    storage_ = c10::Storage(c10::make_intrusive<c10::StorageImpl>(
-        c10::StorageImpl::use_byte_size_t(), bytes, Allocator()->allocate(bytes), Allocator(),
-        /*resizable=*/true));
-  }
-  at::Tensor Next(at::IntArrayRef sizes) {
-    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(
-        c10::Storage(storage_), kCudaKey, c10::scalarTypeToTypeMeta(at::kFloat));
-    c10::TensorImpl* impl = t.unsafeGetTensorImpl();
-    impl->set_storage_offset(used_++ * step_);
-    impl->set_sizes_contiguous(sizes);
-    return t;
-  }
-
- private:
-  c10::Storage storage_;
-  int64_t step_, used_ = 0;
-};
+// A per-channel output.  Every one has a storage of its own, as the Python path's do: a caller
+// may resize, save or keep one without touching or holding the others.
+at::Tensor Vector(int64_t c) { return Empty(c, at::kFloat); }
 
 // Scratch of at least `bytes`, for the length of the call.
 struct Scratch {
@@ -233,9 +213,8 @@ PyObject* BnForward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   const c10::cuda::CUDAGuard guard(x.device());
   at::Tensor y = EmptyLike(x);
-  FloatBlock block(5, c);
-  at::Tensor s0 = block.Next(c), s1 = block.Next(c), s2 = block.Next(c), s3 = block.Next(c);
-  at::Tensor r3 = block.Next({});
+  at::Tensor s0 = Vector(c), s1 = Vector(c), s2 = Vector(c), s3 = Vector(c);
+  at::Tensor r3 = Empty({}, at::kFloat);
   const auto F = [](const at::Tensor& t) { return static_cast<float*>(t.data_ptr()); };
   int rc;
   if (training) {
@@ -278,8 +257,7 @@ PyObject* BnGradient(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   const c10::cuda::CUDAGuard guard(x.device());
   at::Tensor dx = EmptyLike(x);
-  FloatBlock block(4, c);
-  at::Tensor ds = block.Next(c), db = block.Next(c), r4 = block.Next(c), r5 = block.Next(c);
+  at::Tensor ds = Vector(c), db = Vector(c), r4 = Vector(c), r5 = Vector(c);
   const auto F = [](const at::Tensor& t) { return static_cast<float*>(t.data_ptr()); };
   int rc;
   {

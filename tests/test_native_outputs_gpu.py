@@ -1,4 +1,4 @@
-"""Outputs of the native host path: tensors of their own, whatever they share underneath."""
+"""Outputs of the native host path: tensors of their own, down to the storage."""
 import pytest
 import torch
 
@@ -29,6 +29,26 @@ def test_small_outputs_do_not_overlap(kernel_lib, c):
     torch.cuda.synchronize()
     again = raw_ops.FusedBatchNormV3(x, v, v, e, e)
     assert torch.equal(kept, before) and torch.equal(again.batch_mean, before)
+
+
+def test_small_outputs_have_their_own_storage(kernel_lib):
+    """Growing one output in place, or keeping one, touches and holds none of the others."""
+    c = 64
+    x = torch.randn(64, c, device="cuda")
+    v, e = torch.rand(c, device="cuda") + 0.5, torch.empty(0, device="cuda")
+    f = raw_ops.FusedBatchNormV3(x, v, v, e, e)
+    g = raw_ops.FusedBatchNormGradV3(x, x, v, f.reserve_space_1, f.reserve_space_2)
+    for out in (f, g):
+        for t in out:
+            assert t.storage_offset() == 0
+            assert t.untyped_storage().nbytes() == t.numel() * t.element_size()
+        assert len({t.untyped_storage().data_ptr() for t in out if t.numel()}) \
+            == sum(1 for t in out if t.numel())
+        before = [t.clone() for t in out]
+        for k, t in enumerate(out):
+            t.resize_(4 * t.numel() + 256).fill_(7.0)
+            for a, b in zip(out[k + 1:], before[k + 1:]):
+                assert torch.equal(a, b)
 
 
 def test_strides_and_names_follow_the_input(kernel_lib):
