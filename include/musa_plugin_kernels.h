@@ -468,6 +468,13 @@ size_t BnWorkspaceBytes(int64_t outer, int64_t channels, int64_t inner);
  *   that is not 1 (est_* may be NULL when it is 1);
  *   saved_mean = mean, saved_var = population variance.
  * y may be x itself (in place); any other overlap of y with x is not allowed.
+ * Large channels-last layers (rows of whole 16-byte packs, 16 MiB of inputs and
+ * more; the gradient too) are one cooperative kernel of a CTA per SM: it starts
+ * once every SM has room, so it waits for kernels of other streams that hold an
+ * SM's shared memory, and a kernel that runs on another stream must not wait for
+ * work behind this call.  MusaKernelsSetTuning(26, -1) keeps the chain of smaller
+ * kernels, which run on the SMs that are free; so does a context that owns fewer
+ * SMs than the device.
  * Replaces muDNN BatchNorm::RunComposite plus the copies and the Bessel
  * fix-up after it (musa_ext/kernels/nn/musa_fused_batchnorm_op.cc:106-171). */
 int LaunchBnFwdTrain_F32(const void* x, const float* scale, const float* offset,
