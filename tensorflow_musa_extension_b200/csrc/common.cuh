@@ -278,6 +278,36 @@ inline int PerDevice(std::atomic<int>* table, Init init) {
   return v;
 }
 
+// v = the values at p (in L2) where `there`, zeros otherwise.  A predicated load: several of them stay in
+// flight together, where the compiler sinks conditional loads into the branches that use them.
+__device__ __forceinline__ void LoadIf(const float* p, bool there, float (&v)[1]) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.s32 q, %2, 0;\n"
+      "mov.f32 %0, 0f00000000;\n"
+      "@q ld.global.cg.f32 %0, [%1];\n"
+      "}\n"
+      : "=f"(v[0])
+      : "l"(p), "r"(static_cast<int>(there))
+      : "memory");
+}
+__device__ __forceinline__ void LoadIf(const float* p, bool there, float (&v)[4]) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.s32 q, %5, 0;\n"
+      "mov.f32 %0, 0f00000000;\n"
+      "mov.f32 %1, 0f00000000;\n"
+      "mov.f32 %2, 0f00000000;\n"
+      "mov.f32 %3, 0f00000000;\n"
+      "@q ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+      "}\n"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+      : "l"(p), "r"(static_cast<int>(there))
+      : "memory");
+}
+
 inline bool Aligned16(const void* p) {
   return (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
 }

@@ -829,14 +829,13 @@ __global__ void __launch_bounds__(256) RowNormLoopKernel(RowArgs a) {
   }
 }
 
-// dgamma / dbeta = sum over the CTAs' partial rows, fixed order.  A CTA adds 16
+// dgamma / dbeta = sum over the CTAs' partial rows, fixed order, fp64.  A CTA adds 16
 // columns; kQuads: the rows are in the order of RowNormKernel's slabs and come four
-// columns a load.  Bound by latency: one memory round trip with all loads of a
-// thread in flight, a tree over those five (single columns: ten) rows in fp32 and
-// fp64 from there on.  (Every partial widened by itself is 4096 conversions to fp64
-// per SM at 16 a cycle: bf16 [16384,1024], a call of 20.4 us without this kernel,
-// takes 22.8 us that way and 22.3 so; two loads at a time, 8 columns a CTA and a
-// serial last step took 23.5.  [1024,1024]: 7.3, 6.8 and 8.3.)
+// columns a load.  Bound by latency: a thread's loads are in flight together (320 partial rows in slab
+// order and 160 in plain order a memory round trip; a launch leaves at most 4 per SM), which takes
+// loads without a branch: the lanes of a warp read eight partial rows in slab order, where the last row
+// again past the end is cheaper than predicated loads and additions, and two in plain order, where
+// those are (fp32 [6144,1024], the call, 17.2 and 18.5 us; bf16 [524,500] 5.6 and 5.4).
 template <typename T, bool kQuads>
 __global__ void __launch_bounds__(256)
     LnGradFinalizeKernel(const float* __restrict__ partial, int n_partial,
@@ -846,7 +845,6 @@ __global__ void __launch_bounds__(256)
   constexpr int kWide = kQuads ? 4 : 1;            // columns per load
   constexpr int kUnits = kColumns / kWide;         // loads per partial row and CTA
   constexpr int kLanes = kWarps * 32 / kUnits;     // partial rows at once
-  using P = Pack<float, kWide>;
   __shared__ double red[kWarps][kColumns];
   const int tid = threadIdx.x;
   const int64_t unit = static_cast<int64_t>(blockIdx.x) * kUnits + tid % kUnits;
@@ -869,26 +867,30 @@ __global__ void __launch_bounds__(256)
   if (unit * kWide < 2 * static_cast<int64_t>(row_size)) {
     const float* const from = partial + unit * kWide;
     for (int p = tid / kUnits; p < n_partial; p += kLoads * kLanes) {
-      P v[kLoads];
+      Pack<float, kWide> v[kLoads];
 #pragma unroll
       for (int i = 0; i < kLoads; ++i) {
         const int r = p + i * kLanes;
-#pragma unroll
-        for (int w = 0; w < kWide; ++w) v[i].v[w] = 0.0f;
-        if (r < n_partial) {
-          v[i] = *reinterpret_cast<const P*>(from + static_cast<int64_t>(r) * 2 * row_size);
+        if constexpr (kQuads) {   // (past the end: the last row again, replaced by zeros)
+          v[i] = *reinterpret_cast<const Pack<float, kWide>*>(
+              from + static_cast<int64_t>(r < n_partial ? r : n_partial - 1) * 2 * row_size);
+        } else {
+          LoadIf(from + static_cast<int64_t>(r) * 2 * row_size, r < n_partial, v[i].v);
         }
       }
 #pragma unroll
-      for (int m = 1; m < kLoads; m *= 2) {
+      for (int i = 0; i < kLoads; ++i) {
+        const bool there = i == 0 || p + i * kLanes < n_partial;
 #pragma unroll
-        for (int i = 0; i + m < kLoads; i += 2 * m) {
-#pragma unroll
-          for (int w = 0; w < kWide; ++w) v[i].v[w] += v[i + m].v[w];
+        for (int w = 0; w < kWide; ++w) {
+          if constexpr (kQuads) {
+            if (!there) v[i].v[w] = 0.0f;
+            s[w] += static_cast<double>(v[i].v[w]);
+          } else if (there) {
+            s[w] += static_cast<double>(v[i].v[w]);
+          }
         }
       }
-#pragma unroll
-      for (int w = 0; w < kWide; ++w) s[w] += static_cast<double>(v[0].v[w]);
     }
   }
 #pragma unroll

@@ -3,6 +3,7 @@ from one partial row to more than one thread requests at once, columns that do n
 CTA, rows in slab order and in plain order."""
 import numpy as np
 import pytest
+import torch
 
 from oracle import np_ref
 from helpers import assert_close, np_dtype, to_numpy, to_torch
@@ -40,3 +41,27 @@ def test_column_sums(kernel_lib, dtype, n, blocks):
             assert_close(to_numpy(got[k]), want[k], rt, at, name)
         for a, b in zip(got, again):
             assert (to_numpy(a) == to_numpy(b)).all()
+
+
+# One row a CTA: rows in slab order, rows that start inside a pack, rows beyond the register layouts.
+@pytest.mark.parametrize("dtype,n", [("float32", 4096), ("float32", 4097), ("float32", 20000),
+                                     ("bfloat16", 8192), ("bfloat16", 8191)])
+def test_partial_rows_add_in_64_bits(kernel_lib, dtype, n):
+    """Partial rows that cancel: of 2^30, -2^30 and 1, in turn, an fp64 sum leaves the exact number of
+    ones, an fp32 sum of two of them rounds the one away.  An infinity and a NaN stay in their
+    columns."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = min(sms, 140) // 3 * 3
+    dt = getattr(torch, dtype)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(rows, n, device="cuda", generator=gen).to(dt)
+    dy = torch.tensor([2.0 ** 30, -2.0 ** 30, 1.0], device="cuda").repeat(rows // 3)[:, None]
+    dy = dy.repeat(1, n).to(dt)
+    gamma, beta = torch.ones(n, device="cuda", dtype=dt), torch.zeros(n, device="cuda", dtype=dt)
+    db = raw_ops.MusaLayerNormGrad(dy, x, gamma, beta)[2]
+    assert torch.equal(db, torch.full_like(db, rows // 3))
+    dy[5, 3], dy[70, 9] = float("inf"), float("nan")
+    db = raw_ops.MusaLayerNormGrad(dy, x, gamma, beta)[2].float()
+    assert db[3] == float("inf") and torch.isnan(db[9])
+    db[3] = db[9] = rows // 3
+    assert torch.equal(db, torch.full_like(db, rows // 3))
