@@ -274,10 +274,10 @@ __global__ void __launch_bounds__(kGridThreads, 1)
   cooperative_groups::this_grid().sync();
 
   // ---- Totals of the CTA's entries over the gy CTAs of its column block: `lanes` threads
-  // share a group of four.  (Loads past L1: other SMs wrote them.)  Ten partial rows
-  // are requested at once - each is an L2 round trip - and added as a tree in fp32, whose few
-  // roundings of single partial sums are far below that of the results; everything after it is fp64
-  // (converting every partial took 1300 cycles).
+  // share a group of four.  Five partial rows are requested at once: each is an L2 round trip.
+  // (Past the end the last row again, instead, makes that row a hot spot: 1 us.)  Every partial is
+  // widened by itself and added in fp64, as in the chain; a tree of ten in fp32 before that measured the
+  // same (fp16 [200704,256] forward + gradient 117.6 us and 117.9).
   float* const coef = scratch + 5 * 1024;   // [4][nch], behind 16 KB of totals
   {
     double* const tot = reinterpret_cast<double*>(scratch);   // [lanes][n_out]
@@ -286,32 +286,22 @@ __global__ void __launch_bounds__(kGridThreads, 1)
     const int lanes = kGridThreads >> log_units;
     const int lane = tid >> log_units, unit = tid & (units - 1);
     {
-      constexpr int kLoads = 10;
+      constexpr int kLoads = 5;
       double t[4] = {0.0, 0.0, 0.0, 0.0};
-      const float4* p = reinterpret_cast<const float4*>(partial) + (lane * gx + bx) * units + unit;
-      const int step = lanes * gx * units;
+      const float* p = partial + ((lane * gx + bx) * units + unit) * 4;
+      const int step = lanes * gx * units * 4;
 #pragma unroll 1
       for (int r = lane; r < gy; r += kLoads * lanes) {
-        float4 v[kLoads];
+        float v[kLoads][4];
 #pragma unroll
-        for (int i = 0; i < kLoads; ++i, p += step) {
-          v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (r + i * lanes < gy) v[i] = __ldcg(p);
-        }
+        for (int i = 0; i < kLoads; ++i, p += step) LoadIf(p, r + i * lanes < gy, v[i]);
 #pragma unroll
-        for (int w = 1; w < kLoads; w *= 2) {
+        for (int i = 0; i < kLoads; ++i) {
+          if (r + i * lanes < gy) {
 #pragma unroll
-          for (int i = 0; i + w < kLoads; i += 2 * w) {
-            v[i].x += v[i + w].x;
-            v[i].y += v[i + w].y;
-            v[i].z += v[i + w].z;
-            v[i].w += v[i + w].w;
+            for (int e = 0; e < 4; ++e) t[e] += static_cast<double>(v[i][e]);
           }
         }
-        t[0] += static_cast<double>(v[0].x);
-        t[1] += static_cast<double>(v[0].y);
-        t[2] += static_cast<double>(v[0].z);
-        t[3] += static_cast<double>(v[0].w);
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) tot[lane * n_out + unit * 4 + i] = t[i];

@@ -85,3 +85,45 @@ def test_in_place_streams_and_capture(kernel_lib):
     for out in (*outs, captured):
         for a, b in zip(out, want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,c,tx,big,small", [
+    ("float32", 32, 8, 40, 0), ("bfloat16", 64, 8, 40, 0), ("float32", 64, 16, 40, 0),
+    ("float16", 32, 4, 14, -14),
+    # Sums of the ones below the normal range of fp32; sums of `big` next to its end.
+    ("float32", 32, 8, -100, -140), ("float32", 32, 8, 118, 90)])
+def test_partial_sums_add_in_64_bits(kernel_lib, dtype, c, tx, big, small):
+    """CTAs whose sums cancel: their rows hold `big`, -`big` and 1 in turn, an fp64 total leaves the
+    exact sum of the ones, an fp32 sum of two of them rounds it away.  An infinity and a
+    NaN stay in their channels."""
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count
+    lanes, each = 512 // tx, 4
+    big, small = 2.0 ** big, 2.0 ** small
+    kind = torch.arange(lanes * each * ctas, device="cuda") // lanes % ctas
+    kind = torch.where(kind >= ctas // 3 * 3, 3, kind % 3)
+    value = torch.tensor([big, -big, small, 0.0], device="cuda")[kind]
+    dy = value[:, None].repeat(1, c).to(getattr(torch, dtype))
+    x = torch.ones_like(dy)
+    ones, zeros = torch.ones(c, device="cuda"), torch.zeros(c, device="cuda")
+    suffix = {"float32": "F32", "float16": "F16", "bfloat16": "BF16"}[dtype]
+    want = float(lanes * each * (ctas // 3)) * small
+
+    def grad():
+        dx, ds, do = torch.empty_like(x), torch.empty(c, device="cuda"), torch.empty(c, device="cuda")
+        ws = torch.empty(kernel_lib.BnWorkspaceBytes(len(x), c, 1), dtype=torch.uint8, device="cuda")
+        with tuned(kernel_lib, (26, tx)):
+            assert getattr(kernel_lib, "LaunchBnGrad_" + suffix)(
+                dy.data_ptr(), x.data_ptr(), ones.data_ptr(), zeros.data_ptr(), ones.data_ptr(),
+                dx.data_ptr(), ds.data_ptr(), do.data_ptr(), len(x), c, 1, 0.0, True, ws.data_ptr(),
+                ws.numel(), torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        return ds, do
+
+    # x - mean and 1 / std are one: both sums are the sum of dy.
+    for t in grad():
+        assert torch.equal(t, torch.full_like(t, want))
+    dy[5, 3], dy[lanes * 7 + 1, 9] = float("inf"), float("nan")
+    for t in grad():
+        assert t[3] == float("inf") and torch.isnan(t[9])
+        t[3] = t[9] = want
+        assert torch.equal(t, torch.full_like(t, want))
