@@ -423,13 +423,25 @@ int GridCtas() {
 //  - The last two lines are not where the form stops paying (bf16 [156250,64] forward 17.4 -> 12.5): they
 //    keep the chains of two and three kernels that the launch counters are tested with
 //    ([200000,64], [4096,2048]).
+// Rows that are not whole 128-byte lines share lines between CTAs or between their row lanes, which
+// are read again where L2 does not hold them in between.  Up to a size that costs less than the form
+// saves; beyond it, chain -> this form, forward and gradient, launches of a graph:
+//   64-byte multiples    bf16 [218453,480] (200 MiB) 104, 166 -> 100, 165; 250 MiB 133, 209 -> 130, 213;
+//                        390 MiB 201, 334 -> 217, 346
+//   others               bf16 [67108,1000] (128 MiB) 69, 116 -> 64, 107; 200 MiB 112, 172 -> 107,
+//                        182; [1260307,104] (250 MiB) 134, 211 -> 138, 228
+//   of 17 to 31 packs    bf16 [209715,200] (80 MiB) 49, 80 -> 46, 79; 96 MiB 59, 97 -> 60, 99; 200 MiB
+//                        121, 189 -> 147, 229
+constexpr int64_t kMiB = 1 << 20;
+
 template <typename T, int kMode>
-bool GridPays(int64_t size, int64_t cv) {
-  constexpr int64_t kMiB = 1 << 20;
+bool GridPays(int64_t size, int64_t row_bytes, int64_t cv) {
   if (size * GridRing<kMode>::kStreams < 16 * kMiB) return false;
-  if (cv < 16) return size >= 32 * kMiB;
-  if (cv >= 256) return size > 16 * kMiB;
-  return true;
+  if (cv < 16 && size < 32 * kMiB) return false;
+  if (cv >= 256 && size <= 16 * kMiB) return false;
+  if (row_bytes % 128 == 0) return true;
+  if (row_bytes % 64 == 0) return size <= 256 * kMiB;
+  return size <= (cv > 16 && cv < 32 ? 80 : 128) * kMiB;
 }
 
 }  // namespace
@@ -442,19 +454,27 @@ BnGridPlan PlanBnGrid(const Geom& g) {
   constexpr int kVec = VecWidth<T>::value;
   const int64_t cv = g.channels / kVec;
   if (cv < kGridMinTx) return p;
-  if (tuned == 0 && !GridPays<T, kMode>(g.outer * g.channels * sizeof(T), cv)) return p;
+  const int64_t row_bytes = cv * 16, size = g.outer * row_bytes;
+  if (tuned == 0 && !GridPays<T, kMode>(size, row_bytes, cv)) return p;
   const int ctas = GridCtas<T, kMode>();
   if (ctas == 0 || cv > static_cast<int64_t>(ctas) * kGridMaxTx) return p;
   // The column block that keeps the most threads busy; 64-byte segments only where that is worth 2 %
   // more (bf16 [25390,512] gradient 19.1 us at 256 and 128 bytes, 19.8 at 64; [104166,96] forward
-  // 13.4, 12.5, 11.4), 128 bytes before 256 where few column blocks leave each CTA many
-  // partial rows to add (bf16 [101562,128] forward 14.9 and 14.0).  Widths that are no power of two
+  // 13.4, 12.5, 11.4) and they share no line with a neighbour's, 128 bytes before 256 where few column
+  // blocks leave each CTA many partial rows to add (bf16 [101562,128] forward 14.9 and 14.0), the other
+  // way round where rows are cut off the lines (bf16 [800995,72] forward 91 us at 64 and 128 bytes, 59
+  // with the row in one block; [288358,200] 73, 70, 66).  Large layers of one and a half
+  // lines a row take the row in one block too (bf16 [1365333,96] gradient 216 us at 64
+  // bytes, 203 so; [349525,96] 48.0 and 52.6).  Widths that are no power of two
   // leave lines shared by two CTAs: fp32 [31250,800] forward 60.5 us at 240 bytes, 43.2 at 256.
   double best = 0.0;
-  const int order[3] = {cv <= 32 ? 8 : 16, cv <= 32 ? 16 : 8, 4};
+  const bool halves = row_bytes % 64 == 0, narrow_first = cv <= 32 && halves;
+  const bool whole_row = cv <= 16 && row_bytes % 128 != 0 && size > 128 * kMiB;
+  const int order[3] = {narrow_first ? 8 : 16, narrow_first ? 16 : 8, 4};
   for (const int tx : order) {
     const int64_t gx = CeilDiv(cv, static_cast<int64_t>(tx));
     if (gx > ctas || (tuned >= kGridMinTx && tx != tuned)) continue;
+    if (tuned < kGridMinTx && ((tx == 4 && !halves) || (whole_row && gx > 1))) continue;
     const int64_t gy = ctas / gx;
     const double busy = static_cast<double>(cv * gy * (kGridThreads / tx)) * (tx == 4 ? 0.98 : 1.0);
     if (busy > best) {

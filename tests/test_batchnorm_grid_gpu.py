@@ -47,6 +47,27 @@ def test_against_oracle_and_chain(kernel_lib, dtype, rows, c):
         assert np.all(np.abs(a - b) <= 1e-5 * np.abs(b) + 1e-5 * max(_rms(b), 1e-12))
 
 
+@pytest.mark.parametrize("rows,c,kernels", [
+    # Rows that are not whole lines, up to their limits and one row beyond: 64-byte multiples, others,
+    # 17 to 31 packs.
+    (1398101, 96, (1, 1)), (1398102, 96, (3, 3)), (67108, 1000, (1, 1)), (67109, 1000, (2, 2)),
+    (932067, 72, (1, 1)), (932068, 72, (3, 3)), (209715, 200, (1, 1)), (209716, 200, (3, 3)),
+    # Whole lines have no limit.
+    (1100000, 128, (1, 1))])
+def test_rule(kernel_lib, rows, c, kernels):
+    """Kernels of the forward and the gradient by the rule, with the cluster form shut out."""
+    x = torch.zeros(rows, c, device="cuda", dtype=torch.bfloat16)
+    dy, s, o = torch.zeros_like(x), torch.ones(c, device="cuda"), torch.ones(c, device="cuda")
+    e = torch.empty(0, device="cuda")
+    with tuned(kernel_lib, (25, 3)):
+        counts = [kernel_lib.MusaKernelsLaunchCount()]
+        f = raw_ops.FusedBatchNormV3(x, s, o, e, e, epsilon=EPS)
+        counts.append(kernel_lib.MusaKernelsLaunchCount())
+        raw_ops.FusedBatchNormGradV3(dy, x, s, f.reserve_space_1, f.reserve_space_2, None, EPS)
+        counts.append(kernel_lib.MusaKernelsLaunchCount())
+    assert (counts[1] - counts[0], counts[2] - counts[1]) == kernels
+
+
 def test_in_place_streams_and_capture(kernel_lib):
     """Large layers by the rule: y on top of x, two streams at once, and a captured call give the
     bits of a plain call."""
