@@ -411,18 +411,19 @@ int GridCtas() {
   return found > 0 ? found : 0;
 }
 
-// Where the form is taken; `size`: bytes of x.  Against the cluster form and the chain, us with
-// inputs beyond L2, launches of a graph (chain -> this form): bf16 [25390,512] forward 18.0 -> 13.8,
-// gradient 23.9 -> 19.1; fp32 [100352,64] 17.0 -> 13.6 and 23.6 -> 18.8; bf16 [201171,256] 50.7 ->
-// 43.5 and 81.2 -> 73.7; [802816,256] 191.4 -> 188.4 and 299 -> 307.  Launched one by one on a stream
-// a cooperative kernel starts 2 us after its predecessor, which the chain's programmatic launches hide, and
-// the chain's element-wise kernels run 15 % slower behind it (the SM keeps its small L1): a
-// ResNet-50 step of batch 256 takes 1760 us in the chain, 1767 with the largest gradients in the chain and
-// the rest here, 1702 with all of them here.
-//  - Below 16 MiB of inputs the cluster form is faster or level (fp32 [5859,512] forward 8.5 against 9.0).
-//  - The last two lines are not where the form stops paying (bf16 [156250,64] forward 17.4 -> 12.5): they
-//    keep the chains of two and three kernels that the launch counters are tested with
-//    ([200000,64], [4096,2048]).
+// Where the form is taken: from 16 MiB of inputs.  Us, inputs beyond L2, launches of
+// a graph / one by one on a stream, against what runs otherwise (-> this form):
+//   the chain        bf16 [4096,2048] forward 13.6 / 14.4 -> 11.1 / 13.9, gradient 17.0 / 18.1 ->
+//                    14.3 / 16.5; [3136,2048] gradient 14.7 / 15.7 -> 12.2 / 14.2; [100352,64] gradient
+//                    16.6 / 17.9 -> 12.4 / 14.3; [163840,64] forward 16.4 / 17.5 -> 12.7 / 15.2; fp32
+//                    [262144,16] forward 14.0 / 15.0 -> 11.4 / 13.9; bf16 [100352,256] forward 27.1 /
+//                    28.3 -> 22.4 / 24.8, gradient 42.7 / 43.8 -> 34.7 / 37.1; [401408,256] 99.0 /
+//                    99.9 -> 92.8 / 95.5 and 157 / 158 -> 152 / 155
+//   cluster kernels  (below that line) fp32 [6144,512] forward 8.8 / 9.1 -> 9.6 / 12.4; bf16 [32768,128]
+//                    forward 9.9 / 10.1 -> 8.6 / 10.7; [25088,256] 12.3 / 12.4 -> 9.9 / 12.3: on a stream, where
+//                    a cooperative kernel starts 2 us after its predecessor, level at best.  Narrow layers of 8 to 16 MiB that the
+//                    cluster form leaves to the chain would gain here (bf16 [65536,64] forward 11.0 /
+//                    11.9 -> 8.7 / 11.2).
 // Rows that are not whole 128-byte lines share lines between CTAs or between their row lanes, which
 // are read again where L2 does not hold them in between.  Up to a size that costs less than the form
 // saves; beyond it, chain -> this form, forward and gradient, launches of a graph:
@@ -432,13 +433,15 @@ int GridCtas() {
 //                        182; [1260307,104] (250 MiB) 134, 211 -> 138, 228
 //   of 17 to 31 packs    bf16 [209715,200] (80 MiB) 49, 80 -> 46, 79; 96 MiB 59, 97 -> 60, 99; 200 MiB
 //                        121, 189 -> 147, 229
+// Whole lines have no upper end, although the gradient of the largest 16-bit layers alone is 2 % faster in the
+// chain (bf16 [802816,256] 306 / 307 -> 311 / 313; fp32 of those bytes 316 / 318 -> 311 / 313): forward
+// and gradient in turn are level (501 / 504 -> 498 / 503), and one pass in the chain behind one here
+// takes both 6 % longer than either (531 / 534).
 constexpr int64_t kMiB = 1 << 20;
 
 template <typename T, int kMode>
 bool GridPays(int64_t size, int64_t row_bytes, int64_t cv) {
   if (size * GridRing<kMode>::kStreams < 16 * kMiB) return false;
-  if (cv < 16 && size < 32 * kMiB) return false;
-  if (cv >= 256 && size <= 16 * kMiB) return false;
   if (row_bytes % 128 == 0) return true;
   if (row_bytes % 64 == 0) return size <= 256 * kMiB;
   return size <= (cv > 16 && cv < 32 ? 80 : 128) * kMiB;

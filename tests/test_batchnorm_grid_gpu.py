@@ -48,6 +48,11 @@ def test_against_oracle_and_chain(kernel_lib, dtype, rows, c):
 
 
 @pytest.mark.parametrize("rows,c,kernels", [
+    # 16 MiB of inputs and more, narrow and wide: one kernel a pass.
+    (262144, 32, (1, 1)), (200000, 64, (1, 1)), (100352, 64, (3, 1)), (25088, 256, (3, 1)),
+    (4096, 2048, (1, 1)), (3136, 2048, (2, 1)),
+    # One row less than that: the chain.
+    (131071, 64, (3, 1)), (65535, 64, (3, 3)),
     # Rows that are not whole lines, up to their limits and one row beyond: 64-byte multiples, others,
     # 17 to 31 packs.
     (1398101, 96, (1, 1)), (1398102, 96, (3, 3)), (67108, 1000, (1, 1)), (67109, 1000, (2, 2)),
