@@ -1,5 +1,6 @@
 """The grid-wide one-kernel form of large channels-last BatchNorm layers against the
-CPU oracle and the chain of kernels (tuning key 26: 1 takes the form at every size)."""
+CPU oracle and the chain of kernels (tuning key 26: 1 takes the form at every size, 4, 8 and 16 in column blocks
+of that many packs)."""
 import numpy as np
 import pytest
 import torch
@@ -12,23 +13,34 @@ from test_batchnorm_gpu import EPS, _rms, check_forward, check_grad, launch_ops,
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dtype,rows,c", [
-    # One row; fewer rows than a CTA has row lanes; fewer than there are row lanes in all
-    # (CTAs without a row); one more than that; the narrowest column count; a last
-    # column block that is partly empty, at 4, 8 and 16 packs a block.
-    ("bfloat16", 1, 32), ("float32", 7, 16), ("float16", 300, 64), ("bfloat16", 9473, 64),
-    ("float32", 3001, 20), ("bfloat16", 5000, 40), ("float16", 4099, 96), ("float32", 2500, 160),
-    ("bfloat16", 777, 4104), ("float32", 1025, 2052),
+@pytest.mark.parametrize("dtype,rows,c,tx", [
+    # One row, and fewer rows than a CTA has row lanes: a column block per CTA (c = 0: as many
+    # blocks of 16 packs as SMs).  The scratch holds no other cut of so few rows.
+    ("float32", 1, 0, 1), ("bfloat16", 7, 0, 1),
+    # Fewer rows than there are row lanes in all (CTAs without a row); one more than that.
+    ("float16", 300, 64, 1), ("bfloat16", 9473, 64, 1),
+    # A last column block that is partly empty, at 4, 8 and 16 packs a block.
+    ("float32", 3001, 20, 4), ("float32", 3001, 20, 8), ("float32", 3001, 20, 16),
+    ("bfloat16", 5000, 40, 4), ("bfloat16", 5000, 40, 8), ("bfloat16", 5000, 40, 16),
+    ("bfloat16", 777, 4104, 1), ("float32", 1025, 2052, 1),
+    # Widths that the rule cuts without a remainder.
+    ("float16", 4099, 96, 1), ("float32", 2500, 160, 1),
+    # Rows that are not whole lines: split between CTAs, and in one block.
+    ("bfloat16", 44001, 200, 1), ("float32", 30011, 100, 1), ("float16", 61001, 136, 1),
+    ("bfloat16", 90001, 72, 1),
     # The rings to the last row, one row more, and several rings.
-    ("float32", 113664, 64), ("bfloat16", 227329, 64), ("float16", 500001, 32)])
-def test_against_oracle_and_chain(kernel_lib, dtype, rows, c):
+    ("float32", 113664, 64, 1), ("bfloat16", 227329, 64, 1), ("float16", 500001, 32, 1)])
+def test_against_oracle_and_chain(kernel_lib, dtype, rows, c, tx):
+    if c == 0:
+        c = torch.cuda.get_device_properties(0).multi_processor_count * (64 if dtype == "float32" else 128)
     x, s, o, dy = bn_inputs(rows + c, (rows, c), dtype, 1.0, 3.0)
     gen = np.random.default_rng(c)
     est = gen.standard_normal(c).astype(np.float32), (gen.random(c) + 0.5).astype(np.float32)
     want = np_ref.fused_batch_norm(x, s, o, *est, epsilon=EPS, exponential_avg_factor=0.25)
     wg = np_ref.fused_batch_norm_grad(dy, x, s, want[3], want[4], EPS)
     terms = _rms(dy) * float(np.max(s / np.sqrt(want[4] + EPS)))
-    with tuned(kernel_lib, (26, 1)):
+    # (Key 25 = 3 shuts the cluster form out: one kernel per pass is this form, more is the chain.)
+    with tuned(kernel_lib, (26, tx), (25, 3)):
         before = kernel_lib.MusaKernelsLaunchCount()
         got = launch_ops(kernel_lib, x, s, o, dy, est=est, factor=0.25)
         assert kernel_lib.MusaKernelsLaunchCount() - before == 3
