@@ -498,6 +498,7 @@ BnGridPlan PlanBnGrid(const Geom& g) {
 template <typename T, int kMode>
 int LaunchBnGrid(const BnGridPlan& p, const T* x, const T* dy, T* out, const ApplyArgs& a,
                  float* partial, const Geom& g, cudaStream_t stream) {
+  if (GetTuning(kTuneBnGridRefuse) != 0) return static_cast<int>(cudaErrorCooperativeLaunchTooLarge);
   using Ring = GridRing<kMode>;
   constexpr int kVec = VecWidth<T>::value;
   GridShape s;

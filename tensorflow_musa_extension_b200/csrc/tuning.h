@@ -36,9 +36,12 @@ enum TuningKey {
                             // one-kernel form; 0: by rule, -1: off (the chain of kernels at every size)
   kTuneBnOnChipCluster = 25,  // CTAs per cluster of the one-kernel form; 0: by rule
   kTuneBnGrid = 26,         // one-kernel forms of large layers (grid-wide; channel-major in
-                            // waves): 0 by rule, 1 wherever possible, -1 off
+                            // waves): 0 by rule, 1 wherever possible (grid-wide: 4, 8 or 16 in column
+                            // blocks of that many packs), -1 off
   kTuneRowCtas = 27,        // most CTAs per SM of the row kernels; 0: by rule
-  kTuneCount = 28
+  kTuneBnGridRefuse = 28,   // 1: the grid-wide form's launch answers that it is too large for the context
+                            // (what the caller does then is tested with it)
+  kTuneCount = 29
 };
 
 int GetTuning(int key);

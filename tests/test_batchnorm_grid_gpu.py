@@ -85,6 +85,23 @@ def test_rule(kernel_lib, rows, c, kernels):
     assert (counts[1] - counts[0], counts[2] - counts[1]) == kernels
 
 
+@pytest.mark.parametrize("rows,c", [(200000, 64), (4096, 2048)])
+def test_refused_launch(kernel_lib, rows, c):
+    """A context that owns fewer SMs than the device refuses the launch (key 28 stands in for that):
+    the chain of kernels takes the call."""
+    x, s, o, dy = bn_inputs(9, (rows, c), "bfloat16", 1.0, 3.0)
+    with tuned(kernel_lib, (24, -1)):
+        before = kernel_lib.MusaKernelsLaunchCount()
+        want = launch_ops(kernel_lib, x, s, o, dy)
+        kernels = kernel_lib.MusaKernelsLaunchCount() - before
+    with tuned(kernel_lib, (28, 1)):
+        before = kernel_lib.MusaKernelsLaunchCount()
+        got = launch_ops(kernel_lib, x, s, o, dy)
+        assert kernel_lib.MusaKernelsLaunchCount() - before == kernels > 3
+    for a, b in zip((t for out in got for t in out), (t for out in want for t in out)):
+        assert torch.equal(a, b)
+
+
 def test_in_place_streams_and_capture(kernel_lib):
     """Large layers by the rule: y on top of x, two streams at once, and a captured call give the
     bits of a plain call."""
