@@ -1099,10 +1099,15 @@ int Dispatch(const RowArgs& a, bool aligned, GradRows* rows_out, cudaStream_t st
     // fill no more than half of the four-pack layout of their group take two
     // (fp32 rows of 768: LayerNorm 5.5 against 4.6 TB/s; bf16 [65536,512], exactly
     // half: LayerNorm 33.5 -> 25.9 us, RMSNorm gradient 38.9 -> 34.0; bf16 rows of 500 and
-    // fp32 rows of 250 gain 10 to 28 %) - but the forward LayerNorm of large fp32
-    // tensors of whole packs, at exactly half, wants the deeper ring ([65536,1024] 91 us
-    // with four, 98 with two; [16384,1024] 25.7 and 23.2).  Tuning values 1 .. 4
-    // force a layout.
+    // fp32 rows of 250 gain 10 to 28 %).  Two ops on large fp32 tensors of whole packs, at exactly
+    // half (rows of 64, 256 and 1024), want the deeper ring of four.  Us, two / four:
+    //   LayerNorm         rows of 1024, 64 MiB 23.3 / 25.9, 128 MiB 47.6 / 47.9, 160 MiB 59.9 /
+    //   forward           58.9, 256 MiB 97.8 / 91.7; of 256, 48 MiB 17.1 / 18.0, 64 MiB 23.6 / 23.5,
+    //                     80 MiB 29.7 / 28.7, 128 MiB 49.9 / 46.1; of 64, within 4 % of each other
+    //   RMSNorm gradient  rows of 256, 112 MiB 55.6 / 55.6, 160 MiB 79.9 / 77.5, 400 MiB 208 / 188; of
+    //                     64, 160 MiB 77.5 / 80.2, 200 MiB 96.9 / 99.0, 400 MiB 200 / 194; of 1024,
+    //                     200 MiB 93 / 100, 400 MiB 196 / 196
+    // Tuning values 1 .. 4 force a layout.
     int want = GetTuning(kTuneRowNormPacks);
     if (want < 1 || want > 4) {
       want = 4;
@@ -1115,9 +1120,15 @@ int Dispatch(const RowArgs& a, bool aligned, GradRows* rows_out, cudaStream_t st
           break;
         }
       }
-      const bool deep = sizeof(T) == 4 && kOp == kOpLnFwd && packs == 2 * group &&
-                        a.row_size % VecWidth<T>::value == 0 &&
-                        a.rows * a.row_size > (int64_t{1} << 24);
+      bool deep = false;
+      if constexpr (sizeof(T) == 4 && (kOp == kOpLnFwd || kOp == kOpRmsGrad)) {
+        constexpr int64_t kMValues = 1 << 20;
+        const int64_t line = kOp == kOpLnFwd ? (a.row_size > 512 ? 32 : 16) * kMValues
+                             : a.row_size > 512 ? a.rows * a.row_size
+                                                : (a.row_size > 128 ? 32 : 64) * kMValues;
+        deep = packs == 2 * group && a.row_size % VecWidth<T>::value == 0 &&
+               a.rows * a.row_size > line;
+      }
       if (packs <= 2 * group && !deep) {
         want = 2;
       } else if (packs <= 3 * group && packs > 2 * group) {
