@@ -2848,8 +2848,10 @@ inline OnChipPlan PlanOnChipPlanes(const Geom& g, const void* x, const void* out
 // the same kernel in waves of single CTAs.  Every value is read once; a CTA takes no more
 // than half an SM's shared memory, so that two share the SM and one loads while the
 // other writes.  A wave costs about 4 us beside its bytes, so CTAs have to be well filled
-// (7 to 12 slots) and waves too - two thirds where the chain walks long planes, nine
-// tenths where its channel-group kernels take short ones.  Us, chain -> this form: bf16
+// (7 to 12 slots) and waves too: two thirds for planes of 400 values and more (waves filled to 0.8:
+// 1.09 to 1.48 times as fast as the chain over planes of 400 to 1024, 8 to 11 slots, both
+// types and passes), nine tenths for shorter ones, where the chain is faster per byte (planes of 64 to
+// 360: 0.95 full 1.06 to 1.75 times as fast, 0.8 full 0.99 to 1.35).  Us, chain -> this form: bf16
 // [64,500,24,24] forward 29.9 -> 20.3, [16,512,28,28] gradient 20.3 -> 15.1, [20,1000,28,28]
 // 32.4 -> 27.9; fp32 [10,640,40,40] forward 37.7 -> 21.5, [32,512,20,20] 19.6 -> 16.0,
 // [100,2000,10,10] gradient 68.4 -> 54.8.  Beyond the lines: bf16 [128,2048,8,8] forward, 2 slots,
