@@ -44,12 +44,12 @@ RESNET50_BN = [(1, 112, 112, 64), (6, 56, 56, 64), (4, 56, 56, 256), (8, 28, 28,
                (4, 7, 7, 2048)]
 BATCH = 256
 EPS = 1e-3
-# DRAM bytes per launch from an ncu capture (the summary under profiles/ names
-# the command): 822.2 MB read + 376.4 MB written for 1233.1 MB algorithmic.
-# The whole step: sum over its 318 launches, one single-pass capture per metric with
-# L2 left as the previous kernel left it (profiles/resnet50_bn_step_launch_list.md).
-NCU_TRAFFIC_BYTES = {"bn_grad_apply_bf16_256x56x56x256": 1198591488,
-                     "resnet50_bn_step": 37391728896}
+# DRAM bytes from single-pass ncu captures of one step, one per metric, with L2 left as the
+# previous kernel left it (profiles/resnet50_bn_step_launch_list.md): the gradient of the
+# [256,56,56,256] layers per launch (1557.5 MB read + 410.4 MB written for 1233.1 MB
+# algorithmic), and the sum over the step's 106 launches.
+NCU_TRAFFIC_BYTES = {"bn_grad_bf16_256x56x56x256": 1967949888,
+                     "resnet50_bn_step": 35787736576}
 # One-directional rate of a cudaMemcpyAsync between two B200 of one NVSwitch
 # node, as measured by `bench.py --probe peer_copy` (nominal 900 GB/s).
 PEER_COPY_GBS = 770.0
@@ -353,10 +353,11 @@ def run_ours(args):
         finish(torch, dist, world)
         return
 
-    # Kernels per step, counted by the library itself over one eager step
-    # (three per pass - statistics, finalize, element-wise - or two where the
-    # element-wise kernel adds the partial rows itself; a collective-library
-    # exchange adds launches that are not this library's and are not counted).
+    # Kernels per step, counted by the library itself over one eager step (one
+    # per pass on a single GPU; the cross-replica chain has three per pass, or two
+    # where the element-wise kernel adds the partial rows itself; a
+    # collective-library exchange adds launches that are not this library's and
+    # are not counted).
     step()
     torch.cuda.synchronize()
     launched = lib.MusaKernelsLaunchCount()
@@ -1084,9 +1085,9 @@ def measure_ops(torch, lib, raw_ops, dev, args):
         entry("bn_grad_" + tag, ms, 3 * s_bytes, x.numel(), "L2 flushed before each launch")
         del x, dy, y
 
-    # Dominant kernel of the headline workload: the gradient element-wise pass
-    # (reads dy and x, writes dx: 3 * S per launch), timed alone on the largest
-    # ResNet-50 layer, [256, 56, 56, 256] bf16 (S = 411 MB).
+    # Dominant kernel of the headline workload: the gradient of the largest ResNet-50
+    # layers, [256, 56, 56, 256] bf16 (S = 411 MB), one launch of the grid-wide kernel
+    # (3 * S: reads dy and x, writes dx; what no ring and no L2 holds is read twice).
     rows, c = BATCH * 56 * 56, 256
     x = torch.randn(rows, c, device=dev).to(torch.bfloat16)
     dy = (torch.randn(rows, c, device=dev) * 1e-2).to(torch.bfloat16)
@@ -1096,12 +1097,24 @@ def measure_ops(torch, lib, raw_ops, dev, args):
     varc = torch.ones(c, device=dev)
     sums = torch.zeros(2 * c, device=dev)
     ds, do = torch.empty(c, device=dev), torch.empty(c, device=dev)
+    need = lib.BnWorkspaceBytes(rows, c, 1)
+    ws = torch.empty(need, dtype=torch.uint8, device=dev)
     s_bytes = x.numel() * 2
-    ms, ms_stream = both(lambda: lib.LaunchBnGradApplyFromSums(
-        2, dy.data_ptr(), x.data_ptr(), sc.data_ptr(), mean.data_ptr(), varc.data_ptr(),
-        sums.data_ptr(), float(rows), dx.data_ptr(), None, None, rows, c, 1, EPS, st))
+
+    def gradient():
+        lib.LaunchBnGrad_BF16(
+            dy.data_ptr(), x.data_ptr(), sc.data_ptr(), mean.data_ptr(), varc.data_ptr(),
+            dx.data_ptr(), ds.data_ptr(), do.data_ptr(), rows, c, 1, EPS, True, ws.data_ptr(),
+            need, st)
+
+    before = lib.MusaKernelsLaunchCount()
+    gradient()
+    kernels = lib.MusaKernelsLaunchCount() - before
+    ms, ms_stream = both(gradient)
     achieved = 3 * s_bytes / (ms * 1e-3) / 1e9
-    roof = {"bound": "hbm", "kernel": "BnApplyLastKernel<bf16, grad>",
+    # (A device that refuses cooperative launches runs the chain of kernels.)
+    roof = {"bound": "hbm", "kernel": "BnGridKernel<bf16, grad>" if kernels == 1 else
+            "BnStatsPipeKernel .. BnApplyLastKernel <bf16, grad>, %d launches" % kernels,
             "case": "[256,56,56,256] bf16, 3*S = %d bytes per launch" % (3 * s_bytes),
             "achieved": round(achieved, 1), "peak": peak, "peak_kind": peak_kind,
             "unit": "GB/s", "frac": round(achieved / peak, 4), "ms": round(ms, 4),
@@ -1109,12 +1122,20 @@ def measure_ops(torch, lib, raw_ops, dev, args):
             "nominal_gbs": NOMINAL_HBM_GBS, "traffic": None}
     roof["ms_back_to_back"] = round(ms_stream, 4)
     roof["frac_back_to_back"] = round(3 * s_bytes / (ms_stream * 1e-3) / 1e9 / peak, 4)
-    # The whole op this kernel belongs to (statistics + element-wise pass).
+    # The whole op is this one kernel.
     roof["op"] = "bn_grad_r50_56x56x256_bf16"
     roof["op_frac"] = ops["bn_grad_r50_56x56x256_bf16"]["frac_of_peak"]
-    roof["traffic"] = NCU_TRAFFIC_BYTES["bn_grad_apply_bf16_256x56x56x256"]
-    roof["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of this "
-                              "kernel and case (profiles/bn_grad_apply_bf16_256x56x56x256_ncu_full.md)")
+    if kernels == 1:
+        roof["traffic"] = NCU_TRAFFIC_BYTES["bn_grad_bf16_256x56x56x256"]
+        roof["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel and "
+                                  "case, average of its launches in the step "
+                                  "(profiles/resnet50_bn_step_launch_list.md)")
+
+    # The element-wise pass alone, as the cross-replica gradient launches it.
+    entry("bn_grad_apply_56x56x256_bf16", both(lambda: lib.LaunchBnGradApplyFromSums(
+        2, dy.data_ptr(), x.data_ptr(), sc.data_ptr(), mean.data_ptr(), varc.data_ptr(),
+        sums.data_ptr(), float(rows), dx.data_ptr(), None, None, rows, c, 1, EPS, st)),
+        3 * s_bytes, x.numel(), "S=411 MB (inputs beyond L2)")
     return ops, roof
 
 
