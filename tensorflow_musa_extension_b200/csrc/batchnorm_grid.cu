@@ -433,10 +433,11 @@ int GridCtas() {
 //                        182; [1260307,104] (250 MiB) 134, 211 -> 138, 228
 //   of 17 to 31 packs    bf16 [209715,200] (80 MiB) 49, 80 -> 46, 79; 96 MiB 59, 97 -> 60, 99; 200 MiB
 //                        121, 189 -> 147, 229
-// Whole lines have no upper end, although the gradient of the largest 16-bit layers alone is 2 % faster in the
-// chain (bf16 [802816,256] 306 / 307 -> 311 / 313; fp32 of those bytes 316 / 318 -> 311 / 313): forward
-// and gradient in turn are level (501 / 504 -> 498 / 503), and one pass in the chain behind one here
-// takes both 6 % longer than either (531 / 534).
+// Whole lines have no upper end, although the gradient alone of most layers of 250 MiB and more is 2 % faster
+// in the chain (bf16 [802816,256] 306 / 307 -> 311 / 313, [64000,2048] 190 -> 195, fp32 [16000,4096] 191 ->
+// 196; but fp32 [1605632,64] 316 / 318 -> 311 / 313): forward and gradient in turn are level or better (bf16
+// [802816,256] 501 / 504 -> 498 / 503), and one pass in the chain behind one here takes both 6 % longer
+// than either (531 / 534).
 constexpr int64_t kMiB = 1 << 20;
 
 template <typename T, int kMode>

@@ -103,8 +103,8 @@ def test_refused_launch(kernel_lib, rows, c):
 
 
 def test_in_place_streams_and_capture(kernel_lib):
-    """Large layers by the rule: y on top of x, two streams at once, and a captured call give the
-    bits of a plain call."""
+    """Large layers by the rule: y on top of x, two streams at once, a call beside another stream's
+    kernel, and a captured call give the bits of a plain call."""
     e = torch.empty(0, device="cuda")
     x, s, o, dy = (to_torch(a) for a in bn_inputs(1, (60000, 256), "bfloat16", 1.0, 3.0))
 
@@ -130,6 +130,10 @@ def test_in_place_streams_and_capture(kernel_lib):
         for st in streams:
             with torch.cuda.stream(st):
                 outs.append(step())
+    torch.cuda.synchronize()
+    with torch.cuda.stream(streams[0]):
+        torch.cuda._sleep(2_000_000)   # about a millisecond on one SM
+    outs.append(step())
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
