@@ -702,11 +702,12 @@ __global__ void __launch_bounds__(RowThreads(kGroup, kOp),
       }
     }
     __syncthreads();
-    // Whole packs: in the slabs' own order, four columns at a time (column by column, with
-    // the divisions that takes, this tail was 1.5 us of the call; LnGradFinalizeKernel
-    // knows the order).
+    // In the slabs' own order (LnGradFinalizeKernel knows it; to plain order, with the
+    // divisions that takes, this tail was 1.5 us of the call), whole packs four columns at a
+    // time - but not for the shortest rows, whose kernel the compiler then schedules worse, the row
+    // loop with it: bf16 [3276800,32] 283 us so, 269 column by column, [1638400,64] 144 and 137.
     float* out = a.partial + static_cast<int64_t>(blockIdx.x) * 2 * a.row_size;
-    if constexpr (kShifted) {
+    if constexpr (kShifted || kGroup == 8) {
       for (int c = threadIdx.x; c < 2 * a.row_size; c += kThreads) {
         float s = slab[c];
         for (int l = 1; l < kRows; ++l) s += slab[static_cast<size_t>(l) * 2 * a.row_size + c];
